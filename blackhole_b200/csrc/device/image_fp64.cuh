@@ -15,6 +15,7 @@
 // a host build of the same arithmetic.
 #pragma once
 
+#include "ieee_fp64.cuh"
 #include "launch.h"
 
 namespace bhk {
@@ -32,23 +33,25 @@ __device__ __forceinline__ double dmin_(double a, double b) { return (b < a) ? b
 
 __device__ __forceinline__ Yd rhs(const Yd &y, const RayC &c) {
   const double r = y.r, u = y.u;
-  const double A = ((r * r) + c.a2) - (c.a * c.lam);
-  const double D = ((r * r) - (2.0 * r)) + c.a2;
+  // a product with 2 is exact, so fma(2, x, y) rounds as 2 x + y does
+  const double rr = r * r;
+  const double A = (rr + c.a2) - (c.a * c.lam);
+  const double D = fma(-2.0, r, rr) + c.a2;
   const double u2 = u * u;
   const double s2 = dmax_(1.0 - u2, 1e-12);
   Yd d;
   d.r = y.pr;
   d.u = y.pu;
-  d.pr = ((2.0 * r) * A) - ((r - 1.0) * c.K);
+  d.pr = fma(2.0, r * A, -((r - 1.0) * c.K));
   d.pu = u * ((c.a2 - c.qTh) - ((2.0 * c.a2) * u2));
   // horizon-regular azimuth psi = phi - a G(r), G' = 1/Delta: psi' = a -
   // lambda/sin^2 - a (A + p_r)/Delta, with (A + p_r)/Delta = K/(A - p_r) on
   // the first integral for ingoing rays (the rationalization of the
   // reference's GPU step, src/cuda/device_physics.cuh:453-525)
-  const bool in = y.pr < 0.0;
+  const bool in = is_neg(y.pr);
   const double num = in ? c.K : (A + y.pr);
   const double den = in ? (A - y.pr) : D;
-  d.phi = (c.a - (c.lam / s2)) - (c.a * (num / den));
+  d.phi = (c.a - div_rn(c.lam, s2)) - (c.a * div_rn(num, den));
   return d;
 }
 
@@ -72,7 +75,7 @@ __device__ __forceinline__ Yd axpy(const Yd &y, double h, const Yd &k) {
 // R(r) with E = 1, M = 1.
 __device__ __forceinline__ double pot_R(double r, const RayC &c) {
   const double A = ((r * r) + (c.a * c.a)) - (c.a * c.lam);
-  const double D = ((r * r) - (2.0 * r)) + (c.a * c.a);
+  const double D = fma(-2.0, r, r * r) + (c.a * c.a);
   return (A * A) - (D * c.K);
 }
 
@@ -97,16 +100,16 @@ __device__ __forceinline__ double project(Yd &y, const RayC &c, bool want_drift 
   const double Rv = pot_R(y.r, c);
   const double r2 = y.r * y.r;
   if (Rv > kProjTau * (r2 * r2)) {
-    const double m = sqrt(Rv);
-    y.pr = (y.pr < 0.0) ? -m : m;
+    const double m = sqrt_rn(Rv);
+    y.pr = is_neg(y.pr) ? -m : m;
   }
   const double Uv = pot_U(y.u, c);
   const double scale = fabs(c.qTh) + (c.a * c.a);
   double drift = 0.0;
   if (Uv > kProjTau * scale) {
     if (want_drift) drift = fabs((y.pu * y.pu) - Uv) / ((1.0 - (y.u * y.u)) * scale);
-    const double m = sqrt(Uv);
-    y.pu = (y.pu < 0.0) ? -m : m;
+    const double m = sqrt_rn(Uv);
+    y.pu = is_neg(y.pu) ? -m : m;
   }
   return drift;
 }
@@ -116,19 +119,19 @@ __device__ __forceinline__ Yd rk4(const Yd &y, double h, const RayC &c, const Yd
   const double hh = 0.5 * h;
   const Yd k2 = rhs(axpy(y, hh, k1), c);
   Yd s;
-  s.r = k1.r + 2.0 * k2.r;
-  s.u = k1.u + 2.0 * k2.u;
-  s.phi = k1.phi + 2.0 * k2.phi;
-  s.pr = k1.pr + 2.0 * k2.pr;
-  s.pu = k1.pu + 2.0 * k2.pu;
+  s.r = fma(2.0, k2.r, k1.r);
+  s.u = fma(2.0, k2.u, k1.u);
+  s.phi = fma(2.0, k2.phi, k1.phi);
+  s.pr = fma(2.0, k2.pr, k1.pr);
+  s.pu = fma(2.0, k2.pu, k1.pu);
   const Yd k3 = rhs(axpy(y, hh, k2), c);
-  s.r = s.r + 2.0 * k3.r;
-  s.u = s.u + 2.0 * k3.u;
-  s.phi = s.phi + 2.0 * k3.phi;
-  s.pr = s.pr + 2.0 * k3.pr;
-  s.pu = s.pu + 2.0 * k3.pu;
+  s.r = fma(2.0, k3.r, s.r);
+  s.u = fma(2.0, k3.u, s.u);
+  s.phi = fma(2.0, k3.phi, s.phi);
+  s.pr = fma(2.0, k3.pr, s.pr);
+  s.pu = fma(2.0, k3.pu, s.pu);
   const Yd k4 = rhs(axpy(y, h, k3), c);
-  const double w = h / 6.0;
+  const double w = div_6(h);
   Yd n;
   n.r = y.r + w * (s.r + k4.r);
   n.u = y.u + w * (s.u + k4.u);
@@ -192,14 +195,14 @@ __device__ __forceinline__ DPRes dp45(const Yd &y, double h, const RayC &c, cons
   (h * ((((((dp::e1 * k1.f) + (dp::e3 * k3.f)) + (dp::e4 * k4.f)) + (dp::e5 * k5.f)) + (dp::e6 * k6.f)) + \
         (dp::e7 * o.k7.f)))
 #define BHK_SC(f) (atol + rtol * dmax_(fabs(y.f), fabs(o.y5.f)))
-  const double q0 = BHK_ECOMP(r) / BHK_SC(r);
-  const double q1 = BHK_ECOMP(u) / BHK_SC(u);
-  const double q2 = BHK_ECOMP(phi) / BHK_SC(phi);
-  const double q3 = BHK_ECOMP(pr) / BHK_SC(pr);
-  const double q4 = BHK_ECOMP(pu) / BHK_SC(pu);
+  const double q0 = div_rn(BHK_ECOMP(r), BHK_SC(r));
+  const double q1 = div_rn(BHK_ECOMP(u), BHK_SC(u));
+  const double q2 = div_rn(BHK_ECOMP(phi), BHK_SC(phi));
+  const double q3 = div_rn(BHK_ECOMP(pr), BHK_SC(pr));
+  const double q4 = div_rn(BHK_ECOMP(pu), BHK_SC(pu));
 #undef BHK_ECOMP
 #undef BHK_SC
-  o.err = sqrt(((((q0 * q0) + (q1 * q1)) + (q2 * q2)) + (q3 * q3) + (q4 * q4)) / 5.0);
+  o.err = sqrt_rn(div_5(((((q0 * q0) + (q1 * q1)) + (q2 * q2)) + (q3 * q3) + (q4 * q4))));
   return o;
 }
 
@@ -208,15 +211,18 @@ __device__ __forceinline__ DPRes dp45(const Yd &y, double h, const RayC &c, cons
 // iteration y <- y (6 - z y^5) / 5 from 2^(-j/5) rises monotonically to
 // z^(-1/5). Free of libm, so host and device give the same bits.
 __device__ __forceinline__ double inv_fifth_root(double x) {
-  int e = 0;
-  const double m = frexp(x, &e);
+  // frexp and ldexp of a normal x by its exponent field (step_factor's caller
+  // never passes a subnormal: sqrt_rn hands those back as the square, < 1e-290,
+  // whose factor is past every bound)
+  const int hi = __double2hiint(x);
+  const int e = (hi >> 20) - 1022;
   int k = e / 5;
   int j = e - 5 * k;
   if (j < 0) {
     j += 5;
     k -= 1;
   }
-  const double z = ldexp(m, j);
+  const double z = __hiloint2double((hi & 0x000fffff) | ((1022 + j) << 20), __double2loint(x));
   double y = (j == 0)   ? 1.0
              : (j == 1) ? 0.87055056329612412
              : (j == 2) ? 0.75785828325519899
@@ -226,9 +232,9 @@ __device__ __forceinline__ double inv_fifth_root(double x) {
   for (int it = 0; it < 6; ++it) {
     const double y2 = y * y;
     const double y5 = (y2 * y2) * y;
-    y = (y * (6.0 - (z * y5))) / 5.0;
+    y = div_5(y * (6.0 - (z * y5)));
   }
-  return ldexp(y, -k);
+  return __hiloint2double(__double2hiint(y) - (k << 20), __double2loint(y));
 }
 
 // Step factor of the Hairer-Norsett-Wanner controller (safety 0.9, bounds

@@ -143,7 +143,7 @@ __device__ __forceinline__ int iterate(const BhkImageParams &p, const BhkImageOu
     if (R.y.r >= p.r_esc) return 2;
     const double hh = p.step_coeff * dmin_(R.y.r, p.step_rcap);
     const double sigma = (R.y.r * R.y.r) + ((p.a2 * R.y.u) * R.y.u);
-    const double h = hh / sigma;
+    const double h = div_rn(hh, sigma);
     const Yd k0 = rhs(R.y, R.c);
     Yd yn = rk4(R.y, h, R.c, k0);
     ++R.steps;
@@ -469,7 +469,7 @@ __global__ void __launch_bounds__(128) k_trace_paths_fp64(const __grid_constant_
     ++n;
     if (n >= max_points || R.y.r <= p.r_hor || R.y.r >= p.r_esc) break;
     const double hh = p.step_coeff * dmin_(R.y.r, p.step_rcap);
-    const double h = hh / ((R.y.r * R.y.r) + ((p.a2 * R.y.u) * R.y.u));
+    const double h = div_rn(hh, (R.y.r * R.y.r) + ((p.a2 * R.y.u) * R.y.u));
     R.y = rk4(R.y, h, R.c, rhs(R.y, R.c));
     project(R.y, R.c);
   }
