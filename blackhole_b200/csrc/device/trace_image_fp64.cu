@@ -72,13 +72,29 @@ __device__ __forceinline__ void init_ray(const BhkImageParams &p, long long pix,
   }
 }
 
-// Crossing of u = 0 inside the accepted step y0 -> y1 (y1 before the
-// projection) with k0 = rhs(y0), k1 = rhs(y1): Hermite interpolation.
-__device__ __forceinline__ void step_crossing(const Yd &y0, const Yd &k0, const Yd &y1, const Yd &k1, double h,
-                                              double &r_c, double &phi_c) {
-  const bhh_dev::Ends e{y0.r, y0.u, y0.phi, y0.pr, y0.pu, k0.pr, k0.pu, k0.phi,
-                        y1.r, y1.u, y1.phi, y1.pr, y1.pu, k1.pr, k1.pu, k1.phi};
-  bhh_dev::hermite_crossing(e, h, r_c, phi_c);
+// The step in which a lane's ray crosses u = 0, y0 -> y1 (y1 before the
+// projection) with k0 = rhs(y0), k1 = rhs(y1), kept in shared memory until
+// the warp locates its held lanes' crossings together (trace_loop).
+struct HeldSteps {
+  double v[17][128];
+};
+
+__device__ __forceinline__ void hold_step(HeldSteps &hs, const Yd &y0, const Yd &k0, const Yd &y1, const Yd &k1,
+                                          double h) {
+  const int t = threadIdx.x;
+  hs.v[0][t] = y0.r, hs.v[1][t] = y0.u, hs.v[2][t] = y0.phi, hs.v[3][t] = y0.pr, hs.v[4][t] = y0.pu;
+  hs.v[5][t] = k0.pr, hs.v[6][t] = k0.pu, hs.v[7][t] = k0.phi;
+  hs.v[8][t] = y1.r, hs.v[9][t] = y1.u, hs.v[10][t] = y1.phi, hs.v[11][t] = y1.pr, hs.v[12][t] = y1.pu;
+  hs.v[13][t] = k1.pr, hs.v[14][t] = k1.pu, hs.v[15][t] = k1.phi;
+  hs.v[16][t] = h;
+}
+
+__device__ __forceinline__ void held_crossing(const HeldSteps &hs, double &r_c, double &phi_c) {
+  const int t = threadIdx.x;
+  const bhh_dev::Ends e{hs.v[0][t], hs.v[1][t], hs.v[2][t],  hs.v[3][t],  hs.v[4][t],  hs.v[5][t],
+                        hs.v[6][t], hs.v[7][t], hs.v[8][t],  hs.v[9][t],  hs.v[10][t], hs.v[11][t],
+                        hs.v[12][t], hs.v[13][t], hs.v[14][t], hs.v[15][t]};
+  bhh_dev::hermite_crossing(e, hs.v[16][t], r_c, phi_c);
 }
 
 // Records a crossing at (r_c, phi_c) when it lies on the disk; returns true
@@ -132,11 +148,12 @@ __device__ __forceinline__ void finish(const BhkImageParams &p, const BhkImageOu
 }
 
 // One iteration of the trace loop for an active ray; returns the class when
-// the ray terminates, -1 otherwise.
+// the ray terminates, kCross when the step crosses the equator (the step is
+// held in hs), kRun otherwise.
 // DRIFT: keep the largest Carter-constant residual the projection removes (a
 // separate instantiation, so the plain kernels carry none of it).
 template <int INTEG, bool DRIFT = false>
-__device__ __forceinline__ int iterate(const BhkImageParams &p, const BhkImageOut &o, RayFp64 &R) {
+__device__ __forceinline__ int iterate(const BhkImageParams &p, HeldSteps &hs, RayFp64 &R) {
   if (INTEG == 0) {
     if (R.steps >= p.max_steps) return 3;
     if (R.y.r <= p.r_hor) return 0;
@@ -147,17 +164,14 @@ __device__ __forceinline__ int iterate(const BhkImageParams &p, const BhkImageOu
     const Yd k0 = rhs(R.y, R.c);
     Yd yn = rk4(R.y, h, R.c, k0);
     ++R.steps;
-    if ((R.y.u * yn.u) < 0.0) {
-      double r_c, phi_c;
-      step_crossing(R.y, k0, yn, rhs(yn, R.c), h, r_c, phi_c);
-      if (on_crossing(p, o, R, r_c, phi_c)) return 1;
-    }
+    const bool cross = (R.y.u * yn.u) < 0.0;
+    if (cross) hold_step(hs, R.y, k0, yn, rhs(yn, R.c), h);
     if (DRIFT)
       R.drift = dmax_(R.drift, project(yn, R.c, true));
     else
       project(yn, R.c);
     R.y = yn;
-    return -1;
+    return cross ? bhsrc::kCross : bhsrc::kRun;
   } else {
     const long long max_attempts = 4LL * p.max_steps + 64;
     if (R.steps >= p.max_steps || R.attempts >= max_attempts) return 3;
@@ -169,15 +183,9 @@ __device__ __forceinline__ int iterate(const BhkImageParams &p, const BhkImageOu
     // keeps its state and re-projects it, which is exact no-op because every
     // state is already on its first integrals (projected at set-up).
     const bool acc = d.err <= 1.0;
-    bool stop = false;
-    if (acc) {
-      ++R.steps;
-      if ((R.y.u * d.y5.u) < 0.0) {
-        double r_c, phi_c;
-        step_crossing(R.y, R.k1, d.y5, d.k7, R.h, r_c, phi_c);
-        stop = on_crossing(p, o, R, r_c, phi_c);
-      }
-    }
+    const bool cross = acc && (R.y.u * d.y5.u) < 0.0;
+    if (acc) ++R.steps;
+    if (cross) hold_step(hs, R.y, R.k1, d.y5, d.k7, R.h);
     R.y = acc ? d.y5 : R.y;
     R.k1 = acc ? d.k7 : R.k1;
     const double drift = project(R.y, R.c, DRIFT);
@@ -185,53 +193,67 @@ __device__ __forceinline__ int iterate(const BhkImageParams &p, const BhkImageOu
     R.k1.r = R.y.pr;  // projection moves only the momenta
     R.k1.u = R.y.pu;
     R.h = R.h * step_factor(d.err, acc);
-    return stop ? 1 : -1;
+    return cross ? bhsrc::kCross : bhsrc::kRun;
   }
 }
 
-// The persistent loop shared by the single-frame and batch kernels. Every
-// `refill` integration steps, the lanes whose ray finished take new work
-// items with one warp-aggregated atomicAdd on the counter (ballot + popc).
+// The persistent loop shared by the single-frame and batch kernels. A lane
+// whose ray crosses the equator or ends is held (see kHold) until the warp
+// serves its held lanes together: crossings are located, outputs of ended
+// rays written, and new work items taken with one warp-aggregated atomicAdd
+// on the counter (ballot + popc).
 template <int INTEG, bool DRIFT = false, class Src>
 __device__ __forceinline__ void trace_loop(const Src &src, unsigned long long *__restrict__ counter, int refill) {
+  __shared__ HeldSteps hs;
   const unsigned lane = threadIdx.x & 31u;
   const unsigned lanemask_lt = (1u << lane) - 1u;
   const unsigned long long total = (unsigned long long)src.total();
   RayFp64 R;
-  bool active = false;
+  int st = bhsrc::kEmpty;
   bool exhausted = false;
+  int waited = bhsrc::kHold;  // the first pass fills every lane
   for (;;) {
-    const unsigned need = __ballot_sync(kFull, !active && !exhausted);
-    if (need) {
-      const int leader = __ffs(need) - 1;
-      unsigned long long base = 0;
-      if ((int)lane == leader) base = atomicAdd(counter, (unsigned long long)__popc(need));
-      base = __shfl_sync(kFull, base, leader);
-      if (!active && !exhausted) {
-        const unsigned long long mine = base + (unsigned long long)__popc(need & lanemask_lt);
-        if (mine < total) {
-          long long pix;
-          const int f = src.frame_of((long long)mine, pix);
-          init_ray(src.params(f), pix, R);
-          R.f = f;
-          active = true;
-        } else {
-          exhausted = true;
+    const unsigned running = __ballot_sync(kFull, st == bhsrc::kRun);
+    const unsigned held = __ballot_sync(kFull, st != bhsrc::kRun && !(st == bhsrc::kEmpty && exhausted));
+    if (held) {
+      waited += __popc(held) * refill;
+      if (waited >= bhsrc::kHold || !running) {
+        waited = 0;
+        if (st == bhsrc::kCross) {
+          double r_c, phi_c;
+          held_crossing(hs, r_c, phi_c);
+          st = on_crossing(src.params(R.f), src.out(R.f), R, r_c, phi_c) ? 1 : bhsrc::kRun;
         }
-      }
-    }
-    if (!__any_sync(kFull, active)) break;
-    for (int k = 0; k < refill; ++k) {
-      if (active) {
-        const BhkImageParams &P = src.params(R.f);
-        const int cls = iterate<INTEG, DRIFT>(P, src.out(R.f), R);
-        if (cls >= 0) {
-          finish(P, src.out(R.f), R, cls);
+        if (st >= 0) {
+          finish(src.params(R.f), src.out(R.f), R, st);
           src.pixel_done(R.f);
-          active = false;
+          st = bhsrc::kEmpty;
+        }
+        const unsigned need = __ballot_sync(kFull, st == bhsrc::kEmpty && !exhausted);
+        if (need) {
+          const int leader = __ffs(need) - 1;
+          unsigned long long base = 0;
+          if ((int)lane == leader) base = atomicAdd(counter, (unsigned long long)__popc(need));
+          base = __shfl_sync(kFull, base, leader);
+          if (st == bhsrc::kEmpty && !exhausted) {
+            const unsigned long long mine = base + (unsigned long long)__popc(need & lanemask_lt);
+            if (mine < total) {
+              long long pix;
+              const int f = src.frame_of((long long)mine, pix);
+              init_ray(src.params(f), pix, R);
+              R.f = f;
+              st = bhsrc::kRun;
+            } else {
+              exhausted = true;
+            }
+          }
         }
       }
+    } else if (!running) {
+      break;
     }
+    for (int k = 0; k < refill; ++k)
+      if (st == bhsrc::kRun) st = iterate<INTEG, DRIFT>(src.params(R.f), hs, R);
   }
 }
 

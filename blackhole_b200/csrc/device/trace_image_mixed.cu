@@ -358,12 +358,47 @@ __device__ __forceinline__ bool vol_step(const BhkImageParams &p, const BhkVolum
   return false;
 }
 
+// The step in which a lane's ray crosses u = 0 (start y0 + lo0 with k0 =
+// rhs(y0), end y1 + lo1 before the projection with k1 = rhs(y1), length h),
+// kept in shared memory until the warp locates its held lanes' crossings
+// together (trace_loop).
+struct HeldSteps {
+  float v[23][128];
+};
+
+__device__ __forceinline__ void hold_step(HeldSteps &hs, const Yf &y0, const Lof &lo0, const Yf &k0, const Yf &y1,
+                                          const Lof &lo1, const Yf &k1, float h) {
+  const int t = threadIdx.x;
+  hs.v[0][t] = y0.r, hs.v[1][t] = y0.u, hs.v[2][t] = y0.phi, hs.v[3][t] = y0.pr, hs.v[4][t] = y0.pu;
+  hs.v[5][t] = lo0.r, hs.v[6][t] = lo0.u, hs.v[7][t] = lo0.phi;
+  hs.v[8][t] = k0.pr, hs.v[9][t] = k0.pu, hs.v[10][t] = k0.phi;
+  hs.v[11][t] = y1.r, hs.v[12][t] = y1.u, hs.v[13][t] = y1.phi, hs.v[14][t] = y1.pr, hs.v[15][t] = y1.pu;
+  hs.v[16][t] = lo1.r, hs.v[17][t] = lo1.u, hs.v[18][t] = lo1.phi;
+  hs.v[19][t] = k1.pr, hs.v[20][t] = k1.pu, hs.v[21][t] = k1.phi;
+  hs.v[22][t] = h;
+}
+
+__device__ __forceinline__ void held_crossing(const HeldSteps &hs, double &r_c, double &phi_c) {
+  const int t = threadIdx.x;
+  const bhh_dev::Ends e{to_f64(hs.v[0][t], hs.v[5][t]),   to_f64(hs.v[1][t], hs.v[6][t]),
+                        to_f64(hs.v[2][t], hs.v[7][t]),   (double)hs.v[3][t],
+                        (double)hs.v[4][t],               (double)hs.v[8][t],
+                        (double)hs.v[9][t],               (double)hs.v[10][t],
+                        to_f64(hs.v[11][t], hs.v[16][t]), to_f64(hs.v[12][t], hs.v[17][t]),
+                        to_f64(hs.v[13][t], hs.v[18][t]), (double)hs.v[14][t],
+                        (double)hs.v[15][t],              (double)hs.v[19][t],
+                        (double)hs.v[20][t],              (double)hs.v[21][t]};
+  bhh_dev::hermite_crossing(e, (double)hs.v[22][t], r_c, phi_c);
+}
+
 // Applies the increment d of an accepted step (acc) to the ray: compensated
 // positions, crossing test and record, projection; returns true if the ray
 // stops. A rejected attempt (acc false) runs the same instructions with a
 // zero increment -- adding 0 leaves a compensated pair unchanged and the
 // projection is idempotent on a projected state -- so accepted and rejected
-// lanes of a warp never diverge. k0 = rhs(y0); k1 = rhs(y1) when the caller
+// lanes of a warp never diverge. Returns the lane's state: kCross when the
+// step crosses the equator (held in hs; kCrossStop when the slab has stopped
+// the ray too), 1 when the slab alone stopped it, else kRun. k0 = rhs(y0); k1 = rhs(y1) when the caller
 // has it (DP45's FSAL stage), else NULL and evaluated only at a crossing.
 // TRACK: also keep the ray's closest approach (camera rays): the smallest r
 // of the step ends, and inside a step where p_r turns from negative to
@@ -374,9 +409,8 @@ __device__ __forceinline__ bool vol_step(const BhkImageParams &p, const BhkVolum
 // DRIFT: keep the largest Carter-constant residual the projection removes (a
 // separate instantiation, so the plain kernels carry none of it).
 template <bool TRACK = false, bool VOL = false, bool DRIFT = false>
-__device__ __forceinline__ bool accept(const BhkImageParams &p, const BhkImageOut &o, RayMx &R, const Yf &d,
-                                       bool acc, float h, const Yf &k0, const Yf *k1,
-                                       const BhkVolume *vol = nullptr) {
+__device__ __forceinline__ int accept(const BhkImageParams &p, HeldSteps &hs, RayMx &R, const Yf &d, bool acc, float h, const Yf &k0, const Yf *k1,
+                                      const BhkVolume *vol = nullptr) {
   const Yf y0 = R.y;
   const Lof lo0 = R.lo;
   comp_add(R.y.r, R.lo.r, acc ? d.r : 0.0f);
@@ -404,25 +438,15 @@ __device__ __forceinline__ bool accept(const BhkImageParams &p, const BhkImageOu
   }
   bool stop = false;
   if (VOL && acc && k1) stop = vol_step(p, *vol, R, y0, lo0, k0, *k1, h);
-  if (acc && (y0.u + lo0.u) * (R.y.u + R.lo.u) < 0.0f) {
-    const Yf kk = k1 ? *k1 : rhs(R.y, R.c);
-    const bhh_dev::Ends e{to_f64(y0.r, lo0.r),   to_f64(y0.u, lo0.u),   to_f64(y0.phi, lo0.phi),
-                          (double)y0.pr,         (double)y0.pu,         (double)k0.pr,
-                          (double)k0.pu,         (double)k0.phi,        to_f64(R.y.r, R.lo.r),
-                          to_f64(R.y.u, R.lo.u), to_f64(R.y.phi, R.lo.phi), (double)R.y.pr,
-                          (double)R.y.pu,        (double)kk.pr,         (double)kk.pu,
-                          (double)kk.phi};
-    double r_c, phi_c;
-    bhh_dev::hermite_crossing(e, (double)h, r_c, phi_c);
-    stop = on_crossing(p, o, R, r_c, phi_c) || stop;
-  }
+  const bool cross = acc && (y0.u + lo0.u) * (R.y.u + R.lo.u) < 0.0f;
+  if (cross) hold_step(hs, y0, lo0, k0, R.y, R.lo, k1 ? *k1 : rhs(R.y, R.c), h);
   const float drift = project(R.y, R.lo, R.cd, DRIFT);
   if (DRIFT && acc) R.drift = fmaxf(R.drift, drift);
-  return stop;
+  return cross ? (stop ? bhsrc::kCrossStop : bhsrc::kCross) : (stop ? 1 : bhsrc::kRun);
 }
 
 template <int INTEG, bool TRACK = false, bool VOL = false, bool DRIFT = false>
-__device__ __forceinline__ int iterate(const BhkImageParams &p, const BhkImageOut &o, RayMx &R,
+__device__ __forceinline__ int iterate(const BhkImageParams &p, HeldSteps &hs, RayMx &R,
                                        const BhkVolume *vol = nullptr) {
   const float r_hor = R.r_hor, r_esc = R.r_esc;
   if (INTEG == 0) {
@@ -433,7 +457,7 @@ __device__ __forceinline__ int iterate(const BhkImageParams &p, const BhkImageOu
     const float h = __fdividef(hh, fmaf(R.c.a2 * R.y.u, R.y.u, R.y.r * R.y.r));
     const Yf k0 = rhs(R.y, R.c);
     const Yf d = rk4_inc(R.y, h, R.c, k0);
-    return accept<TRACK, VOL, DRIFT>(p, o, R, d, true, h, k0, nullptr, vol) ? 1 : -1;
+    return accept<TRACK, VOL, DRIFT>(p, hs, R, d, true, h, k0, nullptr, vol);
   } else {
     const long long max_attempts = 4LL * p.max_steps + 64;
     if (R.steps >= p.max_steps || R.attempts >= max_attempts) return 3;
@@ -443,12 +467,12 @@ __device__ __forceinline__ int iterate(const BhkImageParams &p, const BhkImageOu
     const DPf d = dp45(R.y, R.h, R.c, R.k1, R.rtol, R.atol, true);
     const bool acc = d.err <= 1.0f;
     const float h = R.h;
-    const bool stop = accept<TRACK, VOL, DRIFT>(p, o, R, d.d, acc, h, R.k1, &d.k7, vol);
+    const int st = accept<TRACK, VOL, DRIFT>(p, hs, R, d.d, acc, h, R.k1, &d.k7, vol);
     R.k1 = acc ? d.k7 : R.k1;
     R.k1.r = R.y.pr;  // projection moved only the momenta
     R.k1.u = R.y.pu;
     R.h = h * step_factor(d.err, acc);
-    return stop ? 1 : -1;
+    return st;
   }
 }
 
@@ -459,7 +483,7 @@ struct CameraSrc {
   const BhkImageOut &o;
   __device__ __forceinline__ long long total() const { return p.n_pix; }
   __device__ __forceinline__ int frame_of(long long w, long long &pix) const {
-    pix = w;
+    pix = bhsrc::tile_pixel(w, cam.width, p.n_pix);
     return 0;
   }
   __device__ __forceinline__ const BhkImageParams &params(int) const { return p; }
@@ -542,48 +566,62 @@ __device__ __forceinline__ void init_from(const CameraVolSrc &src, int f, long l
 // trace_image_fp64.cu).
 template <int INTEG, bool DRIFT = false, class Src>
 __device__ __forceinline__ void trace_loop(const Src &src, unsigned long long *__restrict__ counter, int refill) {
+  __shared__ HeldSteps hs;
   const unsigned lane = threadIdx.x & 31u;
   const unsigned lanemask_lt = (1u << lane) - 1u;
   const unsigned long long total = (unsigned long long)src.total();
   RayMx R;
-  bool active = false;
+  int st = bhsrc::kEmpty;
   bool exhausted = false;
+  int waited = bhsrc::kHold;  // the first pass fills every lane
   for (;;) {
-    const unsigned need = __ballot_sync(kFull, !active && !exhausted);
-    if (need) {
-      const int leader = __ffs(need) - 1;
-      unsigned long long base = 0;
-      if ((int)lane == leader) base = atomicAdd(counter, (unsigned long long)__popc(need));
-      base = __shfl_sync(kFull, base, leader);
-      if (!active && !exhausted) {
-        const unsigned long long mine = base + (unsigned long long)__popc(need & lanemask_lt);
-        if (mine < total) {
-          long long pix;
-          const int f = src.frame_of((long long)mine, pix);
-          init_from(src, f, pix, R);
-          R.f = f;
-          active = true;
-        } else {
-          exhausted = true;
+    const unsigned running = __ballot_sync(kFull, st == bhsrc::kRun);
+    const unsigned held = __ballot_sync(kFull, st != bhsrc::kRun && !(st == bhsrc::kEmpty && exhausted));
+    if (held) {
+      waited += __popc(held) * refill;
+      if (waited >= bhsrc::kHold || !running) {
+        waited = 0;
+        if (st == bhsrc::kCross || st == bhsrc::kCrossStop) {
+          double r_c, phi_c;
+          held_crossing(hs, r_c, phi_c);
+          const bool last = on_crossing(src.params(R.f), src.out(R.f), R, r_c, phi_c);
+          st = last || st == bhsrc::kCrossStop ? 1 : bhsrc::kRun;
         }
-      }
-    }
-    if (!__any_sync(kFull, active)) break;
-    for (int k = 0; k < refill; ++k) {
-      if (active) {
-        const BhkImageParams &P = src.params(R.f);
-        const int cls =
-            iterate<INTEG, tracks_closest<Src>::value, has_volume<Src>::value, DRIFT>(P, src.out(R.f), R,
-                                                                                     volume_of(src));
-        if (cls >= 0) {
+        if (st >= 0) {
+          const BhkImageParams &P = src.params(R.f);
           if (tracks_closest<Src>::value) write_closest(P, src.out(R.f), R);
-          if (has_volume<Src>::value) write_vol(P, src.out(R.f), R, cls == 1);
-          finish(P, src.out(R.f), R, cls);
+          if (has_volume<Src>::value) write_vol(P, src.out(R.f), R, st == 1);
+          finish(P, src.out(R.f), R, st);
           src.pixel_done(R.f);
-          active = false;
+          st = bhsrc::kEmpty;
+        }
+        const unsigned need = __ballot_sync(kFull, st == bhsrc::kEmpty && !exhausted);
+        if (need) {
+          const int leader = __ffs(need) - 1;
+          unsigned long long base = 0;
+          if ((int)lane == leader) base = atomicAdd(counter, (unsigned long long)__popc(need));
+          base = __shfl_sync(kFull, base, leader);
+          if (st == bhsrc::kEmpty && !exhausted) {
+            const unsigned long long mine = base + (unsigned long long)__popc(need & lanemask_lt);
+            if (mine < total) {
+              long long pix;
+              const int f = src.frame_of((long long)mine, pix);
+              init_from(src, f, pix, R);
+              R.f = f;
+              st = bhsrc::kRun;
+            } else {
+              exhausted = true;
+            }
+          }
         }
       }
+    } else if (!running) {
+      break;
     }
+    for (int k = 0; k < refill; ++k)
+      if (st == bhsrc::kRun)
+        st = iterate<INTEG, tracks_closest<Src>::value, has_volume<Src>::value, DRIFT>(src.params(R.f), hs, R,
+                                                                                    volume_of(src));
   }
 }
 
