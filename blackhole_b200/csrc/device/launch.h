@@ -163,9 +163,11 @@ typedef struct BhkRtParams {
   const float *cells;   // float4 (n_e, Theta_e, |B|, 0) [n_r][n_th][n_ph]
   int32_t n_r, n_th, n_ph, pad0;
   double r_min, r_max, inv_log_range;  // 1 / log(r_max / r_min)
+  double fr_scale, inv_n_ph;           // (n_r - 1) inv_log_range, 1 / n_ph
   const float *lut;     // [n_lt][n_lx] ln(j_nu / (n_e nu_B))
   int32_t n_lt, n_lx;
   double lt0, lt1, lx0, lx1;           // log Theta_e and log x ranges
+  double lt_scale, lx_scale;           // (n_lt - 1) / (lt1 - lt0), (n_lx - 1) / (lx1 - lx0)
   double nu, length_cm, ds_max, min_transmit;
 } BhkRtParams;
 
@@ -173,7 +175,7 @@ typedef struct BhkRtParams {
 int bhk_trace_rt_mixed(const BhkImageParams *p, const BhkRtParams *q, double *i_nu, double *tau, int32_t *cls,
                        int32_t *steps, unsigned long long *work_counter, void *stream);
 int bhk_trace_rt_fp64(const BhkImageParams *p, const BhkRtParams *q, double *i_nu, double *tau, int32_t *cls,
-                      int32_t *steps, unsigned long long *work_counter, int grid, int block, void *stream);
+                      int32_t *steps, unsigned long long *work_counter, void *stream);
 
 // Synthetic torus grid (grmhd.cu): modes [n_modes] of (kx, ky, kz, phase).
 // Resample packed simulation frames into the medium grid (grmhd.cu).

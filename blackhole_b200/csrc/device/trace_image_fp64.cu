@@ -282,102 +282,155 @@ __global__ void __launch_bounds__(128, 4) k_trace_batch_fp64(const __grid_consta
 
 // ---- along-ray radiative transfer -------------------------------------------
 
-// Transfer over one accepted step y0 -> y1 (derivatives k0, k1 at its ends):
-// samples at most ds_max apart in affine length, positions by cubic Hermite
-// interpolation in Mino time.
-__device__ __forceinline__ void rt_segment(const BhkImageParams &p, const BhkRtParams &q, const RayC &c,
-                                           const Yd &y0, const Yd &k0, const Yd &y1, const Yd &k1, double h,
-                                           double &I, double &T, double &tau) {
+// The samples of one accepted step y0 -> y1 (derivatives k0, k1 at its ends,
+// length h in Mino time): at most ds_max apart in affine length. 0 where the
+// step stays beyond r_max: on t in [0, 1] the cubic Hermite r(t) >= min(r0,
+// r1) - (4/27) |h| (|r0'| + |r1'|).
+__device__ __forceinline__ int rt_count(const BhkImageParams &p, const BhkRtParams &q, const Yd &y0, const Yd &k0,
+                                        const Yd &y1, const Yd &k1, double h) {
   const double rm = 0.5 * (y0.r + y1.r) + 0.125 * h * (k0.r - k1.r);
   const double um = 0.5 * (y0.u + y1.u) + 0.125 * h * (k0.u - k1.u);
   const double sig_m = rm * rm + p.a2 * um * um;
-  // a step that stays beyond r_max samples nothing: on t in [0, 1] the cubic
-  // Hermite r(t) >= min(r0, r1) - (4/27) |h| (|r0'| + |r1'|)
   const double rlow = (y0.r < y1.r ? y0.r : y1.r) - (4.0 / 27.0) * fabs(h) * (fabs(k0.r) + fabs(k1.r));
-  if (rlow > q.r_max) return;
-  double ns = ceil((sig_m * h) / q.ds_max);
+  if (rlow > q.r_max) return 0;
+  double ns = ceil(div_rn(sig_m * h, q.ds_max));
   ns = ns < 1.0 ? 1.0 : (ns > 64.0 ? 64.0 : ns);
-  const int nsub = (int)ns;
-  const double dt = h / ns;
-  for (int m = 0; m < nsub; ++m) {
-    const double t = ((double)m + 0.5) / ns;
-    const double t2 = t * t, t3 = t2 * t;
-    const double h00 = 2.0 * t3 - 3.0 * t2 + 1.0, h10 = t3 - 2.0 * t2 + t;
-    const double h01 = -2.0 * t3 + 3.0 * t2, h11 = t3 - t2;
-    const double r = h00 * y0.r + h10 * h * k0.r + h01 * y1.r + h11 * h * k1.r;
-    const double u = h00 * y0.u + h10 * h * k0.u + h01 * y1.u + h11 * h * k1.u;
-    const double psi = h00 * y0.phi + h10 * h * k0.phi + h01 * y1.phi + h11 * h * k1.phi;
-    const double dl = (r * r + p.a2 * u * u) * dt;  // affine length of the sample, M
-    double n, th, b;
-    if (!bhrt::sample(q, r, u, phi_of_psi(psi, r, p), n, th, b)) continue;
-    const double g = bhrt::redshift(p.a, r, u, c.lam);
-    if (!(g > 0.0)) continue;
-    double j, al;
-    bhrt::synchrotron(q, n, th, b, q.nu / g, j, al);
-    const double jo = g * g * j, ao = al / g;
-    const double ds = dl * q.length_cm;
-    const double ts = ao * ds;
-    const double om = (ts < 1.0e-4) ? ts * (1.0 - 0.5 * ts) : -expm1(-ts);
-    I = (ao > 0.0) ? I + T * ((jo / ao) * om) : I + T * (jo * ds);
-    T = T * (1.0 - om);
-    tau = tau + ts;
-  }
+  return (int)ns;
 }
 
-__global__ void __launch_bounds__(128) k_trace_rt_fp64(const __grid_constant__ BhkImageParams p,
-                                                       const __grid_constant__ BhkRtParams q,
-                                                       double *__restrict__ i_nu, double *__restrict__ tau_out,
-                                                       int *__restrict__ cls_out, int *__restrict__ steps_out,
-                                                       unsigned long long *__restrict__ counter) {
+using RtWarp = bhrt::WarpSamples<double>;
+
+// Leaves a step for the warp's samples.
+__device__ __forceinline__ void rt_hold(RtWarp &w, const Yd &y0, const Yd &k0, const Yd &y1, const Yd &k1, double h,
+                                        int nsub, double lam) {
+  const int l = threadIdx.x & 31;
+  w.step[0][l] = y0.r, w.step[1][l] = k0.r, w.step[2][l] = y1.r, w.step[3][l] = k1.r;
+  w.step[4][l] = y0.u, w.step[5][l] = k0.u, w.step[6][l] = y1.u, w.step[7][l] = k1.u;
+  w.step[8][l] = y0.phi, w.step[9][l] = k0.phi, w.step[10][l] = y1.phi, w.step[11][l] = k1.phi;
+  w.step[12][l] = h, w.step[13][l] = (double)nsub, w.step[14][l] = lam;
+}
+
+// Sample m of lane l's step, its position by cubic Hermite interpolation in
+// Mino time: the source term over the segment, the fraction absorbed and the
+// optical depth (all zero outside the medium).
+__device__ __forceinline__ void rt_sample(const BhkImageParams &p, const BhkRtParams &q, RtWarp &w, int l, int m,
+                                          int slot) {
+  const double h = w.step[12][l], ns = w.step[13][l];
+  const double dt = div_rn(h, ns);
+  const double t = div_rn((double)m + 0.5, ns);
+  const double t2 = t * t, t3 = t2 * t;
+  const double h00 = 2.0 * t3 - 3.0 * t2 + 1.0, h10 = t3 - 2.0 * t2 + t;
+  const double h01 = -2.0 * t3 + 3.0 * t2, h11 = t3 - t2;
+  const double r = h00 * w.step[0][l] + h10 * h * w.step[1][l] + h01 * w.step[2][l] + h11 * h * w.step[3][l];
+  const double u = h00 * w.step[4][l] + h10 * h * w.step[5][l] + h01 * w.step[6][l] + h11 * h * w.step[7][l];
+  const double psi = h00 * w.step[8][l] + h10 * h * w.step[9][l] + h01 * w.step[10][l] + h11 * h * w.step[11][l];
+  const double dl = (r * r + p.a2 * u * u) * dt;  // affine length of the sample, M
+  double src = 0.0, om = 0.0, ts = 0.0, n, th, b;
+  if (bhrt::sample(q, r, u, psi, p, n, th, b)) {
+    const double g = bhrt::redshift(p.a, r, u, w.step[14][l]);
+    if (g > 0.0) {
+      double j, al;
+      bhrt::synchrotron(q, n, th, b, div_rn(q.nu, g), j, al);
+      const double jo = g * g * j, ao = div_rn(al, g);
+      const double ds = dl * q.length_cm;
+      ts = ao * ds;
+      om = (ts < 1.0e-4) ? ts * (1.0 - 0.5 * ts) : -expm1(-ts);
+      src = (ao > 0.0) ? (jo / ao) * om : jo * ds;
+    }
+  }
+  w.res[0][slot] = src;
+  w.res[1][slot] = om;
+  w.res[2][slot] = ts;
+}
+
+// A warp traces up to `slots` rays at a time and samples the medium for all
+// of them together (bhrt::warp_samples). With fewer rays than the resident
+// lanes, slots < 32 spreads them over more warps: the steps cost the same per
+// warp, and a warp's samples fill its lanes either way.
+__global__ void __launch_bounds__(128, 3) k_trace_rt_fp64(const __grid_constant__ BhkImageParams p,
+                                                          const __grid_constant__ BhkRtParams q,
+                                                          double *__restrict__ i_nu, double *__restrict__ tau_out,
+                                                          int *__restrict__ cls_out, int *__restrict__ steps_out,
+                                                          unsigned long long *__restrict__ counter, int slots) {
+  __shared__ RtWarp warps[4];
+  RtWarp &w = warps[threadIdx.x >> 5];
   const unsigned lane = threadIdx.x & 31u;
+  const unsigned lanemask_lt = (1u << lane) - 1u;
+  const long long max_attempts = 4LL * p.max_steps + 64;
+  RayFp64 R;
+  double I = 0.0, T = 1.0, tau = 0.0;
+  int st = bhsrc::kEmpty;
+  bool exhausted = (int)lane >= slots;
+  int waited = bhsrc::kHold;
   for (;;) {
-    unsigned long long base = 0;
-    if (lane == 0) base = atomicAdd(counter, 32ull);
-    base = __shfl_sync(kFull, base, 0);
-    if (base >= (unsigned long long)p.n_pix) break;
-    const long long pix = (long long)base + lane;
-    if (pix >= p.n_pix) continue;
-    RayFp64 R;
-    init_ray(p, pix, R);
-    double I = 0.0, T = 1.0, tau = 0.0;
-    int cls = 3;
-    const long long max_attempts = 4LL * p.max_steps + 64;
-    for (;;) {
-      if (R.steps >= p.max_steps || R.attempts >= max_attempts) {
-        cls = 3;
-        break;
-      }
-      if (R.y.r <= p.r_hor) {
-        cls = 0;
-        break;
-      }
-      if (R.y.r >= p.r_esc) {
-        cls = 2;
-        break;
-      }
-      ++R.attempts;
-      const DPRes d = dp45(R.y, R.h, R.c, R.k1, p.rtol, p.atol, true);
-      if (d.err <= 1.0) {
-        ++R.steps;
-        rt_segment(p, q, R.c, R.y, R.k1, d.y5, d.k7, R.h, I, T, tau);
-        R.y = d.y5;
-        R.k1 = d.k7;
-        project(R.y, R.c);
-        R.k1.r = R.y.pr;
-        R.k1.u = R.y.pu;
-        R.h = R.h * step_factor(d.err, true);
-        if (T < q.min_transmit) {
-          cls = 4;
-          break;
+    const unsigned running = __ballot_sync(kFull, st == bhsrc::kRun);
+    const unsigned held = __ballot_sync(kFull, st != bhsrc::kRun && !(st == bhsrc::kEmpty && exhausted));
+    if (held) {
+      waited += __popc(held);
+      if (waited >= bhsrc::kHold || !running) {
+        waited = 0;
+        if (st >= 0) {
+          if (i_nu) i_nu[R.pix] = I;
+          if (tau_out) tau_out[R.pix] = tau;
+          if (cls_out) cls_out[R.pix] = st;
+          if (steps_out) steps_out[R.pix] = R.steps;
+          st = bhsrc::kEmpty;
         }
+        const unsigned need = __ballot_sync(kFull, st == bhsrc::kEmpty && !exhausted);
+        if (need) {
+          const int leader = __ffs(need) - 1;
+          unsigned long long base = 0;
+          if ((int)lane == leader) base = atomicAdd(counter, (unsigned long long)__popc(need));
+          base = __shfl_sync(kFull, base, leader);
+          if (st == bhsrc::kEmpty && !exhausted) {
+            const long long mine = (long long)(base + (unsigned long long)__popc(need & lanemask_lt));
+            if (mine < p.n_pix) {
+              init_ray(p, bhsrc::tile_pixel(mine, p.width, p.n_pix), R);
+              I = 0.0, T = 1.0, tau = 0.0;
+              st = bhsrc::kRun;
+            } else {
+              exhausted = true;
+            }
+          }
+        }
+      }
+    } else if (!running) {
+      break;
+    }
+    int nsub = 0;
+    bool acc = false;
+    if (st == bhsrc::kRun) {
+      if (R.steps >= p.max_steps || R.attempts >= max_attempts) {
+        st = 3;
+      } else if (R.y.r <= p.r_hor) {
+        st = 0;
+      } else if (R.y.r >= p.r_esc) {
+        st = 2;
       } else {
-        R.h = R.h * step_factor(d.err, false);
+        ++R.attempts;
+        const DPRes d = dp45(R.y, R.h, R.c, R.k1, p.rtol, p.atol, true);
+        acc = d.err <= 1.0;
+        if (acc) {
+          ++R.steps;
+          nsub = rt_count(p, q, R.y, R.k1, d.y5, d.k7, R.h);
+          if (nsub) rt_hold(w, R.y, R.k1, d.y5, d.k7, R.h, nsub, R.c.lam);
+          R.y = d.y5;
+          R.k1 = d.k7;
+          project(R.y, R.c);
+          R.k1.r = R.y.pr;
+          R.k1.u = R.y.pu;
+        }
+        R.h = R.h * step_factor(d.err, acc);
       }
     }
-    if (i_nu) i_nu[pix] = I;
-    if (tau_out) tau_out[pix] = tau;
-    if (cls_out) cls_out[pix] = cls;
-    if (steps_out) steps_out[pix] = R.steps;
+    bhrt::warp_samples(
+        w, nsub, [&](int l, int m, int slot) { rt_sample(p, q, w, l, m, slot); },
+        [&](int slot) {
+          I = I + T * w.res[0][slot];
+          T = T * (1.0 - w.res[1][slot]);
+          tau = tau + w.res[2][slot];
+        });
+    if (acc && T < q.min_transmit) st = 4;
   }
 }
 
@@ -456,12 +509,17 @@ extern "C" int bhk_trace_batch_fp64_occupancy(int integrator, int block, int *bl
 }
 
 extern "C" int bhk_trace_rt_fp64(const BhkImageParams *p, const BhkRtParams *q, double *i_nu, double *tau,
-                                 int32_t *cls, int32_t *steps, unsigned long long *counter, int grid, int block,
-                                 void *stream) {
+                                 int32_t *cls, int32_t *steps, unsigned long long *counter, void *stream) {
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   cudaError_t e = cudaMemsetAsync(counter, 0, sizeof(unsigned long long), s);
   if (e != cudaSuccess) return set_err(e, "work-counter reset");
-  bhk::k_trace_rt_fp64<<<grid, block, 0, s>>>(*p, *q, i_nu, tau, cls, steps, counter);
+  int dev = 0, sms = 0, per_sm = 0;
+  if ((e = cudaGetDevice(&dev)) != cudaSuccess ||
+      (e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev)) != cudaSuccess ||
+      (e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, bhk::k_trace_rt_fp64, 128, 0)) != cudaSuccess)
+    return set_err(e, "k_trace_rt_fp64 occupancy");
+  const bhrt::Slots L = bhrt::slots_for(p->n_pix, (long long)sms * per_sm);
+  bhk::k_trace_rt_fp64<<<L.grid, 128, 0, s>>>(*p, *q, i_nu, tau, cls, steps, counter, L.slots);
   e = cudaGetLastError();
   if (e != cudaSuccess) return set_err(e, "k_trace_rt_fp64 launch");
   return 0;

@@ -670,45 +670,51 @@ __global__ void __launch_bounds__(128) k_trace_batch_mixed(const __grid_constant
 // variants): positions by cubic Hermite interpolation of the accepted step,
 // at most ds_max apart in affine length; intensity and optical depth summed
 // in FP64.
-__device__ __forceinline__ void rt_segment_f(const BhkImageParams &p, const bhrt::MediumF &q, const RayCf &c,
-                                             const Yf &y0, const Yf &k0, const Yf &y1, const Yf &k1, float h,
-                                             double &I, float &T, double &tau) {
-  const float a2 = c.a2;
+// Samples of one accepted step: 0 where it stays beyond r_max (see the FP64
+// transfer).
+__device__ __forceinline__ int rt_count_f(const bhrt::MediumF &q, float a2, const Yf &y0, const Yf &k0, const Yf &y1,
+                                          const Yf &k1, float h) {
   const float rm = fmaf(0.125f * h, k0.r - k1.r, 0.5f * (y0.r + y1.r));
   const float um = fmaf(0.125f * h, k0.u - k1.u, 0.5f * (y0.u + y1.u));
-  // a step that stays beyond r_max samples nothing (see the FP64 transfer)
   const float rlow = fminf(y0.r, y1.r) - (4.0f / 27.0f) * fabsf(h) * (fabsf(k0.r) + fabsf(k1.r));
-  if (rlow > q.r_max) return;
+  if (rlow > q.r_max) return 0;
   const float sig_m = fmaf(rm, rm, a2 * um * um);
-  const float ns = fminf(fmaxf(ceilf(__fdividef(sig_m * h, q.ds_max)), 1.0f), 64.0f);
-  const int nsub = (int)ns;
-  const float dt = __fdividef(h, ns);
-  const float rp = (float)p.r_plus, rmn = (float)p.r_minus, ro = (float)p.r_obs;
-  const float gscale = c.a == 0.0f ? 0.0f : __fdividef(c.a, rp - rmn);
-  const float g_obs = __fdividef(ro - rmn, ro - rp);
-  for (int m = 0; m < nsub; ++m) {
-    const float t = __fdividef((float)m + 0.5f, ns);
-    const float t2 = t * t, t3 = t2 * t;
-    const float h00 = 2.0f * t3 - 3.0f * t2 + 1.0f, h10 = t3 - 2.0f * t2 + t;
-    const float h01 = -2.0f * t3 + 3.0f * t2, h11 = t3 - t2;
-    const float r = h00 * y0.r + h10 * h * k0.r + h01 * y1.r + h11 * h * k1.r;
-    const float u = h00 * y0.u + h10 * h * k0.u + h01 * y1.u + h11 * h * k1.u;
-    const float psi = h00 * y0.phi + h10 * h * k0.phi + h01 * y1.phi + h11 * h * k1.phi;
-    const float phi = psi + gscale * __logf(__fdividef(r - rp, r - rmn) * g_obs);  // phi = psi + a (G(r) - G(r_obs))
-    float n, th, b;
-    if (!bhrt::sample_f(q, r, u, phi, n, th, b)) continue;
-    const float g = bhrt::redshift_f(c.a, r, u, c.lam);
-    float ln_alpha, ln_s;
-    if (!bhrt::ln_emission_f(q, n, th, b, g, ln_alpha, ln_s)) continue;
-    const float dl = fmaf(r, r, a2 * u * u) * dt;  // affine length of the sample, M
-    const float ts = __expf(ln_alpha + __logf(dl) + q.ln_len);
-    const float om = ts < 1.0e-4f ? ts * (1.0f - 0.5f * ts) : -expm1f(-ts);
-    I += (double)(T * __expf(ln_s) * om);
-    T *= 1.0f - om;
-    tau += (double)ts;
-  }
+  return (int)fminf(fmaxf(ceilf(__fdividef(sig_m * h, q.ds_max)), 1.0f), 64.0f);
 }
 
+// Sample m of ns of the step y0 -> y1: e^(ln S), the fraction absorbed and the
+// optical depth (all zero outside the medium).
+__device__ __forceinline__ void rt_sample_f(const BhkImageParams &p, const bhrt::MediumF &q, float a, float a2,
+                                            float lam, const Yf &y0, const Yf &k0, const Yf &y1, const Yf &k1,
+                                            float h, float ns, int m, float &src, float &om, float &ts) {
+  const float dt = __fdividef(h, ns);
+  const float rp = (float)p.r_plus, rmn = (float)p.r_minus, ro = (float)p.r_obs;
+  const float gscale = a == 0.0f ? 0.0f : __fdividef(a, rp - rmn);
+  const float g_obs = __fdividef(ro - rmn, ro - rp);
+  const float t = __fdividef((float)m + 0.5f, ns);
+  const float t2 = t * t, t3 = t2 * t;
+  const float h00 = 2.0f * t3 - 3.0f * t2 + 1.0f, h10 = t3 - 2.0f * t2 + t;
+  const float h01 = -2.0f * t3 + 3.0f * t2, h11 = t3 - t2;
+  const float r = h00 * y0.r + h10 * h * k0.r + h01 * y1.r + h11 * h * k1.r;
+  const float u = h00 * y0.u + h10 * h * k0.u + h01 * y1.u + h11 * h * k1.u;
+  const float psi = h00 * y0.phi + h10 * h * k0.phi + h01 * y1.phi + h11 * h * k1.phi;
+  const float phi = psi + gscale * __logf(__fdividef(r - rp, r - rmn) * g_obs);  // phi = psi + a (G(r) - G(r_obs))
+  float n, th, b;
+  src = 0.0f, om = 0.0f, ts = 0.0f;
+  if (!bhrt::sample_f(q, r, u, phi, n, th, b)) return;
+  const float g = bhrt::redshift_f(a, r, u, lam);
+  float ln_alpha, ln_s;
+  if (!bhrt::ln_emission_f(q, n, th, b, g, ln_alpha, ln_s)) return;
+  const float dl = fmaf(r, r, a2 * u * u) * dt;  // affine length of the sample, M
+  ts = __expf(ln_alpha + __logf(dl) + q.ln_len);
+  om = ts < 1.0e-4f ? ts * (1.0f - 0.5f * ts) : -expm1f(-ts);
+  src = __expf(ln_s);
+}
+
+// One warp, 32 rays from the counter at a time, each lane sampling its own
+// ray: neighbours (8 x 4 tiles) reach the medium together, so their samples
+// do too. New rays only when all 32 have ended -- filled lane by lane, the
+// 512^2 frame took 3.0 to 4.0 ms, its lanes at different depths, against 2.74.
 __global__ void __launch_bounds__(128) k_trace_rt_mixed(const __grid_constant__ BhkImageParams p,
                                                         const __grid_constant__ bhrt::MediumF q,
                                                         double *__restrict__ i_nu, double *__restrict__ tau_out,
@@ -720,8 +726,8 @@ __global__ void __launch_bounds__(128) k_trace_rt_mixed(const __grid_constant__ 
     if (lane == 0) base = atomicAdd(counter, 32ull);
     base = __shfl_sync(kFull, base, 0);
     if (base >= (unsigned long long)p.n_pix) break;
-    const long long pix = (long long)base + lane;
-    if (pix >= p.n_pix) continue;
+    if ((long long)base + lane >= p.n_pix) continue;
+    const long long pix = bhsrc::tile_pixel((long long)base + lane, p.width, p.n_pix);
     RayMx R;
     init_ray(p, pix, R);
     double I = 0.0, tau = 0.0;
@@ -752,7 +758,14 @@ __global__ void __launch_bounds__(128) k_trace_rt_mixed(const __grid_constant__ 
         comp_add(R.y.phi, R.lo.phi, d.d.phi);
         R.y.pr += d.d.pr;
         R.y.pu += d.d.pu;
-        rt_segment_f(p, q, R.c, y0, k0, R.y, d.k7, h, I, T, tau);
+        const int nsub = rt_count_f(q, R.c.a2, y0, k0, R.y, d.k7, h);
+        for (int m = 0; m < nsub; ++m) {
+          float src, om, ts;
+          rt_sample_f(p, q, R.c.a, R.c.a2, R.c.lam, y0, k0, R.y, d.k7, h, (float)nsub, m, src, om, ts);
+          I += (double)(T * src * om);
+          T *= 1.0f - om;
+          tau += (double)ts;
+        }
         project(R.y, R.lo, R.cd);
         R.k1 = d.k7;
         R.k1.r = R.y.pr;
@@ -773,6 +786,105 @@ __global__ void __launch_bounds__(128) k_trace_rt_mixed(const __grid_constant__ 
   }
 }
 
+// The same for a few rays: a warp holds `slots` of them, so that every resident
+// warp has some, and samples the medium for all of them together
+// (bhrt::warp_samples). It serves images whose rays the kernel above could not
+// spread over more than one wave of warps: one ray's chain of steps and samples
+// is the time there. Frames of the a = 0.94 torus, 16^2 / 64^2 / 128^2 / 256^2:
+// 0.39 / 0.48 / 0.73 / 1.25 ms against 0.96 / 0.88 / 1.03 / 1.38; past one wave
+// the plain loop is the faster (320^2: 1.77 against 1.47 ms, 512^2: 3.6 against
+// 2.6), since 32 full lanes need no search for their samples.
+__global__ void __launch_bounds__(128) k_trace_rt_mixed_few(const __grid_constant__ BhkImageParams p,
+                                                            const __grid_constant__ bhrt::MediumF q,
+                                                            double *__restrict__ i_nu, double *__restrict__ tau_out,
+                                                            int *__restrict__ cls_out, int *__restrict__ steps_out,
+                                                            unsigned long long *__restrict__ counter, int slots) {
+  __shared__ bhrt::WarpSamples<float> warps[4];
+  bhrt::WarpSamples<float> &w = warps[threadIdx.x >> 5];
+  const int lane = threadIdx.x & 31;
+  const long long max_attempts = 4LL * p.max_steps + 64;
+  const float a = (float)p.a, a2 = (float)(p.a * p.a);
+  for (;;) {
+    unsigned long long base = 0;
+    if (lane == 0) base = atomicAdd(counter, (unsigned long long)slots);
+    base = __shfl_sync(kFull, base, 0);
+    if (base >= (unsigned long long)p.n_pix) break;
+    const bool mine = lane < slots && (long long)base + lane < p.n_pix;
+    RayMx R;
+    long long pix = 0;
+    if (mine) {
+      pix = bhsrc::tile_pixel((long long)base + lane, p.width, p.n_pix);
+      init_ray(p, pix, R);
+    }
+    double I = 0.0, tau = 0.0;
+    float T = 1.0f;
+    int st = mine ? bhsrc::kRun : bhsrc::kEmpty;
+    while (__any_sync(kFull, st == bhsrc::kRun)) {
+      int nsub = 0;
+      bool acc = false;
+      if (st == bhsrc::kRun) {
+        if (R.steps >= p.max_steps || R.attempts >= max_attempts) {
+          st = 3;
+        } else if (R.y.r <= R.r_hor) {
+          st = 0;
+        } else if (R.y.r >= R.r_esc) {
+          st = 2;
+        } else {
+          ++R.attempts;
+          const float h = R.h;
+          const DPf d = dp45(R.y, h, R.c, R.k1, R.rtol, R.atol, true);
+          acc = d.err <= 1.0f;
+          if (acc) {
+            ++R.steps;
+            const Yf y0 = R.y, k0 = R.k1;
+            comp_add(R.y.r, R.lo.r, d.d.r);
+            comp_add(R.y.u, R.lo.u, d.d.u);
+            comp_add(R.y.phi, R.lo.phi, d.d.phi);
+            R.y.pr += d.d.pr;
+            R.y.pu += d.d.pu;
+            nsub = rt_count_f(q, R.c.a2, y0, k0, R.y, d.k7, h);
+            if (nsub) {
+              w.step[0][lane] = y0.r, w.step[1][lane] = k0.r, w.step[2][lane] = R.y.r, w.step[3][lane] = d.k7.r;
+              w.step[4][lane] = y0.u, w.step[5][lane] = k0.u, w.step[6][lane] = R.y.u, w.step[7][lane] = d.k7.u;
+              w.step[8][lane] = y0.phi, w.step[9][lane] = k0.phi, w.step[10][lane] = R.y.phi;
+              w.step[11][lane] = d.k7.phi, w.step[12][lane] = h, w.step[13][lane] = (float)nsub;
+              w.step[14][lane] = R.c.lam;
+            }
+            project(R.y, R.lo, R.cd);
+            R.k1 = d.k7;
+            R.k1.r = R.y.pr;
+            R.k1.u = R.y.pu;
+          }
+          R.h = h * step_factor(d.err, acc);
+        }
+      }
+      bhrt::warp_samples(
+          w, nsub,
+          [&](int l, int m, int slot) {
+            const Yf y0{w.step[0][l], w.step[4][l], w.step[8][l], 0.0f, 0.0f};
+            const Yf k0{w.step[1][l], w.step[5][l], w.step[9][l], 0.0f, 0.0f};
+            const Yf y1{w.step[2][l], w.step[6][l], w.step[10][l], 0.0f, 0.0f};
+            const Yf k1{w.step[3][l], w.step[7][l], w.step[11][l], 0.0f, 0.0f};
+            rt_sample_f(p, q, a, a2, w.step[14][l], y0, k0, y1, k1, w.step[12][l], w.step[13][l], m, w.res[0][slot],
+                        w.res[1][slot], w.res[2][slot]);
+          },
+          [&](int slot) {
+            const float om = w.res[1][slot];
+            I += (double)(T * w.res[0][slot] * om);
+            T *= 1.0f - om;
+            tau += (double)w.res[2][slot];
+          });
+      if (acc && T < q.min_transmit) st = 4;
+    }
+    if (mine) {
+      if (i_nu) i_nu[pix] = I;
+      if (tau_out) tau_out[pix] = tau;
+      if (cls_out) cls_out[pix] = st;
+      if (steps_out) steps_out[pix] = R.steps;
+    }
+  }
+}
+
 }  // namespace bhm
 
 extern "C" int bhk_trace_rt_mixed(const BhkImageParams *p, const BhkRtParams *q, double *i_nu, double *tau,
@@ -784,9 +896,16 @@ extern "C" int bhk_trace_rt_mixed(const BhkImageParams *p, const BhkRtParams *q,
       cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess ||
       cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, bhm::k_trace_rt_mixed, 128, 0) != cudaSuccess)
     return -1;
+  const bhrt::MediumF m = bhrt::medium_f(*q);
+  if (p->n_pix <= 128LL * sms * per_sm) {  // one wave
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, bhm::k_trace_rt_mixed_few, 128, 0) != cudaSuccess)
+      return -1;
+    const bhrt::Slots L = bhrt::slots_for(p->n_pix, (long long)sms * per_sm);
+    bhm::k_trace_rt_mixed_few<<<L.grid, 128, 0, s>>>(*p, m, i_nu, tau, cls, steps, counter, L.slots);
+    return cudaGetLastError() == cudaSuccess ? 0 : -1;
+  }
   const long long need = (p->n_pix + 127) / 128;
   const int grid = (int)(need < (long long)sms * per_sm ? need : (long long)sms * per_sm);
-  const bhrt::MediumF m = bhrt::medium_f(*q);
   bhm::k_trace_rt_mixed<<<grid > 0 ? grid : 1, 128, 0, s>>>(*p, m, i_nu, tau, cls, steps, counter);
   return cudaGetLastError() == cudaSuccess ? 0 : -1;
 }

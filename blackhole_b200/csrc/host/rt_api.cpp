@@ -131,6 +131,8 @@ int bh_kerr_trace_rt(const BH_KerrScene *scene, const BH_GrmhdGrid *grid, const 
   q.r_min = grid->r_min;
   q.r_max = grid->r_max;
   q.inv_log_range = 1.0 / std::log(grid->r_max / grid->r_min);
+  q.fr_scale = q.inv_log_range * (grid->n_r - 1);
+  q.inv_n_ph = 1.0 / grid->n_phi;
   q.lut = static_cast<const float *>(lut->table);
   q.n_lt = lut->n_theta;
   q.n_lx = lut->n_x;
@@ -138,6 +140,8 @@ int bh_kerr_trace_rt(const BH_KerrScene *scene, const BH_GrmhdGrid *grid, const 
   q.lt1 = lut->log_theta_max;
   q.lx0 = lut->log_x_min;
   q.lx1 = lut->log_x_max;
+  q.lt_scale = (q.n_lt - 1) / (q.lt1 - q.lt0);
+  q.lx_scale = (q.n_lx - 1) / (q.lx1 - q.lx0);
   q.nu = r.nu_hz;
   q.length_cm = r.length_cm;
   q.ds_max = r.ds_max;
@@ -149,10 +153,7 @@ int bh_kerr_trace_rt(const BH_KerrScene *scene, const BH_GrmhdGrid *grid, const 
       return bhh_fail("bh_kerr_trace_rt: k_trace_rt_mixed launch failed");
     return 0;
   }
-  int dev = 0, sms = 0;
-  cudaGetDevice(&dev);
-  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  if (bhk_trace_rt_fp64(&p, &q, i_nu, tau, cls, steps, counter, sms * 4, 128, stream) != 0)
+  if (bhk_trace_rt_fp64(&p, &q, i_nu, tau, cls, steps, counter, stream) != 0)
     return bhh_fail(bhk_last_error());
   return 0;
 }
