@@ -32,16 +32,21 @@ __device__ __forceinline__ bool is_neg(double x) {
   return (unsigned long long)__double_as_longlong(x) > 0x8000000000000000ull;
 }
 
-// a / b.
-__device__ __forceinline__ double div_rn(double a, double b) {
+// 1 / b to 0.51 ulp, and a / b from it.
+__device__ __forceinline__ double rcp_near(double b) {
   double y;
   asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(b));
   double e = fma(-b, y, 1.0);
   e = fma(e, e, e);
-  y = fma(y, e, y);
+  return fma(y, e, y);
+}
+__device__ __forceinline__ double div_by(double a, double b, double y) {
   const double q = a * y;
   return fma(fma(-b, q, a), y, q);
 }
+
+// a / b.
+__device__ __forceinline__ double div_rn(double a, double b) { return div_by(a, b, rcp_near(b)); }
 
 // a / 5 and a / 6: y is the rounded reciprocal itself.
 __device__ __forceinline__ double div_5(double a) {
