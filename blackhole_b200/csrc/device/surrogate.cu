@@ -1,37 +1,20 @@
-// Learned transfer function: BF16 tensor-core (tcgen05) GEMM with fused
-// epilogues, input features, loss, gradient collection and Adam.
+// Learned transfer function: BF16 tensor-core (tcgen05) GEMM, fused FP16
+// inference, input features and Adam (the training step's forward and backward
+// passes are in surrogate_train.cu).
 //
-// One GEMM kernel serves every matrix product of training and inference:
-// C = A * B^T with A [M][K] and B [N][K] both K-major BF16 in HBM, tiles of
-// 128 x BN (BN = 16, 192 or 256), K in chunks of 64 streamed by TMA into a
-// 4-stage shared-memory ring (128-byte swizzle), FP32 accumulation in TMEM,
-// one thread issuing tcgen05.mma, four warps in the epilogue (one TMEM lane
-// quarter each). Backward products that reduce over the batch read
-// transposed activations (written by the forward epilogue), so every operand
-// is K-major and no transpose pass exists.
-#include <cuda.h>
-#include <cuda_bf16.h>
-#include <cuda_runtime.h>
-
+// The GEMM, C = A * B^T with A [M][K] and B [N][K] both K-major BF16 in HBM:
+// tiles of 128 x BN (BN = 16, 192 or 256), K in chunks of 64 streamed by TMA
+// into a 4-stage shared-memory ring (128-byte swizzle), FP32 accumulation in
+// TMEM, one thread issuing tcgen05.mma, four warps in the epilogue (one TMEM
+// lane quarter each).
 #include <algorithm>
 #include <cstdio>
-#include <mutex>
 
-#include "surrogate_net.h"
-#include "umma.cuh"
+#include "surrogate_dev.cuh"
 
 namespace {
 
-constexpr int kBM = 128;
-constexpr int kBK = 64;
 constexpr int kStages = 4;
-// Waits on other warps' progress run out after the caller's limit (default
-// 2 s; bh_surrogate_set_wait_limit) and record an error code. Work this
-// thread itself started (TMA loads, MMAs) is then drained with a fixed limit
-// before TMEM is freed and the CTA exits: it completes on its own.
-constexpr uint64_t kDrainNs = 1000000000ull;
-
-enum : int { kErrProducer = 11, kErrMma = 12, kErrDone = 13 };
 
 template <int BN>
 struct GemmCfg {
@@ -43,55 +26,6 @@ struct GemmCfg {
   static_assert(kStage % 1024 == 0, "stage buffers must stay 1024-byte aligned");
   static_assert(BN % 16 == 0 && BN >= 16 && BN <= 256, "UMMA N for M = 128");
 };
-
-__device__ __forceinline__ float tanh_approx(float x) {
-  float r;
-  asm("tanh.approx.f32 %0, %1;" : "=f"(r) : "f"(x));
-  return r;
-}
-
-// SiLU(y) = y sigmoid(y) with sigmoid(y) = (1 + tanh(y/2)) / 2: one MUFU
-// operation per element (training and inference use the same form).
-__device__ __forceinline__ float silu(float y) {
-  const float h = 0.5f * y;
-  return fmaf(h, tanh_approx(h), h);
-}
-
-__device__ __forceinline__ float silu_grad(float y) {
-  const float s = fmaf(0.5f, tanh_approx(0.5f * y), 0.5f);
-  return s * (1.0f + y * (1.0f - s));
-}
-
-__device__ __forceinline__ uint32_t pack_bf16(float lo, float hi) {
-  const __nv_bfloat162 h = __floats2bfloat162_rn(lo, hi);
-  return *reinterpret_cast<const uint32_t*>(&h);
-}
-
-__device__ __forceinline__ uint32_t pack_f16(float lo, float hi) {
-  uint32_t r;
-  asm("cvt.rn.f16x2.f32 %0, %1, %2;" : "=r"(r) : "f"(hi), "f"(lo));
-  return r;
-}
-
-// SiLU of two pre-activations given as halves hy = y / 2 (FP32), returned as
-// packed FP16: hy (1 + tanh hy) = y sigmoid(y), with one tanh.approx.f16x2
-// (one MUFU operation for both) and one f16x2 FMA. The activation is the next
-// layer's FP16 operand, so nothing is unpacked; FP16 keeps 11 significant
-// bits, as many as the MUFU tanh delivers.
-__device__ __forceinline__ uint32_t silu_f16x2(float hy_lo, float hy_hi) {
-  const uint32_t h = pack_f16(hy_lo, hy_hi);
-  uint32_t t, r;
-  asm("tanh.approx.f16x2 %0, %1;" : "=r"(t) : "r"(h));
-  asm("fma.rn.f16x2 %0, %1, %2, %2;" : "=r"(r) : "r"(t), "r"(h));
-  return r;
-}
-
-__device__ __forceinline__ void store_bf16x16(__nv_bfloat16* dst, const float (&h)[16]) {
-  uint4* p = reinterpret_cast<uint4*>(dst);
-  p[0] = make_uint4(pack_bf16(h[0], h[1]), pack_bf16(h[2], h[3]), pack_bf16(h[4], h[5]), pack_bf16(h[6], h[7]));
-  p[1] = make_uint4(pack_bf16(h[8], h[9]), pack_bf16(h[10], h[11]), pack_bf16(h[12], h[13]),
-           pack_bf16(h[14], h[15]));
-}
 
 __device__ __forceinline__ void store_f32x16(float* dst, const float (&h)[16]) {
   float4* p = reinterpret_cast<float4*>(dst);
@@ -108,69 +42,6 @@ struct EpiF32 {
   __device__ void operator()(int64_t row, int col, const float (&v)[16], int split) const {
     if (row >= M) return;
     store_f32x16(C + ((int64_t)split * M + row) * N + col, v);
-  }
-};
-
-struct EpiHidden {
-  const float* bias;
-  __nv_bfloat16* H;
-  __nv_bfloat16* HT;
-  float* Y;
-  int64_t M;
-  int N;
-  int64_t ldt;
-  __device__ void operator()(int64_t row, int col, const float (&v)[16], int) const {
-    if (row >= M) return;
-    float y[16], h[16];
-#pragma unroll
-    for (int i = 0; i < 16; ++i) {
-      y[i] = v[i] + __ldg(bias + col + i);
-      h[i] = silu(y[i]);
-    }
-    if (Y) store_f32x16(Y + row * N + col, y);
-    store_bf16x16(H + row * N + col, h);
-    if (HT) {
-#pragma unroll
-      for (int i = 0; i < 16; ++i) HT[(int64_t)(col + i) * ldt + row] = __float2bfloat16_rn(h[i]);
-    }
-  }
-};
-
-struct EpiHead {
-  const float* bias;
-  float* out;
-  int64_t M;
-  __device__ void operator()(int64_t row, int col, const float (&v)[16], int) const {
-    if (row >= M) return;
-    float o[16];
-#pragma unroll
-    for (int i = 0; i < 16; ++i) o[i] = v[i] + __ldg(bias + col + i);
-    store_f32x16(out + row * BHS_HEAD + col, o);
-  }
-};
-
-struct EpiBackward {
-  const float* Y;
-  __nv_bfloat16* dY;
-  __nv_bfloat16* dYT;
-  int64_t M;
-  int N;
-  int64_t ldt;
-  __device__ void operator()(int64_t row, int col, const float (&v)[16], int) const {
-    if (row >= M) return;
-    const float4* yp = reinterpret_cast<const float4*>(Y + row * N + col);
-    float d[16];
-#pragma unroll
-    for (int q = 0; q < 4; ++q) {
-      const float4 y = yp[q];
-      d[4 * q + 0] = v[4 * q + 0] * silu_grad(y.x);
-      d[4 * q + 1] = v[4 * q + 1] * silu_grad(y.y);
-      d[4 * q + 2] = v[4 * q + 2] * silu_grad(y.z);
-      d[4 * q + 3] = v[4 * q + 3] * silu_grad(y.w);
-    }
-    store_bf16x16(dY + row * N + col, d);
-#pragma unroll
-    for (int i = 0; i < 16; ++i) dYT[(int64_t)(col + i) * ldt + row] = __float2bfloat16_rn(d[i]);
   }
 };
 
@@ -296,51 +167,6 @@ __global__ void __launch_bounds__(128, 1)
 
 // ---- features ----------------------------------------------------------------
 
-// 2^(k/3), k = 0..15: Fourier frequencies in units of pi.
-__constant__ float c_freq[BHS_FOURIER] = {1.0f,
-                     1.2599210498948732f,
-                     1.5874010519681994f,
-                     2.0f,
-                     2.5198420997897464f,
-                     3.1748021039363987f,
-                     4.0f,
-                     5.0396841995794928f,
-                     6.3496042078727974f,
-                     8.0f,
-                     10.079368399158986f,
-                     12.699208415745595f,
-                     16.0f,
-                     20.158736798317971f,
-                     25.398416831491190f,
-                     32.0f};
-
-// Fourier features of one input x: (sin, cos)(pi 2^(k/3) x), k = 0..15,
-// interleaved. Frequencies k = 0, 1, 2 come from sincospif; every further
-// one doubles the angle of the one three below (sin 2t = 2 s c,
-// cos 2t = (c - s)(c + s)), which keeps the absolute error near 1e-6.
-__device__ __forceinline__ void fourier_pairs(float x, float (&v)[2 * BHS_FOURIER]) {
-#pragma unroll
-  for (int k = 0; k < 3; ++k) sincospif(c_freq[k] * x, &v[2 * k], &v[2 * k + 1]);
-#pragma unroll
-  for (int k = 3; k < BHS_FOURIER; ++k) {
-    const float sn = v[2 * (k - 3)], cs = v[2 * (k - 3) + 1];
-    v[2 * k] = 2.0f * sn * cs;
-    v[2 * k + 1] = (cs - sn) * (cs + sn);
-  }
-}
-
-// The network's scaled inputs: x = (alpha/15, beta/15, 2a - 1, 2 cos theta - 1)
-// and the constants of motion lambda/15, eta/225.
-__device__ __forceinline__ void scaled_inputs(float4 q, float (&x)[4], float& lam, float& eta) {
-  x[0] = q.x * (1.0f / 15.0f);
-  x[1] = q.y * (1.0f / 15.0f);
-  x[2] = 2.0f * q.z - 1.0f;
-  x[3] = 2.0f * q.w - 1.0f;
-  const float st = sqrtf(fmaxf(0.0f, 1.0f - q.w * q.w));
-  lam = -q.x * st * (1.0f / 15.0f);
-  eta = (q.y * q.y + (q.x * q.x - q.z * q.z) * q.w * q.w) * (1.0f / 225.0f);
-}
-
 // The network's input features of one ray: columns 32 d + 2k, 32 d + 2k + 1
 // = Fourier pair k of input d (d = 0..3), columns 128..133 = the scaled
 // inputs and constants of motion, 134..191 zero.
@@ -362,8 +188,7 @@ __device__ __forceinline__ void ray_features(float4 q, float (&f)[BHS_FEATURES_U
   f[133] = eta;
 }
 
-__global__ void k_features(const float* __restrict__ in, int64_t n, __nv_bfloat16* __restrict__ F,
-                           __nv_bfloat16* __restrict__ FT, int64_t ldt) {
+__global__ void k_features(const float* __restrict__ in, int64_t n, __nv_bfloat16* __restrict__ F) {
   const int64_t r = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (r >= n) return;
   float f[BHS_FEATURES_USED];
@@ -379,72 +204,6 @@ __global__ void k_features(const float* __restrict__ in, int64_t n, __nv_bfloat1
     }
     row[u] = make_uint4(pack_bf16(h[0], h[1]), pack_bf16(h[2], h[3]), pack_bf16(h[4], h[5]),
               pack_bf16(h[6], h[7]));
-  }
-  if (FT) {
-#pragma unroll
-    for (int j = 0; j < BHS_FEATURES; ++j)
-      FT[(int64_t)j * ldt + r] = __float2bfloat16_rn(j < BHS_FEATURES_USED ? f[j] : 0.0f);
-  }
-}
-
-// ---- loss ------------------------------------------------------------------
-
-// Regression output j (head column 3 + j, target column 2 + j) counts when:
-// j = 0..2, 6: a first disk hit; j = 3..5: a second hit; j = 7..9: escaped.
-__device__ __forceinline__ bool reg_mask(int j, int cls, int nc) {
-  if (j <= 2 || j == 6) return nc >= 1;
-  if (j <= 5) return nc >= 2;
-  return cls == 2;
-}
-
-__global__ void k_loss(const float* __restrict__ out, const float* __restrict__ tg, int64_t B,
-            __nv_bfloat16* __restrict__ dout, __nv_bfloat16* __restrict__ dout_t,
-            float* __restrict__ loss) {
-  const int64_t r = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  float acc[4] = {0.f, 0.f, 0.f, 0.f};
-  if (r < B) {
-    const float* o = out + r * BHS_HEAD;
-    const float* t = tg + r * BHS_TARGETS;
-    const int cls = (int)t[0];
-    const int nc = (int)t[1];
-    const float invB = 1.0f / (float)B;
-    float d[BHS_HEAD];
-#pragma unroll
-    for (int i = 0; i < BHS_HEAD; ++i) d[i] = 0.0f;
-    if (cls >= 0) {
-      const float m = fmaxf(o[0], fmaxf(o[1], o[2]));
-      const float e0 = expf(o[0] - m), e1 = expf(o[1] - m), e2 = expf(o[2] - m);
-      const float Z = e0 + e1 + e2;
-      acc[0] = -(o[cls] - m - logf(Z));
-      d[0] = (e0 / Z - (cls == 0 ? 1.f : 0.f)) * invB;
-      d[1] = (e1 / Z - (cls == 1 ? 1.f : 0.f)) * invB;
-      d[2] = (e2 / Z - (cls == 2 ? 1.f : 0.f)) * invB;
-      const int am = (o[1] > o[0] && o[1] >= o[2]) ? 1 : ((o[2] > o[0] && o[2] > o[1]) ? 2 : 0);
-      acc[2] = am == cls ? 1.f : 0.f;
-      acc[3] = 1.f;
-    }
-#pragma unroll
-    for (int j = 0; j < 10; ++j) {
-      if (reg_mask(j, cls, nc)) {
-        const float e = o[3 + j] - t[2 + j];
-        acc[1] += e * e;
-        d[3 + j] = 2.0f * e * invB;
-      }
-    }
-    uint4* row = reinterpret_cast<uint4*>(dout + r * BHS_HEAD_PAD);
-    row[0] = make_uint4(pack_bf16(d[0], d[1]), pack_bf16(d[2], d[3]), pack_bf16(d[4], d[5]),
-              pack_bf16(d[6], d[7]));
-    row[1] = make_uint4(pack_bf16(d[8], d[9]), pack_bf16(d[10], d[11]), pack_bf16(d[12], d[13]),
-              pack_bf16(d[14], d[15]));
-#pragma unroll
-    for (int i = 0; i < BHS_HEAD; ++i) dout_t[(int64_t)i * B + r] = __float2bfloat16_rn(d[i]);
-  }
-#pragma unroll
-  for (int c = 0; c < 4; ++c) {
-    float v = acc[c];
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-    if ((threadIdx.x & 31) == 0 && v != 0.0f) atomicAdd(loss + c, v);
   }
 }
 
@@ -469,11 +228,6 @@ __global__ void k_loss(const float* __restrict__ out, const float* __restrict__ 
 #define BHS_EPI_PIPE 1
 #endif
 
-// K steps (16 columns each) of layer 0's last 64-column chunk that can hold a
-// nonzero term: features 128..133 lie in the first.
-constexpr int kFeatTailSteps = (BHS_FEATURES_USED - 128 + 15) / 16;
-static_assert(BHS_FEATURES_USED > 128 && BHS_FEATURES_USED <= 144, "feature tail within one K step");
-
 constexpr int kInfThreads = 576;  // 2 control warps + 2 slots x 8 epilogue warps
 constexpr int kEpiThreads = 256;  // epilogue threads per slot
 constexpr int kInfRing = 3;
@@ -495,15 +249,6 @@ struct InferArgs {
   uint64_t wait_ns;  // limit of each wait on another warp's progress
   float bias[kBiasCount];  // layers 0..3 (256 each, halved: b / 2), then the head (16, as is)
 };
-
-__device__ __forceinline__ int layer_chunks(int l) { return (l == 0 ? BHS_FEATURES : BHS_HIDDEN) / kBK; }
-
-// One 16-byte unit (8 BF16, unit j of 8 in a 64-column chunk) of row r of a
-// K-major 128-byte-swizzled tile chunk at shared address cb.
-__device__ __forceinline__ void st_unit(uint32_t cb, int r, int j, uint32_t a, uint32_t b, uint32_t c, uint32_t d) {
-  const uint32_t addr = cb + (uint32_t)r * 128u + ((uint32_t)(j ^ (r & 7)) << 4);
-  asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(addr), "r"(a), "r"(b), "r"(c), "r"(d) : "memory");
-}
 
 __global__ void __launch_bounds__(kInfThreads, 1)
     k_mlp_infer(const __grid_constant__ CUtensorMap w0, const __grid_constant__ CUtensorMap w1,
@@ -732,18 +477,14 @@ __global__ void __launch_bounds__(kInfThreads, 1)
   if (warp == 0) umma::tmem_dealloc(tmem, 512);
 }
 
-// ---- gradients and optimiser -------------------------------------------------
+// ---- optimiser -------------------------------------------------
 
-struct Ptr5 {
-  const void* p[BHS_LAYERS];
-};
 struct MutPtr5 {
   void* p[BHS_LAYERS];
 };
 struct LayerTable {
   int k[BHS_LAYERS], n[BHS_LAYERS];
-  int64_t w_off[BHS_LAYERS], b_off[BHS_LAYERS];
-  int splits[BHS_LAYERS];
+  int64_t w_off[BHS_LAYERS];
 };
 
 LayerTable make_table() {
@@ -752,52 +493,8 @@ LayerTable make_table() {
     t.k[l] = bhs_layer_k(l);
     t.n[l] = bhs_layer_n(l);
     t.w_off[l] = bhs_weight_offset(l);
-    t.b_off[l] = bhs_bias_offset(l);
   }
   return t;
-}
-
-// One block per (layer, output unit): grad[b_l][n] = sum_b dY^T[n][b].
-__global__ void k_bias_grads(Ptr5 dyt, LayerTable t, int64_t B, float* __restrict__ grad) {
-  int u = blockIdx.x, l = 0;
-  while (l < BHS_LAYERS - 1 && u >= t.n[l]) u -= t.n[l++];
-  const __nv_bfloat16* row = static_cast<const __nv_bfloat16*>(dyt.p[l]) + (int64_t)u * B;
-  float s = 0.0f;
-  for (int64_t b = threadIdx.x; b < B; b += blockDim.x) s += __bfloat162float(row[b]);
-  __shared__ float red[32];
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = s;
-  __syncthreads();
-  if (threadIdx.x < 32) {
-    s = threadIdx.x < (blockDim.x >> 5) ? red[threadIdx.x] : 0.0f;
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-    if (threadIdx.x == 0) grad[t.b_off[l] + u] = s;
-  }
-}
-
-// grad[W_l][n][k] = sum_s P_l[s][n][k]; layer 4's partials are [s][k][n].
-__global__ void k_collect_dw(Ptr5 parts, LayerTable t, float* __restrict__ grad) {
-  const int64_t total = t.b_off[BHS_LAYERS - 1];
-  for (int64_t p = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; p < total;
-     p += (int64_t)gridDim.x * blockDim.x) {
-    int l = BHS_LAYERS - 1;
-    while (l > 0 && p < t.w_off[l]) --l;
-    const int64_t q = p - t.w_off[l];
-    if (q >= (int64_t)t.n[l] * t.k[l]) continue;  // a bias slot
-    const int n = (int)(q / t.k[l]), k = (int)(q % t.k[l]);
-    const float* P = static_cast<const float*>(parts.p[l]);
-    float s = 0.0f;
-    if (l == BHS_LAYERS - 1) {
-      const int64_t stride = (int64_t)t.k[l] * t.n[l];
-      for (int sp = 0; sp < t.splits[l]; ++sp) s += P[sp * stride + (int64_t)k * t.n[l] + n];
-    } else {
-      const int64_t stride = (int64_t)t.n[l] * t.k[l];
-      for (int sp = 0; sp < t.splits[l]; ++sp) s += P[sp * stride + q];
-    }
-    grad[p] = s;
-  }
 }
 
 __device__ __forceinline__ void write_bf16_weight(const LayerTable& t, const MutPtr5& wb, const MutPtr5& wt,
@@ -894,39 +591,6 @@ __global__ void k_grid_inputs(double spin, double ct, double a0, double da, doub
 
 // ---- host side: tensor maps and launchers -----------------------------------
 
-typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
-                 const cuuint64_t*, const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave,
-                 CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
-
-EncodeTiledFn encode_fn() {
-  static EncodeTiledFn fn = nullptr;
-  static std::once_flag once;
-  std::call_once(once, [] {
-    void* p = nullptr;
-    cudaDriverEntryPointQueryResult q{};
-    if (cudaGetDriverEntryPointByVersion("cuTensorMapEncodeTiled", &p, 12000, cudaEnableDefault, &q) ==
-        cudaSuccess &&
-      q == cudaDriverEntryPointSuccess)
-      fn = reinterpret_cast<EncodeTiledFn>(p);
-  });
-  return fn;
-}
-
-// K-major 16-bit matrix [rows][ld] (K valid columns), box {64, box_rows}, 128-byte swizzle.
-bool make_map(CUtensorMap* m, const void* base, int64_t rows, int K, int ld, int box_rows,
-              CUtensorMapDataType type = CU_TENSOR_MAP_DATA_TYPE_BFLOAT16) {
-  EncodeTiledFn fn = encode_fn();
-  if (!fn) return false;
-  if ((reinterpret_cast<uintptr_t>(base) & 15u) != 0 || (ld * 2) % 16 != 0) return false;
-  const cuuint64_t dims[2] = {(cuuint64_t)K, (cuuint64_t)rows};
-  const cuuint64_t strides[1] = {(cuuint64_t)ld * 2};
-  const cuuint32_t box[2] = {(cuuint32_t)kBK, (cuuint32_t)box_rows};
-  const cuuint32_t es[2] = {1, 1};
-  return fn(m, type, 2, const_cast<void*>(base), dims, strides, box, es,
-       CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
-       CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
-}
-
 template <int BN, class Epi>
 int launch_tile(const BhsGemm* g, const Epi& epi, int* err, cudaStream_t st) {
   using Cfg = GemmCfg<BN>;
@@ -952,24 +616,7 @@ int launch_tile(const BhsGemm* g, const Epi& epi, int* err, cudaStream_t st) {
 
 template <int BN>
 int launch_bn(const BhsGemm* g, int* err, cudaStream_t st) {
-  switch (g->epilogue) {
-    case BHS_EPI_F32:
-      return launch_tile<BN>(g, EpiF32{static_cast<float*>(g->out), g->M, g->N}, err, st);
-    case BHS_EPI_HIDDEN:
-      return launch_tile<BN>(g,
-                  EpiHidden{g->bias, static_cast<__nv_bfloat16*>(g->out),
-                       static_cast<__nv_bfloat16*>(g->out_t), g->y_out, g->M, g->N, g->ld_t},
-                  err, st);
-    case BHS_EPI_HEAD:
-      return launch_tile<BN>(g, EpiHead{g->bias, static_cast<float*>(g->out), g->M}, err, st);
-    case BHS_EPI_BACKWARD:
-      return launch_tile<BN>(g,
-                  EpiBackward{g->Y, static_cast<__nv_bfloat16*>(g->out),
-                        static_cast<__nv_bfloat16*>(g->out_t), g->M, g->N, g->ld_t},
-                  err, st);
-    default:
-      return -1;
-  }
+  return launch_tile<BN>(g, EpiF32{static_cast<float*>(g->out), g->M, g->N}, err, st);
 }
 
 int blocks_for(int64_t n, int threads) { return (int)((n + threads - 1) / threads); }
@@ -1012,7 +659,6 @@ extern "C" int bhs_launch_infer(const __half* const* wh, const float* host_bias,
 extern "C" int bhs_launch_gemm(const BhsGemm* g, int* d_err, cudaStream_t stream) {
   if (g->M <= 0) return 0;
   if (g->K <= 0 || g->lda % 8 || g->ldb % 8) return -1;
-  if (g->epilogue == BHS_EPI_HEAD && g->N != BHS_HEAD) return -1;
   if (g->N == 256) return launch_bn<256>(g, d_err, stream);
   if (g->N == 192) return launch_bn<192>(g, d_err, stream);
   if (g->N == 16) return launch_bn<16>(g, d_err, stream);
@@ -1020,38 +666,9 @@ extern "C" int bhs_launch_gemm(const BhsGemm* g, int* d_err, cudaStream_t stream
   return -1;
 }
 
-extern "C" int bhs_launch_features(const float* inputs, int64_t n, __nv_bfloat16* F, __nv_bfloat16* FT,
-                  int64_t ld_t, cudaStream_t stream) {
+extern "C" int bhs_launch_features(const float* inputs, int64_t n, __nv_bfloat16* F, cudaStream_t stream) {
   if (n <= 0) return 0;
-  k_features<<<blocks_for(n, 128), 128, 0, stream>>>(inputs, n, F, FT, ld_t);
-  return cudaGetLastError() == cudaSuccess ? 0 : -1;
-}
-
-extern "C" int bhs_launch_loss(const float* out, const float* targets, int64_t B, __nv_bfloat16* dout,
-                __nv_bfloat16* dout_t, float* loss, cudaStream_t stream) {
-  if (B <= 0) return 0;
-  k_loss<<<blocks_for(B, 256), 256, 0, stream>>>(out, targets, B, dout, dout_t, loss);
-  return cudaGetLastError() == cudaSuccess ? 0 : -1;
-}
-
-extern "C" int bhs_launch_bias_grads(const __nv_bfloat16* const* dyt, int64_t B, float* grad, cudaStream_t stream) {
-  Ptr5 p{};
-  for (int l = 0; l < BHS_LAYERS; ++l) p.p[l] = dyt[l];
-  int blocks = 0;
-  for (int l = 0; l < BHS_LAYERS; ++l) blocks += bhs_layer_n(l);
-  k_bias_grads<<<blocks, 256, 0, stream>>>(p, make_table(), B, grad);
-  return cudaGetLastError() == cudaSuccess ? 0 : -1;
-}
-
-extern "C" int bhs_launch_collect_dw(const float* const* partials, const int* splits, float* grad,
-                   cudaStream_t stream) {
-  Ptr5 p{};
-  LayerTable t = make_table();
-  for (int l = 0; l < BHS_LAYERS; ++l) {
-    p.p[l] = partials[l];
-    t.splits[l] = splits[l];
-  }
-  k_collect_dw<<<592, 256, 0, stream>>>(p, t, grad);
+  k_features<<<blocks_for(n, 128), 128, 0, stream>>>(inputs, n, F);
   return cudaGetLastError() == cudaSuccess ? 0 : -1;
 }
 

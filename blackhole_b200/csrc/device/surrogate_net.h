@@ -46,14 +46,8 @@ static inline int64_t bhs_bias_offset(int l) {
 }
 static inline int64_t bhs_param_count(void) { return bhs_weight_offset(BHS_LAYERS); }
 
-// Epilogues of the BF16 GEMM C = A * B^T (A [M][K], B [N][K], both K-major).
-enum BhsEpilogue {
-  BHS_EPI_F32 = 0,     // C (FP32) [split][M][N] -- split-K partial sums
-  BHS_EPI_HIDDEN = 1,  // H = SiLU(C + b) -> BF16 [M][N]; optional H^T [N][ld_t], pre-activation Y (FP32)
-  BHS_EPI_HEAD = 2,    // out = C + b -> FP32 [M][16]
-  BHS_EPI_BACKWARD = 3 // dY = C * SiLU'(Y) -> BF16 [M][N] and dY^T [N][ld_t]
-};
-
+// BF16 GEMM C = A * B^T (A [M][K], B [N][K], both K-major), C FP32
+// [split][M][N]: split-K partial sums.
 typedef struct BhsGemm {
   const void* A;  // BF16 [M][lda]
   const void* B;  // BF16 [N][ldb]
@@ -61,17 +55,41 @@ typedef struct BhsGemm {
   int N, K;
   int lda, ldb;
   int kchunks_per_split;  // 64-wide K chunks per split (0 = all)
-  int epilogue;
-  const float* bias;      // HIDDEN, HEAD
-  const float* Y;         // BACKWARD: pre-activation [M][N]
-  void* out;              // F32 partials, BF16 H / dY, or FP32 head
-  void* out_t;            // BF16 transposed copy [N][ld_t] (optional)
-  float* y_out;           // HIDDEN: pre-activation (optional)
-  int64_t ld_t;
+  void* out;
   uint64_t wait_ns;       // limit of each wait on another warp (>= 1)
 } BhsGemm;
 
 int bhs_launch_gemm(const BhsGemm* g, int* d_err, cudaStream_t stream);
+
+// Buffers of one training handle (device). Rows are rays; batch B, a multiple
+// of 128, at most the batch the buffers were made for.
+typedef struct BhsTrainBuffers {
+  const float* params;                  // FP32 master parameters
+  __nv_bfloat16* wb[BHS_LAYERS];        // W_l [N][K]
+  __nv_bfloat16* wt[BHS_LAYERS];        // W_l^T [K][N] (l >= 1; layer 4: [256][64], zero beyond 16)
+  __nv_bfloat16* F;                     // features [B][192]
+  __nv_bfloat16* h[4];                  // activations [B][256]
+  __nv_bfloat16* dy[4];                 // loss gradient of the pre-activations [B][256]
+  __nv_bfloat16* dout;                  // ... of the head outputs [B][64], zero beyond 16
+  float* y[3];                          // FP32 pre-activations of layers 0..2, in the training kernel's own layout
+  float* part[BHS_LAYERS];              // weight-gradient partials, bhs_train_splits(l, B) x 256 K_l (layer 4: 256 x 16)
+  float* bias_part;                     // [B / 32][1040] bias-gradient partials
+} BhsTrainBuffers;
+
+// The tensor maps of a batch size (opaque): made once per (buffers, batch).
+typedef struct BhsTrainPlan {
+  int64_t batch;
+  alignas(64) unsigned char maps[24][128];
+} BhsTrainPlan;
+
+int bhs_train_splits(int layer, int64_t batch);
+int bhs_train_plan(const BhsTrainBuffers* b, int64_t batch, BhsTrainPlan* plan);
+
+// Forward pass, loss and backward pass of one batch: grad (every parameter)
+// and loss[0..3] += (cross entropy, regression, correct class count, counted
+// rows). inputs [B][4], targets [B][16].
+int bhs_launch_train(const BhsTrainBuffers* b, const BhsTrainPlan* plan, const float* inputs, const float* targets,
+                     float* grad, float* loss, int* d_err, uint64_t wait_ns, cudaStream_t stream);
 
 // Fused inference of n rows (features, 4 hidden layers, head) in one
 // persistent launch: head [n][16] = network(inputs [n][4]), FP16 weights wh
@@ -85,20 +103,7 @@ int bhs_launch_infer(const __half* const* wh, const float* host_bias, const floa
 int bhs_launch_refresh_f16(const float* params, __half* const* wh, cudaStream_t stream);
 
 // Features of n rays from inputs [n][4] = (alpha, beta, spin, cos theta_obs).
-int bhs_launch_features(const float* inputs, int64_t n, __nv_bfloat16* F, __nv_bfloat16* FT, int64_t ld_t,
-            cudaStream_t stream);
-
-// Loss and its gradient w.r.t. the head outputs. out [B][16], targets [B][16].
-// dout [B][64] (columns >= 16 left untouched), dout_t [16][B]. loss[0..3] +=
-// (cross entropy, regression, correct class count, counted rows).
-int bhs_launch_loss(const float* out, const float* targets, int64_t B, __nv_bfloat16* dout,
-          __nv_bfloat16* dout_t, float* loss, cudaStream_t stream);
-
-// grad[bias of layer l][n] = sum_b dY_l^T[n][b] for all layers at once.
-int bhs_launch_bias_grads(const __nv_bfloat16* const* dyt, int64_t B, float* grad, cudaStream_t stream);
-
-// grad[W_l] = sum over splits of the partials (layer 4 stored transposed).
-int bhs_launch_collect_dw(const float* const* partials, const int* splits, float* grad, cudaStream_t stream);
+int bhs_launch_features(const float* inputs, int64_t n, __nv_bfloat16* F, cudaStream_t stream);
 
 // Adam on the master parameters; refreshes the BF16 weights W_l [N][K] and
 // their transposes W_l^T [K][N] (layer 4: [256][64], zero beyond 16).

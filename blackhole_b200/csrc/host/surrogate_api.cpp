@@ -34,16 +34,9 @@ struct BH_Surrogate {
   int64_t step = 0;
   std::vector<void *> allocs;
   float *w = nullptr, *m = nullptr, *v = nullptr, *grad = nullptr;
-  bf16 *wb[BHS_LAYERS] = {}, *wt[BHS_LAYERS] = {};
   __half *wh[BHS_LAYERS] = {};  // FP16 inference copies, refreshed with the host biases
-  // training activations, batch-major [B][.] and transposed [.][B]
-  bf16 *F = nullptr, *FT = nullptr;
-  bf16 *h[4] = {}, *ht[4] = {};
-  float *y[4] = {};
-  float *out = nullptr;
-  bf16 *dout = nullptr, *dout_t = nullptr;
-  bf16 *dy[4] = {}, *dyt[4] = {};
-  float *part[BHS_LAYERS] = {};
+  BhsTrainBuffers tr{};         // BF16 weights, training activations and partial sums
+  BhsTrainPlan plan{};          // tensor maps of the last batch size (batch 0: none)
   float *loss = nullptr;
   int *err = nullptr;
   // renderer buffers (grow-only)
@@ -80,8 +73,6 @@ struct BH_Surrogate {
 
 namespace {
 
-constexpr int kDwChunks = 8;  // 64-row K chunks per split of the batch reduction
-
 int fail_msg(const char *fmt, ...) __attribute__((format(printf, 1, 2)));
 int fail_msg(const char *fmt, ...) {
   char buf[512];
@@ -104,11 +95,6 @@ int alloc(BH_Surrogate *s, T **p, size_t count, const char *what) {
   s->allocs.push_back(q);
   *p = static_cast<T *>(q);
   return 0;
-}
-
-int64_t dw_splits(int64_t batch) {
-  const int64_t chunks = (batch + 63) / 64;
-  return (chunks + kDwChunks - 1) / kDwChunks;
 }
 
 uint64_t splitmix(uint64_t &x) {
@@ -138,99 +124,25 @@ std::vector<float> init_params(uint64_t seed) {
 }
 
 int refresh(BH_Surrogate *s, cudaStream_t st) {
-  if (bhs_launch_refresh_bf16(s->w, s->wb, s->wt, st) != 0) return fail_msg("surrogate: weight refresh launch failed");
+  if (bhs_launch_refresh_bf16(s->w, s->tr.wb, s->tr.wt, st) != 0) return fail_msg("surrogate: weight refresh launch failed");
   return 0;
 }
 
-int gemm(BH_Surrogate *s, const BhsGemm &g0, cudaStream_t st, const char *what) {
-  BhsGemm g = g0;
-  g.wait_ns = s->wait_ns;
-  if (bhs_launch_gemm(&g, s->err, st) != 0)
-    return fail_msg("surrogate: GEMM launch failed (%s: M=%lld N=%d K=%d)", what, static_cast<long long>(g.M), g.N,
-                    g.K);
-  return 0;
-}
-
-BhsGemm make_gemm(const void *A, int lda, const void *B, int ldb, int64_t M, int N, int K, int epi) {
-  BhsGemm g{};
-  g.A = A;
-  g.B = B;
-  g.M = M;
-  g.N = N;
-  g.K = K;
-  g.lda = lda;
-  g.ldb = ldb;
-  g.epilogue = epi;
-  return g;
-}
-
-// Forward (saving what backward needs), loss, backward, gradient collection.
-int forward_backward(BH_Surrogate *s, const float *inputs, const float *targets, int64_t B, float *loss4,
+// Forward pass, loss, backward pass and gradient collection into grad; loss4
+// (NULL: not wanted) receives the batch's sums.
+int forward_backward(BH_Surrogate *s, const float *inputs, const float *targets, int64_t B, float *grad, float *loss4,
                      cudaStream_t st) {
   if (B <= 0 || B > s->max_batch || B % 128 != 0)
     return fail_msg("surrogate: batch %lld must be a positive multiple of 128 up to %lld", static_cast<long long>(B),
                     static_cast<long long>(s->max_batch));
-  if (int rc = cuda_check(cudaMemsetAsync(s->loss, 0, 4 * sizeof(float), st), "cudaMemsetAsync(loss)")) return rc;
-  if (bhs_launch_features(inputs, B, s->F, s->FT, B, st) != 0) return fail_msg("surrogate: feature launch failed");
-  for (int l = 0; l < 4; ++l) {
-    const bf16 *X = l == 0 ? s->F : s->h[l - 1];
-    const int K = bhs_layer_k(l);
-    BhsGemm g = make_gemm(X, K, s->wb[l], K, B, BHS_HIDDEN, K, BHS_EPI_HIDDEN);
-    g.bias = s->w + bhs_bias_offset(l);
-    g.out = s->h[l];
-    g.out_t = s->ht[l];
-    g.y_out = s->y[l];
-    g.ld_t = B;
-    if (int rc = gemm(s, g, st, "forward")) return rc;
+  if (s->plan.batch != B) {
+    s->plan.batch = 0;
+    if (bhs_train_plan(&s->tr, B, &s->plan) != 0) return fail_msg("surrogate: tensor maps of the training batch failed");
   }
-  {
-    BhsGemm g = make_gemm(s->h[3], BHS_HIDDEN, s->wb[4], BHS_HIDDEN, B, BHS_HEAD, BHS_HIDDEN, BHS_EPI_HEAD);
-    g.bias = s->w + bhs_bias_offset(4);
-    g.out = s->out;
-    if (int rc = gemm(s, g, st, "head")) return rc;
-  }
-  if (bhs_launch_loss(s->out, targets, B, s->dout, s->dout_t, s->loss, st) != 0)
-    return fail_msg("surrogate: loss launch failed");
-  {  // head: dW4^T = H4^T dout, dY4 = (dout W4) * SiLU'(Y4)
-    BhsGemm g = make_gemm(s->ht[3], static_cast<int>(B), s->dout_t, static_cast<int>(B), BHS_HIDDEN, BHS_HEAD,
-                          static_cast<int>(B), BHS_EPI_F32);
-    g.kchunks_per_split = kDwChunks;
-    g.out = s->part[4];
-    if (int rc = gemm(s, g, st, "dW4")) return rc;
-    BhsGemm d = make_gemm(s->dout, BHS_HEAD_PAD, s->wt[4], BHS_HEAD_PAD, B, BHS_HIDDEN, BHS_HEAD_PAD,
-                          BHS_EPI_BACKWARD);
-    d.Y = s->y[3];
-    d.out = s->dy[3];
-    d.out_t = s->dyt[3];
-    d.ld_t = B;
-    if (int rc = gemm(s, d, st, "dH4")) return rc;
-  }
-  for (int l = 3; l >= 0; --l) {
-    const int K = bhs_layer_k(l);
-    const bf16 *XT = l == 0 ? s->FT : s->ht[l - 1];
-    BhsGemm g = make_gemm(s->dyt[l], static_cast<int>(B), XT, static_cast<int>(B), BHS_HIDDEN, K,
-                          static_cast<int>(B), BHS_EPI_F32);
-    g.kchunks_per_split = kDwChunks;
-    g.out = s->part[l];
-    if (int rc = gemm(s, g, st, "dW")) return rc;
-    if (l == 0) break;
-    BhsGemm d = make_gemm(s->dy[l], BHS_HIDDEN, s->wt[l], BHS_HIDDEN, B, BHS_HIDDEN, BHS_HIDDEN, BHS_EPI_BACKWARD);
-    d.Y = s->y[l - 1];
-    d.out = s->dy[l - 1];
-    d.out_t = s->dyt[l - 1];
-    d.ld_t = B;
-    if (int rc = gemm(s, d, st, "dH")) return rc;
-  }
-  const bf16 *dyt[BHS_LAYERS] = {s->dyt[0], s->dyt[1], s->dyt[2], s->dyt[3], s->dout_t};
-  if (bhs_launch_bias_grads(dyt, B, s->grad, st) != 0) return fail_msg("surrogate: bias-gradient launch failed");
-  const float *parts[BHS_LAYERS] = {s->part[0], s->part[1], s->part[2], s->part[3], s->part[4]};
-  const int sp = static_cast<int>(dw_splits(B));
-  const int splits[BHS_LAYERS] = {sp, sp, sp, sp, sp};
-  if (bhs_launch_collect_dw(parts, splits, s->grad, st) != 0) return fail_msg("surrogate: dW collection failed");
-  if (loss4)
-    if (int rc = cuda_check(cudaMemcpyAsync(loss4, s->loss, 4 * sizeof(float), cudaMemcpyDeviceToDevice, st),
-                            "cudaMemcpyAsync(loss)"))
-      return rc;
+  float *loss = loss4 ? loss4 : s->loss;
+  if (int rc = cuda_check(cudaMemsetAsync(loss, 0, 4 * sizeof(float), st), "cudaMemsetAsync(loss)")) return rc;
+  if (bhs_launch_train(&s->tr, &s->plan, inputs, targets, grad, loss, s->err, s->wait_ns, st) != 0)
+    return fail_msg("surrogate: training kernels failed to launch");
   return 0;
 }
 
@@ -279,36 +191,33 @@ BH_Surrogate *bh_surrogate_create(int64_t max_batch, uint64_t seed) {
   if (alloc(s, &s->w, P, "cudaMalloc(params)") || alloc(s, &s->m, P, "cudaMalloc(adam m)") ||
       alloc(s, &s->v, P, "cudaMalloc(adam v)") || alloc(s, &s->grad, P, "cudaMalloc(grad)"))
     return bad();
+  BhsTrainBuffers &t = s->tr;
+  t.params = s->w;
   for (int l = 0; l < BHS_LAYERS; ++l) {
     const size_t nk = static_cast<size_t>(bhs_layer_n(l)) * bhs_layer_k(l);
-    if (alloc(s, &s->wb[l], nk, "cudaMalloc(bf16 weights)") || alloc(s, &s->wh[l], nk, "cudaMalloc(f16 weights)"))
+    if (alloc(s, &t.wb[l], nk, "cudaMalloc(bf16 weights)") || alloc(s, &s->wh[l], nk, "cudaMalloc(f16 weights)"))
       return bad();
     const size_t tsz = l == BHS_LAYERS - 1 ? static_cast<size_t>(BHS_HIDDEN) * BHS_HEAD_PAD : nk;
-    if (alloc(s, &s->wt[l], tsz, "cudaMalloc(bf16 weights^T)")) return bad();
+    if (alloc(s, &t.wt[l], tsz, "cudaMalloc(bf16 weights^T)")) return bad();
   }
-  if (alloc(s, &s->F, B * BHS_FEATURES, "cudaMalloc(features)") ||
-      alloc(s, &s->FT, B * BHS_FEATURES, "cudaMalloc(features^T)"))
-    return bad();
+  if (alloc(s, &t.F, B * BHS_FEATURES, "cudaMalloc(features)")) return bad();
   for (int i = 0; i < 4; ++i) {
-    if (alloc(s, &s->h[i], B * BHS_HIDDEN, "cudaMalloc(H)") || alloc(s, &s->ht[i], B * BHS_HIDDEN, "cudaMalloc(H^T)") ||
-        alloc(s, &s->y[i], B * BHS_HIDDEN, "cudaMalloc(Y)") || alloc(s, &s->dy[i], B * BHS_HIDDEN, "cudaMalloc(dY)") ||
-        alloc(s, &s->dyt[i], B * BHS_HIDDEN, "cudaMalloc(dY^T)"))
+    if (alloc(s, &t.h[i], B * BHS_HIDDEN, "cudaMalloc(H)") || alloc(s, &t.dy[i], B * BHS_HIDDEN, "cudaMalloc(dY)"))
       return bad();
+    if (i < 3 && alloc(s, &t.y[i], B * BHS_HIDDEN, "cudaMalloc(Y)")) return bad();
   }
-  if (alloc(s, &s->out, B * BHS_HEAD, "cudaMalloc(head)") ||
-      alloc(s, &s->dout, B * BHS_HEAD_PAD, "cudaMalloc(dout)") ||
-      alloc(s, &s->dout_t, B * BHS_HEAD, "cudaMalloc(dout^T)"))
+  if (alloc(s, &t.dout, B * BHS_HEAD_PAD, "cudaMalloc(dout)") ||
+      alloc(s, &t.bias_part, B / 32 * (4 * BHS_HIDDEN + BHS_HEAD), "cudaMalloc(bias partials)"))
     return bad();
-  const size_t sp = static_cast<size_t>(dw_splits(max_batch));
   for (int l = 0; l < BHS_LAYERS; ++l) {
-    const size_t per = l == BHS_LAYERS - 1 ? static_cast<size_t>(BHS_HIDDEN) * BHS_HEAD
-                                           : static_cast<size_t>(BHS_HIDDEN) * bhs_layer_k(l);
-    if (alloc(s, &s->part[l], sp * per, "cudaMalloc(dW partials)")) return bad();
+    const size_t per = static_cast<size_t>(BHS_HIDDEN) * (l == BHS_LAYERS - 1 ? BHS_HEAD : bhs_layer_k(l));
+    if (alloc(s, &t.part[l], static_cast<size_t>(bhs_train_splits(l, max_batch)) * per, "cudaMalloc(dW partials)"))
+      return bad();
   }
   if (alloc(s, &s->loss, 4, "cudaMalloc(loss)") || alloc(s, &s->err, 1, "cudaMalloc(error flag)")) return bad();
   // Zero what is only partly written: padded dout columns, W4^T padding, moments, flags.
-  if (cuda_check(cudaMemset(s->dout, 0, B * BHS_HEAD_PAD * sizeof(bf16)), "cudaMemset") ||
-      cuda_check(cudaMemset(s->wt[BHS_LAYERS - 1], 0, static_cast<size_t>(BHS_HIDDEN) * BHS_HEAD_PAD * sizeof(bf16)),
+  if (cuda_check(cudaMemset(t.dout, 0, B * BHS_HEAD_PAD * sizeof(bf16)), "cudaMemset") ||
+      cuda_check(cudaMemset(t.wt[BHS_LAYERS - 1], 0, static_cast<size_t>(BHS_HIDDEN) * BHS_HEAD_PAD * sizeof(bf16)),
                  "cudaMemset") ||
       cuda_check(cudaMemset(s->m, 0, P * sizeof(float)), "cudaMemset") ||
       cuda_check(cudaMemset(s->v, 0, P * sizeof(float)), "cudaMemset") ||
@@ -362,7 +271,7 @@ int bh_surrogate_set_state(BH_Surrogate *s, const float *m, const float *v, int6
 
 int bh_surrogate_features(const float *inputs, int64_t n, void *features, void *stream) {
   if (n < 0 || (n > 0 && (!inputs || !features))) return fail_msg("surrogate: bad feature arguments");
-  if (bhs_launch_features(inputs, n, static_cast<bf16 *>(features), nullptr, 0, static_cast<cudaStream_t>(stream)))
+  if (bhs_launch_features(inputs, n, static_cast<bf16 *>(features), static_cast<cudaStream_t>(stream)))
     return fail_msg("surrogate: feature launch failed");
   return 0;
 }
@@ -390,11 +299,7 @@ int bh_surrogate_forward(BH_Surrogate *s, const float *inputs, int64_t n, float 
 int bh_surrogate_gradients(BH_Surrogate *s, const float *inputs, const float *targets, int64_t batch, float *grad,
                            float *loss4, void *stream) {
   if (!s || !inputs || !targets || !grad) return fail_msg("surrogate: bad gradient arguments");
-  auto st = static_cast<cudaStream_t>(stream);
-  if (int rc = forward_backward(s, inputs, targets, batch, loss4, st)) return rc;
-  return cuda_check(cudaMemcpyAsync(grad, s->grad, static_cast<size_t>(s->n_params) * sizeof(float),
-                                    cudaMemcpyDeviceToDevice, st),
-                    "cudaMemcpyAsync(grad)");
+  return forward_backward(s, inputs, targets, batch, grad, loss4, static_cast<cudaStream_t>(stream));
 }
 
 int bh_surrogate_train_step(BH_Surrogate *s, const float *inputs, const float *targets, int64_t batch,
@@ -404,12 +309,12 @@ int bh_surrogate_train_step(BH_Surrogate *s, const float *inputs, const float *t
       !(adam->eps > 0.0f))
     return fail_msg("surrogate: Adam needs lr > 0, betas in [0, 1), eps > 0");
   auto st = static_cast<cudaStream_t>(stream);
-  if (int rc = forward_backward(s, inputs, targets, batch, loss4, st)) return rc;
+  if (int rc = forward_backward(s, inputs, targets, batch, s->grad, loss4, st)) return rc;
   s->step += 1;
   const double t = static_cast<double>(s->step);
   const float lr_t = static_cast<float>(adam->lr * std::sqrt(1.0 - std::pow(adam->beta2, t)) /
                                         (1.0 - std::pow(adam->beta1, t)));
-  if (bhs_launch_adam(s->w, s->grad, s->m, s->v, s->n_params, lr_t, adam->beta1, adam->beta2, adam->eps, s->wb, s->wt,
+  if (bhs_launch_adam(s->w, s->grad, s->m, s->v, s->n_params, lr_t, adam->beta1, adam->beta2, adam->eps, s->tr.wb, s->tr.wt,
                       st) != 0)
     return fail_msg("surrogate: Adam launch failed");
   s->bias_stale = true;
@@ -809,7 +714,13 @@ int bh_bf16_gemm(const void *A, const void *B, int64_t M, int N, int K, float *C
     if (int rc = cuda_check(bhh_malloc(&err, sizeof(int)), "cudaMalloc(error flag)")) return rc;
     cudaMemset(err, 0, sizeof(int));
   }
-  BhsGemm g = make_gemm(A, K, B, K, M, N, K, BHS_EPI_F32);
+  BhsGemm g{};
+  g.A = A;
+  g.B = B;
+  g.M = M;
+  g.N = N;
+  g.K = K;
+  g.lda = g.ldb = K;
   g.out = C;
   g.wait_ns = kDefaultWaitNs;
   if (bhs_launch_gemm(&g, err, static_cast<cudaStream_t>(stream)) != 0) return fail_msg("bf16 gemm: launch failed");
