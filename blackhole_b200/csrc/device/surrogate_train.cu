@@ -14,9 +14,14 @@
 // What bounds it (batch 16384, one B200): 23 GFLOP, 14 us of tensor time at
 // the measured rate. One GEMM launch per product (twenty launches, a tile's
 // loads, MMAs and its row-by-row epilogue one after another, every activation
-// and gradient also written transposed) took 298 us; this takes MEASURED us.
-// 128 tiles leave 20 SMs idle in the pass; a tile's chain of nine products
-// and epilogues is its time (an epilogue's tanh alone is 2,048 cycles a layer).
+// and gradient also written transposed) took 298 us; this takes 85: 45 in the
+// pass, 22 in the weight gradients, 8 in the collection, the rest between
+// them. The pass is bound by the tile's chain of nine products and epilogues
+// and, inside the epilogues, by the L2: its 128 tiles move in step, and write
+// and read back 100 MB of FP32 pre-activations and stream 115 MB of weights (a
+// layer whose pre-activations stay in tensor memory takes 3.9 K cycles, the
+// others 7). With 8 epilogue warps and an mbarrier arrival per thread the
+// pass took 60.
 #include <algorithm>
 #include <cstdio>
 #include <cstring>
@@ -30,8 +35,8 @@ constexpr int kChunk = kTile * kBK * 2;         // 16 KB: 64 columns of a tile, 
 constexpr int kWStage = BHS_HIDDEN * kBK * 2;   // 32 KB: 64 columns of a weight matrix
 constexpr int kWRing = 4;
 constexpr int kBiases = 4 * BHS_HIDDEN + BHS_HEAD;
-constexpr int kPassThreads = 352;               // producer, MMA issuer, 8 epilogue warps, store warp
-constexpr int kEpiThreads = 256;
+constexpr int kEpiWarps = 16;                   // per TMEM lane quarter four, 16 columns of each chunk
+constexpr int kPassThreads = 32 * (kEpiWarps + 3);  // + producer, MMA issuer, store warp
 constexpr int kPassSmem = 4 * kChunk + kWRing * kWStage + kBiases * 4 + 64 + 1024 + 256;
 
 // Tensor maps of a plan, all {64, rows} boxes with the 128-byte swizzle.
@@ -77,7 +82,7 @@ __device__ __forceinline__ void tmem_ld16_nowait(uint32_t taddr, float (&v)[16])
 
 // Loss of one row and its gradient d with respect to the 16 head outputs o:
 // cross entropy of the class and the squared error of the masked targets.
-__device__ __forceinline__ void row_loss(const float (&o)[BHS_HEAD], const float* __restrict__ t, float invB,
+__device__ __forceinline__ void row_loss(const float (&o)[BHS_HEAD], const float (&t)[BHS_TARGETS], float invB,
                                          float (&d)[BHS_HEAD], float (&acc)[4]) {
   const int cls = (int)t[0], nc = (int)t[1];
 #pragma unroll
@@ -142,7 +147,7 @@ __global__ void __launch_bounds__(kPassThreads, 1)
       umma::mbar_init(full(i), 1);
       umma::mbar_init(empty(i), 1);
     }
-    for (int c = 0; c < 4; ++c) umma::mbar_init(ready(c), kEpiThreads);
+    for (int c = 0; c < 4; ++c) umma::mbar_init(ready(c), kEpiWarps);
     umma::mbar_init(acc_full, 1);
     umma::mbar_init(stored, 1);
     umma::mbar_init(drained, 1);
@@ -224,7 +229,7 @@ __global__ void __launch_bounds__(kPassThreads, 1)
       umma::mma_commit(drained);
       umma::mbar_wait(drained, 0, kDrainNs);
     }
-  } else if (warp == 10) {
+  } else if (warp == 2) {
     if (lane == 0) {  // copies each operand set to HBM as its chunks are written
       uint32_t seen[4] = {0u, 0u, 0u, 0u};
       bool ok = true;
@@ -250,17 +255,18 @@ __global__ void __launch_bounds__(kPassThreads, 1)
         }
       bulk_wait();
     }
-  } else {  // epilogue: TMEM lane quarter q (warp % 4); columns 32 hf .. 32 hf + 31 of every chunk
-    const int hf = (warp - 2) >> 2;
+  } else {  // epilogue: TMEM lane quarter q (warp % 4); columns 16 hf .. 16 hf + 15 of every chunk
+    const int hf = (warp - 3) >> 2;
     const int q = warp & 3;
     const int r = q * 32 + lane;
     const uint32_t tacc = tmem + ((uint32_t)(q * 32) << 16);
     uint32_t acc_seen = 0, stores = 0, stores_seen = 0;
     bool ok = true;
-    auto chunk_done = [&](int c) {
+    auto chunk_done = [&](int c) {  // one arrival a warp: an arrival is an atomic on one word
       umma::fence_async_smem();
       umma::tc_fence_before();
-      umma::mbar_arrive(ready(c));
+      __syncwarp();
+      if (lane == 0) umma::mbar_arrive(ready(c));
     };
     // the copy of the last set has read the tile's buffer
     auto wait_stored = [&]() {
@@ -273,47 +279,44 @@ __global__ void __launch_bounds__(kPassThreads, 1)
       ++acc_seen;
       umma::tc_fence_after();
     };
-    // 32 values of this row into chunk c, as BF16
-    auto put32 = [&](int c, const float* v) {
+    // 16 values of this row into chunk c, as BF16
+    auto put16 = [&](int c, const float (&v)[16]) {
 #pragma unroll
-      for (int u = 0; u < 4; ++u)
-        st_unit(act + (uint32_t)c * kChunk, r, 4 * hf + u, pack_bf16(v[8 * u], v[8 * u + 1]),
+      for (int u = 0; u < 2; ++u)
+        st_unit(act + (uint32_t)c * kChunk, r, 2 * hf + u, pack_bf16(v[8 * u], v[8 * u + 1]),
                 pack_bf16(v[8 * u + 2], v[8 * u + 3]), pack_bf16(v[8 * u + 4], v[8 * u + 5]),
                 pack_bf16(v[8 * u + 6], v[8 * u + 7]));
     };
-    // column sums over the warp's 32 rows of n BF16 columns from unit u0 of chunk c: lane l has column l
-    auto column_sum = [&](int c, int u0, int rows, int row0, int col) {
+    // sums over the warp's 32 rows of 16 BF16 columns from unit u0 of chunk c: lanes l and l + 16 get column l
+    auto column_sum = [&](int c, int u0) {
       float s = 0.0f;
+      const int col = lane & 15;
       const uint32_t base = act + (uint32_t)c * kChunk + 2u * (uint32_t)(col & 7);
-#pragma unroll 8
-      for (int i = 0; i < rows; ++i) {
-        const int row = q * 32 + row0 + i;
+#pragma unroll
+      for (int i = 0; i < 16; ++i) {
+        const int row = q * 32 + (lane & 16) + i;
         const uint32_t a = base + (uint32_t)row * 128u + ((uint32_t)((u0 + (col >> 3)) ^ (row & 7)) << 4);
         uint16_t h;
         asm volatile("ld.shared.u16 %0, [%1];" : "=h"(h) : "r"(a) : "memory");
         s += __uint_as_float((uint32_t)h << 16);
       }
-      return s;
+      return s + __shfl_xor_sync(0xffffffffu, s, 16);
     };
     for (int64_t tile = blockIdx.x; ok && tile < tiles; tile += gridDim.x) {
       const int64_t row = tile * kTile + r;
       float* bias_out = A.bias_part + (tile * 4 + q) * kBiases;
-      {  // features: half 0 inputs 0, 1 (chunk 0), half 1 inputs 2, 3 (chunk 1) and the rest (chunk 2)
+      {  // features: warp group hf the pairs of input hf (32 columns), group 3 the rest (chunk 2) as well
         wait_stored();
         if (!ok) break;
-        float x[4], lam, eta;
+        float x[4], lam, eta, v[2 * BHS_FOURIER];
         scaled_inputs(reinterpret_cast<const float4*>(A.in)[row], x, lam, eta);
-#pragma unroll 1
-        for (int d = 2 * hf; d < 2 * hf + 2; ++d) {
-          float v[2 * BHS_FOURIER];
-          fourier_pairs(d == 0 ? x[0] : (d == 1 ? x[1] : (d == 2 ? x[2] : x[3])), v);
+        fourier_pairs(hf == 0 ? x[0] : (hf == 1 ? x[1] : (hf == 2 ? x[2] : x[3])), v);
 #pragma unroll
-          for (int u = 0; u < 4; ++u)
-            st_unit(act + (uint32_t)hf * kChunk, r, 4 * (d & 1) + u, pack_bf16(v[8 * u], v[8 * u + 1]),
-                    pack_bf16(v[8 * u + 2], v[8 * u + 3]), pack_bf16(v[8 * u + 4], v[8 * u + 5]),
-                    pack_bf16(v[8 * u + 6], v[8 * u + 7]));
-        }
-        if (hf == 1) {
+        for (int u = 0; u < 4; ++u)
+          st_unit(act + (uint32_t)(hf >> 1) * kChunk, r, 4 * (hf & 1) + u, pack_bf16(v[8 * u], v[8 * u + 1]),
+                  pack_bf16(v[8 * u + 2], v[8 * u + 3]), pack_bf16(v[8 * u + 4], v[8 * u + 5]),
+                  pack_bf16(v[8 * u + 6], v[8 * u + 7]));
+        if (hf == 3) {
           st_unit(act + 2u * kChunk, r, 0, pack_bf16(x[0], x[1]), pack_bf16(x[2], x[3]), pack_bf16(lam, eta), 0u);
           for (int u = 1; u < 8; ++u) st_unit(act + 2u * kChunk, r, u, 0u, 0u, 0u, 0u);
         }
@@ -327,40 +330,45 @@ __global__ void __launch_bounds__(kPassThreads, 1)
         const uint32_t acc = tacc + acc_col(l);
         const float* b = sb + l * BHS_HIDDEN;
         float4* ys = l < 3 ? reinterpret_cast<float4*>(A.y[l]) + tile * (kTile * BHS_HIDDEN / 4) : nullptr;
-        float va[32], vb[32];
-        umma::tmem_ld32_nowait(acc + 32u * hf, va);
+        float va[16], vb[16];
+        tmem_ld16_nowait(acc + 16u * hf, va);
         umma::tmem_wait_ld();
 #pragma unroll
         for (int c = 0; c < 4; ++c) {
-          float* v = (c & 1) ? vb : va;
-          if (c < 3) umma::tmem_ld32_nowait(acc + 64u * (c + 1) + 32u * hf, (c & 1) ? va : vb);
-          const int col = 64 * c + 32 * hf;
+          float(&v)[16] = (c & 1) ? vb : va;
+          if (c < 3) tmem_ld16_nowait(acc + 64u * (c + 1) + 16u * hf, (c & 1) ? va : vb);
+          const int col = 64 * c + 16 * hf;
 #pragma unroll
-          for (int i = 0; i < 32; ++i) v[i] += b[col + i];
-          if (l < 3) {
-#pragma unroll
-            for (int g = 0; g < 8; ++g)
-              ys[(col / 4 + g) * kTile + r] = make_float4(v[4 * g], v[4 * g + 1], v[4 * g + 2], v[4 * g + 3]);
+          for (int g = 0; g < 4; ++g) {
+            const float4 bb = reinterpret_cast<const float4*>(b + col)[g];
+            v[4 * g] += bb.x, v[4 * g + 1] += bb.y, v[4 * g + 2] += bb.z, v[4 * g + 3] += bb.w;
+            if (l < 3) ys[(col / 4 + g) * kTile + r] = make_float4(v[4 * g], v[4 * g + 1], v[4 * g + 2], v[4 * g + 3]);
           }
 #pragma unroll
-          for (int i = 0; i < 32; ++i) v[i] = silu(v[i]);
-          put32(c, v);
+          for (int i = 0; i < 16; ++i) v[i] = silu(v[i]);
+          put16(c, v);
           chunk_done(c);
           if (c < 3) umma::tmem_wait_ld();
         }
         ++stores;
       }
       if (!ok) break;
+      float t[BHS_TARGETS];
+      if (hf == 0) {
+        const float4* tp = reinterpret_cast<const float4*>(A.targets) + row * 4;
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          const float4 f = tp[i];
+          t[4 * i] = f.x, t[4 * i + 1] = f.y, t[4 * i + 2] = f.z, t[4 * i + 3] = f.w;
+        }
+      }
       wait_acc();
       if (ok) wait_stored();
       if (!ok) break;
       if (hf == 0) {  // head outputs, loss, dout
-        float o[16], d[16], part[4], t[BHS_TARGETS];
+        float o[16], d[16], part[4];
         tmem_ld16_nowait(tacc + acc_col(4), o);
         umma::tmem_wait_ld();
-        const float4* tp = reinterpret_cast<const float4*>(A.targets) + row * 4;
-#pragma unroll
-        for (int i = 0; i < 4; ++i) reinterpret_cast<float4*>(t)[i] = tp[i];
 #pragma unroll
         for (int i = 0; i < BHS_HEAD; ++i) o[i] += sb[4 * BHS_HIDDEN + i];
         row_loss(o, t, 1.0f / (float)A.B, d, part);
@@ -373,8 +381,7 @@ __global__ void __launch_bounds__(kPassThreads, 1)
         g[0] = make_uint4(pk[0], pk[1], pk[2], pk[3]);
         g[1] = make_uint4(pk[4], pk[5], pk[6], pk[7]);
         __syncwarp();
-        float s = column_sum(0, 0, 16, 16 * (lane >> 4), lane & 15);
-        s += __shfl_xor_sync(0xffffffffu, s, 16);
+        const float s = column_sum(0, 0);
         if (lane < 16) bias_out[4 * BHS_HIDDEN + lane] = s;
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
@@ -387,36 +394,41 @@ __global__ void __launch_bounds__(kPassThreads, 1)
       chunk_done(0);
       for (int s = 5; s < 9; ++s) {  // dY_l = (dY_(l+1) W_(l+1)) * SiLU'(Y_l)
         const int l = 8 - s;
+        const float4* ys = l < 3 ? reinterpret_cast<const float4*>(A.y[l]) + tile * (kTile * BHS_HIDDEN / 4) : nullptr;
+        float4 yn[4];  // the next chunk's pre-activations, read ahead
+        if (l < 3) {
+#pragma unroll
+          for (int g = 0; g < 4; ++g) yn[g] = ys[(4 * hf + g) * kTile + r];
+        }
         wait_acc();
         if (ok) wait_stored();
         if (!ok) break;
         const uint32_t acc = tacc + acc_col(s);
-        const float4* ys = l < 3 ? reinterpret_cast<const float4*>(A.y[l]) + tile * (kTile * BHS_HIDDEN / 4) : nullptr;
 #pragma unroll 1
         for (int c = 0; c < 4; ++c) {
-          const int col = 64 * c + 32 * hf;
-          float v[32], y[32];
-          umma::tmem_ld32_nowait(acc + (uint32_t)col, v);
+          const int col = 64 * c + 16 * hf;
+          float v[16], y[16];
+          tmem_ld16_nowait(acc + (uint32_t)col, v);
           if (l == 3) {
-            umma::tmem_ld32_nowait(tacc + acc_col(3) + (uint32_t)col, y);
+            tmem_ld16_nowait(tacc + acc_col(3) + (uint32_t)col, y);
           } else {
 #pragma unroll
-            for (int g = 0; g < 8; ++g) {
-              const float4 f = ys[(col / 4 + g) * kTile + r];
-              y[4 * g] = f.x, y[4 * g + 1] = f.y, y[4 * g + 2] = f.z, y[4 * g + 3] = f.w;
+            for (int g = 0; g < 4; ++g) {
+              y[4 * g] = yn[g].x, y[4 * g + 1] = yn[g].y, y[4 * g + 2] = yn[g].z, y[4 * g + 3] = yn[g].w;
+              if (c < 3) yn[g] = ys[((col + 64) / 4 + g) * kTile + r];
             }
           }
           umma::tmem_wait_ld();
           if (l == 3) {
 #pragma unroll
-            for (int i = 0; i < 32; ++i) y[i] += sb[3 * BHS_HIDDEN + col + i];
+            for (int i = 0; i < 16; ++i) y[i] += sb[3 * BHS_HIDDEN + col + i];
           }
 #pragma unroll
-          for (int i = 0; i < 32; ++i) v[i] *= silu_grad(y[i]);
-          put32(c, v);
+          for (int i = 0; i < 16; ++i) v[i] *= silu_grad(y[i]);
+          put16(c, v);
           chunk_done(c);
-          __syncwarp();
-          bias_out[l * BHS_HIDDEN + col + lane] = column_sum(c, 4 * hf, 32, 0, lane);
+          const float s1 = column_sum(c, 2 * hf);
+          if (lane < 16) bias_out[l * BHS_HIDDEN + col + lane] = s1;
         }
         ++stores;
       }
