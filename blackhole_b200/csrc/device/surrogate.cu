@@ -229,7 +229,7 @@ __global__ void k_features(const float* __restrict__ in, int64_t n, __nv_bfloat1
 #endif
 
 constexpr int kInfThreads = 576;  // 2 control warps + 2 slots x 8 epilogue warps
-constexpr int kEpiThreads = 256;  // epilogue threads per slot
+constexpr int kEpiWarps = 8;  // epilogue warps per slot; each arrives once per layer
 constexpr int kInfRing = 3;
 constexpr int kActChunk = kBM * kBK * 2;       // 16 KB: one 64-column chunk of a tile
 constexpr int kActBytes = 4 * kActChunk;        // 64 KB: 256 columns
@@ -275,7 +275,7 @@ __global__ void __launch_bounds__(kInfThreads, 1)
       umma::mbar_init(empty(i), 1);
     }
     for (int s = 0; s < 2; ++s) {
-      umma::mbar_init(act_ready(s), kEpiThreads);
+      umma::mbar_init(act_ready(s), kEpiWarps);
       umma::mbar_init(acc_full(s), 1);
     }
     umma::mbar_init(drained, 1);
@@ -396,7 +396,8 @@ __global__ void __launch_bounds__(kInfThreads, 1)
         }
       }
       umma::fence_async_smem();
-      umma::mbar_arrive(act_ready(s));
+      __syncwarp();
+      if (lane == 0) umma::mbar_arrive(act_ready(s));
       bool ok = true;
       for (int l = 0; l < BHS_LAYERS - 1; ++l) {
         ok = __all_sync(0xffffffffu, umma::mbar_wait(acc_full(s), ph, A.wait_ns));
@@ -450,7 +451,8 @@ __global__ void __launch_bounds__(kInfThreads, 1)
 #endif
         umma::fence_async_smem();
         umma::tc_fence_before();
-        umma::mbar_arrive(act_ready(s));
+        __syncwarp();
+        if (lane == 0) umma::mbar_arrive(act_ready(s));
       }
       if (ok) ok = __all_sync(0xffffffffu, umma::mbar_wait(acc_full(s), ph, A.wait_ns));
       ph ^= 1u;
