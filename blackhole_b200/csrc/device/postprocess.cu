@@ -13,20 +13,25 @@
 // Here that is three launches instead of nineteen:
 //   k_post_rows : bright-pass fused into the four horizontal blurs. A tile of
 //                 32 rows x 128 columns (+ 32-column halos) in shared memory,
-//                 one lane per row, 8 consecutive outputs per thread, so each
-//                 loaded tap feeds up to 8 FMAs (pitch 193 = 1 mod 32: the
-//                 lanes' rows fall in distinct banks); each output plane is
-//                 staged in shared memory and stored row-coalesced.
+//                 two rows side by side (pitch 193 pairs: 16 row pairs fall in
+//                 distinct banks); a thread has 8 outputs of a row pair. Each
+//                 output plane is staged in shared memory and stored by rows.
 //   k_post_cols : the four vertical blurs, summed in the reference's order
-//                 (r = 4, 8, 16, 32), and the composite; one lane per
-//                 column, 8 rows per thread; the next scale's planes arrive
-//                 by cp.async while this one is blurred.
+//                 (r = 4, 8, 16, 32), and the composite; a thread has 8 rows
+//                 of two neighbouring columns; the planes of the next two
+//                 (channel, scale) jobs arrive by 16-byte cp.async meanwhile,
+//                 no more rows of them than the scale reaches.
 //   k_post_tone : the tone map into the caller's framebuffer.
+// Both blurs multiply and add two values per instruction (fma.rn.f32x2, each
+// half rounded as the scalar one): issue slots, not the FP32 lanes, bound the
+// scalar version (79 and 68 % issue at 42 and 34 % of the FMA pipe). 1920 x
+// 1080, strength 0.5, per launch: rows 76 -> 61, columns 101 -> 54, tone (with
+// a 64-bit division per pixel) 30 -> 28 us (three powf, 84 % issue).
 // The horizontal results travel through 12 float planes (4 scales x RGB,
-// structure of arrays); the composite goes to a separate buffer because the
-// tone map reads a neighbour's colour (below), which an in-place pass would
-// race on. Bytes per pixel: rows 16 in + 48 out, cols 48 + 16 in + 16 out,
-// tone 16 in + 16 out.
+// structure of arrays, rows padded to 64 columns); the composite goes to a
+// separate buffer because the tone map reads a neighbour's colour (below),
+// which an in-place pass would race on. Bytes per pixel: rows 16 in + 48 out,
+// cols 48 + 16 in + 16 out, tone 16 in + 16 out.
 //
 // The tone map's red and blue come from pixel (rx, ry) = (int(u w), int(v h))
 // with u = px / w, v = py / h rounded to float (cuda_postprocess.cu:165-176,
@@ -50,21 +55,43 @@ constexpr int kRun = 8;    // outputs per thread along the blur direction
 constexpr int kRowsY = 32;
 constexpr int kRowsX = 128;
 constexpr int kRowsW = kRowsX + 2 * kHalo;
-constexpr int kRowsPitch = kRowsW + 1;
-constexpr int kRowsThreads = kRowsY * (kRowsX / kRun);  // 512
-constexpr int kOutPitch = kRowsX + 1;
-constexpr size_t kRowsSmem = sizeof(float) * (3 * kRowsY * kRowsPitch + kRowsY * kOutPitch);
+constexpr int kRowsPitch = kRowsW + 1;          // in row pairs
+constexpr int kRowPairs = kRowsY / 2;
+constexpr int kRowsThreads = kRowPairs * (kRowsX / kRun);  // 256
+constexpr int kOutPitch = kRowsX + 4;
+constexpr size_t kRowsSmem = sizeof(float2) * 3 * kRowPairs * kRowsPitch + sizeof(float) * kRowsY * kOutPitch;
 
 // Columns pass tile.
-constexpr int kColsX = 32;
+constexpr int kColsX = 64;
 constexpr int kColsY = 64;
 constexpr int kColsH = kColsY + 2 * kHalo;
-constexpr int kColsThreads = kColsX * (kColsY / kRun);  // 256
-constexpr size_t kColsSmem = sizeof(float) * 2 * 3 * kColsH * kColsX;  // double-buffered scales
+constexpr int kColsThreads = kColsX / 2 * (kColsY / kRun);  // 256
+constexpr int kColsRing = 3;
+constexpr int kColsBuf = kColsH * kColsX;
+constexpr size_t kColsSmem = sizeof(float) * kColsRing * kColsBuf;
+
+// Floats between rows of a plane: whole tiles of columns, so that every row
+// starts on 256 bytes and the last tile reads within the plane.
+__host__ __device__ constexpr int plane_pitch(int w) { return (w + kColsX - 1) / kColsX * kColsX; }
 
 // Scale index and offset of the normalized taps (2r + 1 each) of half-width R.
 __host__ __device__ constexpr int scale_of(int R) { return R == 4 ? 0 : R == 8 ? 1 : R == 16 ? 2 : 3; }
 __host__ __device__ constexpr int tap_off(int R) { return R == 4 ? 0 : R == 8 ? 9 : R == 16 ? 26 : 59; }
+
+// The taps, each twice: both halves of a packed product.
+struct Taps2 {
+  float2 w[124];
+};
+
+__device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) {
+  float2 d;
+  asm("{\n\t.reg .b64 x, y, z;\n\t"
+      "mov.b64 x, {%2, %3};\n\tmov.b64 y, {%4, %5};\n\tmov.b64 z, {%6, %7};\n\t"
+      "fma.rn.f32x2 z, x, y, z;\n\tmov.b64 {%0, %1}, z;\n\t}"
+      : "=f"(d.x), "=f"(d.y)
+      : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y), "f"(c.x), "f"(c.y));
+  return d;
+}
 
 __device__ __forceinline__ float bright_scale(float4 c, float threshold) {
   const float lum = 0.2126f * c.x + 0.7152f * c.y + 0.0722f * c.z;
@@ -72,63 +99,76 @@ __device__ __forceinline__ float bright_scale(float4 c, float threshold) {
   return lum > 0.001f ? excess / lum : 0.0f;
 }
 
-// acc[j] += sum_t w[t] src[(j + t) * stride], t = 0..2R: the blur of R taps
-// either side of output j, src pointing at output 0's first tap. Unrolled,
-// so w[] is read with constant indices from the kernel's parameter bank.
+// acc[j] += sum_t w[t] src[(j + t) * stride], t = 0..2R in order: the blur of
+// R taps either side of output j, src pointing at output 0's first tap, for
+// two values at a time. The 8 values that a tap meets slide through registers.
 template <int R>
-__device__ __forceinline__ void blur_run(const float *src, int stride, const float *w, float (&acc)[kRun]) {
+__device__ __forceinline__ void blur_run(const float2 *src, int stride, const float2 *w, float2 (&acc)[kRun]) {
+  float2 v[kRun];
 #pragma unroll
-  for (int k = 0; k < kRun + 2 * R; ++k) {
-    const float v = src[k * stride];
+  for (int j = 0; j < kRun; ++j) v[j] = src[j * stride];
 #pragma unroll
-    for (int j = 0; j < kRun; ++j) {
-      const int t = k - j;
-      if (t >= 0 && t <= 2 * R) acc[j] = fmaf(w[t], v, acc[j]);
-    }
+  for (int t = 0; t <= 2 * R; ++t) {
+#pragma unroll
+    for (int j = 0; j < kRun; ++j) acc[j] = fma2(w[t], v[(t + j) % kRun], acc[j]);
+    if (t < 2 * R) v[t % kRun] = src[(t + kRun) * stride];
   }
 }
 
-__global__ void __launch_bounds__(kRowsThreads, 2) k_post_rows(const __grid_constant__ BhkPostTaps taps,
+__global__ void __launch_bounds__(kRowsThreads, 2) k_post_rows(const __grid_constant__ Taps2 taps,
                                                              const float4 *__restrict__ fb, int w, int h,
                                                              float threshold, float *__restrict__ planes) {
-  extern __shared__ float sm[];  // [3][kRowsY][kRowsPitch] bright-pass, then [kRowsY][kOutPitch] one output plane
-  float *stage = sm + 3 * kRowsY * kRowsPitch;
+  extern __shared__ float2 sm[];  // [3][kRowPairs][kRowsPitch] bright-pass, then [kRowsY][kOutPitch] one output plane
+  float *stage = reinterpret_cast<float *>(sm + 3 * kRowPairs * kRowsPitch);
   const int x0 = blockIdx.x * kRowsX, y0 = blockIdx.y * kRowsY;
-  static_assert(kRowsY * kRowsW % kRowsThreads == 0, "whole load rounds");
-  constexpr int kLoads = kRowsY * kRowsW / kRowsThreads;  // 12, all in flight at once
-  float4 v[kLoads];
+  static_assert(kRowPairs * kRowsW % (4 * kRowsThreads) == 0, "whole load rounds");
+#pragma unroll 1
+  for (int k0 = 0; k0 < kRowPairs * kRowsW; k0 += 4 * kRowsThreads) {  // 8 pixels in flight a thread
+    float4 v[4][2];
 #pragma unroll
-  for (int k = 0; k < kLoads; ++k) {
-    const int e = threadIdx.x + k * kRowsThreads, row = e / kRowsW, col = e - row * kRowsW;
-    const int y = y0 + row;
-    v[k] = y < h ? fb[(int64_t)y * w + min(max(x0 - kHalo + col, 0), w - 1)] : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-  }
+    for (int k = 0; k < 4; ++k) {
+      const int e = k0 + k * kRowsThreads + threadIdx.x, rp = e / kRowsW, col = e - rp * kRowsW;
+      const int x = min(max(x0 - kHalo + col, 0), w - 1);
 #pragma unroll
-  for (int k = 0; k < kLoads; ++k) {
-    const int e = threadIdx.x + k * kRowsThreads, row = e / kRowsW, col = e - row * kRowsW;
-    const float s = bright_scale(v[k], threshold);
-    sm[(0 * kRowsY + row) * kRowsPitch + col] = v[k].x * s;
-    sm[(1 * kRowsY + row) * kRowsPitch + col] = v[k].y * s;
-    sm[(2 * kRowsY + row) * kRowsPitch + col] = v[k].z * s;
+      for (int i = 0; i < 2; ++i) {
+        const int y = y0 + 2 * rp + i;
+        v[k][i] = y < h ? fb[(int64_t)y * w + x] : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+      }
+    }
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      const int e = k0 + k * kRowsThreads + threadIdx.x, rp = e / kRowsW, col = e - rp * kRowsW;
+      const float s0 = bright_scale(v[k][0], threshold), s1 = bright_scale(v[k][1], threshold);
+      sm[(0 * kRowPairs + rp) * kRowsPitch + col] = make_float2(v[k][0].x * s0, v[k][1].x * s1);
+      sm[(1 * kRowPairs + rp) * kRowsPitch + col] = make_float2(v[k][0].y * s0, v[k][1].y * s1);
+      sm[(2 * kRowPairs + rp) * kRowsPitch + col] = make_float2(v[k][0].z * s0, v[k][1].z * s1);
+    }
   }
-  const int lane = threadIdx.x & 31, run = threadIdx.x >> 5;
-  const int64_t n = (int64_t)w * h;
+  const int rp = threadIdx.x % kRowPairs, run = threadIdx.x / kRowPairs;
+  const int pitch = plane_pitch(w);
   // Results leave through the stage, so that a warp stores 32 consecutive
-  // floats of one row (the compute layout has a lane per row).
+  // float4 of one row (the compute layout has a lane per row pair).
   auto scale = [&](auto rtag) {
     constexpr int R = decltype(rtag)::value, si = scale_of(R);
 #pragma unroll 1
     for (int c = 0; c < 3; ++c) {
       __syncthreads();  // bright-pass written / the previous plane copied out
-      float acc[kRun] = {};
-      blur_run<R>(sm + (c * kRowsY + lane) * kRowsPitch + kHalo + run * kRun - R, 1, taps.w + tap_off(R), acc);
-#pragma unroll
-      for (int j = 0; j < kRun; ++j) stage[lane * kOutPitch + run * kRun + j] = acc[j];
+      float2 acc[kRun] = {};
+      blur_run<R>(sm + (c * kRowPairs + rp) * kRowsPitch + kHalo + run * kRun - R, 1, taps.w + tap_off(R), acc);
+      float4 *s0 = reinterpret_cast<float4 *>(stage + 2 * rp * kOutPitch + run * kRun);
+      float4 *s1 = reinterpret_cast<float4 *>(stage + (2 * rp + 1) * kOutPitch + run * kRun);
+      s0[0] = make_float4(acc[0].x, acc[1].x, acc[2].x, acc[3].x);
+      s0[1] = make_float4(acc[4].x, acc[5].x, acc[6].x, acc[7].x);
+      s1[0] = make_float4(acc[0].y, acc[1].y, acc[2].y, acc[3].y);
+      s1[1] = make_float4(acc[4].y, acc[5].y, acc[6].y, acc[7].y);
       __syncthreads();
-      float *out = planes + (int64_t)(si * 3 + c) * n;
-      for (int e = threadIdx.x; e < kRowsY * kRowsX; e += kRowsThreads) {
-        const int row = e / kRowsX, col = e - row * kRowsX;
-        if (y0 + row < h && x0 + col < w) out[(int64_t)(y0 + row) * w + x0 + col] = stage[row * kOutPitch + col];
+      float *out = planes + (int64_t)(si * 3 + c) * h * pitch;
+#pragma unroll
+      for (int e = threadIdx.x; e < kRowsY * kRowsX / 4; e += kRowsThreads) {
+        const int row = e / (kRowsX / 4), col = 4 * (e % (kRowsX / 4));
+        if (y0 + row < h && x0 + col < pitch)
+          *reinterpret_cast<float4 *>(out + (int64_t)(y0 + row) * pitch + x0 + col) =
+              *reinterpret_cast<const float4 *>(stage + row * kOutPitch + col);
       }
     }
   };
@@ -138,75 +178,77 @@ __global__ void __launch_bounds__(kRowsThreads, 2) k_post_rows(const __grid_cons
   scale(std::integral_constant<int, 32>{});
 }
 
-// One scale's three planes (rows y0 - 32 .. y0 + 95 clamped, columns x0 ..
-// x0 + 31; zeros past the right edge) into a shared buffer, by cp.async.
-__device__ __forceinline__ void cols_fetch(float *buf, const float *__restrict__ planes, int si, int64_t n, int x0,
-                                           int y0, int w, int h) {
-  const int lane = threadIdx.x & 31, grp = threadIdx.x >> 5;
-  const int x = x0 + lane;
-#pragma unroll 4
-  for (int k = 0; k < 3 * kColsH / (kColsThreads / kColsX); ++k) {  // 48 rounds of 8 rows
-    const int cr = grp + k * (kColsThreads / kColsX);                 // channel * kColsH + row
-    const int c = cr / kColsH, row = cr - c * kColsH;
-    const int y = min(max(y0 - kHalo + row, 0), h - 1);
-    float *dst = buf + cr * kColsX + lane;
-    if (x < w) {
-      const float *src = planes + (int64_t)(si * 3 + c) * n + (int64_t)y * w + x;
-      asm volatile("cp.async.ca.shared.global [%0], [%1], 4;\n" ::"r"((unsigned)__cvta_generic_to_shared(dst)),
-                   "l"(src)
-                   : "memory");
-    } else {
-      *dst = 0.0f;
-    }
+// Rows y0 - R .. y0 + 63 + R (clamped) of one channel's plane of scale si,
+// columns x0 .. x0 + 63, into a shared buffer, by cp.async.
+__device__ __forceinline__ void cols_fetch(float *buf, const float *__restrict__ planes, int c, int si, int x0,
+                                           int y0, int pitch, int h) {
+  const int R = 4 << si;
+  const float *src = planes + (int64_t)(si * 3 + c) * h * pitch + x0 + 4 * (threadIdx.x % 16);
+  float *dst = buf + 4 * (threadIdx.x % 16);
+  for (int row = threadIdx.x / 16; row < kColsY + 2 * R; row += kColsThreads / 16) {
+    const int y = min(max(y0 - R + row, 0), h - 1);
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(
+                     (unsigned)__cvta_generic_to_shared(dst + row * kColsX)),
+                 "l"(src + (int64_t)y * pitch)
+                 : "memory");
   }
-  asm volatile("cp.async.commit_group;\n" ::: "memory");
 }
 
-__global__ void __launch_bounds__(kColsThreads) k_post_cols(const __grid_constant__ BhkPostTaps taps,
+__global__ void __launch_bounds__(kColsThreads, 2) k_post_cols(const __grid_constant__ Taps2 taps,
                                                              const float *__restrict__ planes,
                                                              const float4 *__restrict__ fb, int w, int h,
                                                              float strength, float4 *__restrict__ out) {
-  extern __shared__ float sm[];  // two buffers of [3][kColsH][kColsX]: scale s in buffer s % 2
-  constexpr int kBuf = 3 * kColsH * kColsX;
+  extern __shared__ float cols_sm[];  // kColsRing buffers of [kColsH][kColsX]: job 4 c + si in buffer job % kColsRing
   const int x0 = blockIdx.x * kColsX, y0 = blockIdx.y * kColsY;
   const int lane = threadIdx.x & 31, grp = threadIdx.x >> 5;
-  const int64_t n = (int64_t)w * h;
-  float tot[3][kRun] = {};
-  cols_fetch(sm, planes, 0, n, x0, y0, w, h);
-  cols_fetch(sm + kBuf, planes, 1, n, x0, y0, w, h);
-  auto scale = [&](auto rtag) {
-    constexpr int R = decltype(rtag)::value, si = scale_of(R);
-    if constexpr (si < 3)
-      asm volatile("cp.async.wait_group 1;\n" ::: "memory");  // scale si landed, si + 1 may be in flight
-    else
-      asm volatile("cp.async.wait_group 0;\n" ::: "memory");
-    __syncthreads();
-    const float *buf = sm + (si & 1) * kBuf;
-#pragma unroll
-    for (int c = 0; c < 3; ++c) {
-      float acc[kRun] = {};
-      blur_run<R>(buf + (c * kColsH + kHalo + grp * kRun - R) * kColsX + lane, kColsX, taps.w + tap_off(R), acc);
-#pragma unroll
-      for (int j = 0; j < kRun; ++j) tot[c][j] += acc[j];
-    }
-    if constexpr (si + 2 < 4) {
-      __syncthreads();  // every warp is done with this buffer
-      cols_fetch(sm + (si & 1) * kBuf, planes, si + 2, n, x0, y0, w, h);
-    }
+  const int pitch = plane_pitch(w);
+  float2 tr[kRun], tg[kRun], tb[kRun];
+  auto fetch = [&](int job) {
+    if (job < 12) cols_fetch(cols_sm + (job % kColsRing) * kColsBuf, planes, job >> 2, job & 3, x0, y0, pitch, h);
+    asm volatile("cp.async.commit_group;\n" ::: "memory");
   };
-  scale(std::integral_constant<int, 4>{});
-  scale(std::integral_constant<int, 8>{});
-  scale(std::integral_constant<int, 16>{});
-  scale(std::integral_constant<int, 32>{});
-  const int x = x0 + lane;
-  if (x >= w) return;
+  fetch(0);
+  fetch(1);
+#pragma unroll 1
+  for (int c = 0; c < 3; ++c) {
+    float2 tot[kRun] = {};
+    auto scale = [&](auto rtag) {
+      constexpr int R = decltype(rtag)::value, si = scale_of(R);
+      const int job = 4 * c + si;
+      asm volatile("cp.async.wait_group 1;\n" ::: "memory");  // this job landed, the next may be in flight
+      __syncthreads();                                         // ... for every warp, and buffer (job + 2) % 3 is free
+      fetch(job + 2);
+      const float2 *buf = reinterpret_cast<const float2 *>(cols_sm + (job % kColsRing) * kColsBuf);
+      float2 acc[kRun] = {};
+      blur_run<R>(buf + grp * kRun * (kColsX / 2) + lane, kColsX / 2, taps.w + tap_off(R), acc);
+#pragma unroll
+      for (int j = 0; j < kRun; ++j) tot[j].x += acc[j].x, tot[j].y += acc[j].y;
+    };
+    scale(std::integral_constant<int, 4>{});
+    scale(std::integral_constant<int, 8>{});
+    scale(std::integral_constant<int, 16>{});
+    scale(std::integral_constant<int, 32>{});
+#pragma unroll
+    for (int j = 0; j < kRun; ++j) {
+      if (c == 0) tr[j] = tot[j];
+      if (c == 1) tg[j] = tot[j];
+      if (c == 2) tb[j] = tot[j];
+    }
+  }
+  const int x = x0 + 2 * lane;
 #pragma unroll
   for (int j = 0; j < kRun; ++j) {
     const int y = y0 + grp * kRun + j;
     if (y >= h) break;
     const int64_t i = (int64_t)y * w + x;
-    const float4 b = fb[i];
-    out[i] = make_float4(b.x + tot[0][j] * strength, b.y + tot[1][j] * strength, b.z + tot[2][j] * strength, 1.0f);
+    if (x < w) {
+      const float4 b = fb[i];
+      out[i] = make_float4(b.x + tr[j].x * strength, b.y + tg[j].x * strength, b.z + tb[j].x * strength, 1.0f);
+    }
+    if (x + 1 < w) {
+      const float4 b = fb[i + 1];
+      out[i + 1] = make_float4(b.x + tr[j].y * strength, b.y + tg[j].y * strength, b.z + tb[j].y * strength, 1.0f);
+    }
   }
 }
 
@@ -221,34 +263,47 @@ __device__ __forceinline__ float tone_channel(float x, float exposure, float vig
   return powf(fmaxf(aces((x * exposure) * vignette), 0.0f), 1.0f / 2.2f);
 }
 
+// A thread has one column of 4 rows, so that u and the column index are worked out once.
+constexpr int kToneRows = 4;
 __global__ void __launch_bounds__(256) k_post_tone(const float4 *__restrict__ src, int w, int h, float exposure,
                                                    float4 *__restrict__ fb) {
-  const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= (int64_t)w * h) return;
-  const int py = (int)(i / w), px = (int)(i - (int64_t)py * w);
-  const float u = __fdiv_rn((float)px, (float)w), v = __fdiv_rn((float)py, (float)h);
+  const int px = blockIdx.x * 64 + (threadIdx.x & 63);
+  const int y0 = (blockIdx.y * 4 + (threadIdx.x >> 6)) * kToneRows;
+  if (px >= w) return;
+  const float u = __fdiv_rn((float)px, (float)w);
   const int rx = min(max((int)__fmul_rn(u, (float)w), 0), w - 1);
-  const int ry = min(max((int)__fmul_rn(v, (float)h), 0), h - 1);
-  const float4 rb = src[(int64_t)ry * w + rx];
-  const float gch = src[i].y;
-  const float du = u - 0.5f, dv = v - 0.5f;
-  const float dist = sqrtf(du * du + dv * dv);
-  const float vig = sqrtf(fmaxf(1.0f - dist * dist * 0.5f, 0.0f));
-  fb[i] = make_float4(tone_channel(rb.x, exposure, vig), tone_channel(gch, exposure, vig),
-                      tone_channel(rb.z, exposure, vig), 1.0f);
+  const float du = u - 0.5f;
+#pragma unroll
+  for (int k = 0; k < kToneRows; ++k) {
+    const int py = y0 + k;
+    if (py >= h) break;
+    const int64_t i = (int64_t)py * w + px;
+    const float v = __fdiv_rn((float)py, (float)h);
+    const int ry = min(max((int)__fmul_rn(v, (float)h), 0), h - 1);
+    const float4 rb = src[(int64_t)ry * w + rx];
+    const float gch = src[i].y;
+    const float dv = v - 0.5f;
+    const float dist = sqrtf(du * du + dv * dv);
+    const float vig = sqrtf(fmaxf(1.0f - dist * dist * 0.5f, 0.0f));
+    fb[i] = make_float4(tone_channel(rb.x, exposure, vig), tone_channel(gch, exposure, vig),
+                        tone_channel(rb.z, exposure, vig), 1.0f);
+  }
 }
 
 }  // namespace
 
-extern "C" int64_t bhk_post_scratch_floats(int w, int h) { return (int64_t)16 * w * h; }
+// 12 padded planes, then the composite (float4 per pixel; 256-byte aligned rows before it keep it aligned).
+extern "C" int64_t bhk_post_scratch_floats(int w, int h) {
+  return (int64_t)12 * plane_pitch(w) * h + (int64_t)4 * w * h;
+}
 
 extern "C" int bhk_post_process(float *fb, int w, int h, const BhkPostTaps *taps, float threshold, float strength,
                                 float exposure, float *scratch, void *stream) {
   if (w <= 0 || h <= 0) return 0;
   const cudaStream_t st = static_cast<cudaStream_t>(stream);
   const int64_t n = (int64_t)w * h;
-  float *planes = scratch;                                  // 12 n floats
-  float4 *comp = reinterpret_cast<float4 *>(scratch + 12 * n);  // n float4
+  float *planes = scratch;
+  float4 *comp = reinterpret_cast<float4 *>(scratch + (int64_t)12 * plane_pitch(w) * h);
   float4 *f4 = reinterpret_cast<float4 *>(fb);
   if (strength != 0.0f) {
     if (cudaFuncSetAttribute(k_post_rows, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kRowsSmem) !=
@@ -256,13 +311,16 @@ extern "C" int bhk_post_process(float *fb, int w, int h, const BhkPostTaps *taps
         cudaFuncSetAttribute(k_post_cols, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kColsSmem) !=
             cudaSuccess)
       return -1;
+    Taps2 t2;
+    for (int i = 0; i < 124; ++i) t2.w[i] = make_float2(taps->w[i], taps->w[i]);
     const dim3 gr((w + kRowsX - 1) / kRowsX, (h + kRowsY - 1) / kRowsY);
-    k_post_rows<<<gr, kRowsThreads, kRowsSmem, st>>>(*taps, f4, w, h, threshold, planes);
+    k_post_rows<<<gr, kRowsThreads, kRowsSmem, st>>>(t2, f4, w, h, threshold, planes);
     const dim3 gc((w + kColsX - 1) / kColsX, (h + kColsY - 1) / kColsY);
-    k_post_cols<<<gc, kColsThreads, kColsSmem, st>>>(*taps, planes, f4, w, h, strength, comp);
+    k_post_cols<<<gc, kColsThreads, kColsSmem, st>>>(t2, planes, f4, w, h, strength, comp);
   } else if (cudaMemcpyAsync(comp, fb, sizeof(float4) * n, cudaMemcpyDeviceToDevice, st) != cudaSuccess) {
     return -1;
   }
-  k_post_tone<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(comp, w, h, exposure, f4);
+  const dim3 gt((w + 63) / 64, (h + 4 * kToneRows - 1) / (4 * kToneRows));
+  k_post_tone<<<gt, 256, 0, st>>>(comp, w, h, exposure, f4);
   return cudaGetLastError() == cudaSuccess ? 0 : -1;
 }
