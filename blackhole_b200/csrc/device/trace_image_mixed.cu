@@ -63,10 +63,12 @@ __device__ __forceinline__ void init_ray(const BhkImageParams &p, long long pix,
   const double beta = p.beta_min + ((double)j + 0.5) * p.dbeta;
   const double a = p.a;
   const double lam = -alpha * p.sin_o;
-  const double eta = beta * beta + (alpha * alpha - a * a) * p.cos_o * p.cos_o;
-  const double qTh = eta + lam * lam;
+  // fused products written out, as in project()
+  const double t = __dmul_rn(__fma_rn(alpha, alpha, -__dmul_rn(a, a)), p.cos_o);
+  const double eta = __fma_rn(beta, beta, __dmul_rn(t, p.cos_o));
+  const double qTh = __dadd_rn(eta, __dmul_rn(lam, lam));
   const double qR = (p.form == 1) ? eta : qTh;
-  const double K = qR + (lam - a) * (lam - a);
+  const double K = __fma_rn(lam - a, lam - a, qR);
   const double r0 = p.r_obs;
   const double A = r0 * r0 + a * a - a * lam;
   const double D = r0 * r0 - 2.0 * r0 + a * a;
@@ -76,7 +78,7 @@ __device__ __forceinline__ void init_ray(const BhkImageParams &p, long long pix,
   R.c.lam = (float)lam;
   R.c.qTh = (float)qTh;
   R.c.K = (float)K;
-  R.c.a2_minus_alam = (float)(a * a - a * lam);
+  R.c.a2_minus_alam = (float)__dsub_rn(__dmul_rn(a, a), __dmul_rn(a, lam));
   R.c.c_pu = (float)(a * a - qTh);
   R.cd.a = a;
   R.cd.lam = lam;
