@@ -216,6 +216,7 @@ struct MediumF {
   float r_min, r_max, fr_scale;  // (n_r - 1) / log(r_max / r_min)
   float lt0, lt_scale, lx0, lx1, lx_scale;
   float ln_nu, ln_len, ds_max, min_transmit;
+  float inv_n_ph;
   float x_coef;        // h nu / (m_e c^2): x = x_coef / (g Theta_e)
   float ln_nub_gauss;  // ln(e / (2 pi m_e c)): ln nu_B per ln gauss
   float ln_2h_c2;      // ln(2 h / c^2)
@@ -242,6 +243,7 @@ __host__ __device__ inline MediumF medium_f(const BhkRtParams &q) {
   m.ln_len = (float)log(q.length_cm);
   m.ds_max = (float)q.ds_max;
   m.min_transmit = (float)q.min_transmit;
+  m.inv_n_ph = 1.0f / (float)q.n_ph;
   m.x_coef = (float)(kH * q.nu / (kMe * kC * kC));
   m.ln_nub_gauss = (float)log(kE / (kTwoPi * kMe * kC));
   m.ln_2h_c2 = (float)log(2.0 * kH / (kC * kC));
@@ -262,9 +264,13 @@ __device__ __forceinline__ bool sample_f(const MediumF &q, float r, float u, flo
   const float fp = phi * (0.15915494309f * (float)q.n_ph);
   const float fl = floorf(fp);
   const float tp = fp - fl;
-  int k0 = (int)fmodf(fl, (float)q.n_ph);
-  if (k0 < 0) k0 += q.n_ph;
+  // fmodf and eight 64-bit indices here took 5 % of the 512^2 transfer (2.84 -> 2.70 ms)
+  int k0 = (int)fl - q.n_ph * (int)floorf(fl * q.inv_n_ph);  // the rounded quotient is off by one at most
+  k0 += k0 < 0 ? q.n_ph : (k0 >= q.n_ph ? -q.n_ph : 0);
+  k0 = min(max(k0, 0), q.n_ph - 1);  // an azimuth that is no number
   const int k1 = (k0 + 1 == q.n_ph) ? 0 : k0 + 1;
+  const float4 *c00 = q.cells + ((long long)i0 * q.n_th + j0) * q.n_ph;
+  const long long row = (long long)q.n_th * q.n_ph;
   float a0 = 0.0f, a1 = 0.0f, a2 = 0.0f;
 #pragma unroll
   for (int di = 0; di < 2; ++di)
@@ -273,7 +279,7 @@ __device__ __forceinline__ bool sample_f(const MediumF &q, float r, float u, flo
 #pragma unroll
       for (int dk = 0; dk < 2; ++dk) {
         const float w = (di ? tr : 1.0f - tr) * (dj ? tt : 1.0f - tt) * (dk ? tp : 1.0f - tp);
-        const float4 v = __ldg(q.cells + ((long long)(i0 + di) * q.n_th + (j0 + dj)) * q.n_ph + (dk ? k1 : k0));
+        const float4 v = __ldg(c00 + (di ? row : 0) + (dj ? q.n_ph : 0) + (dk ? k1 : k0));
         a0 = fmaf(w, v.x, a0);
         a1 = fmaf(w, v.y, a1);
         a2 = fmaf(w, v.z, a2);
