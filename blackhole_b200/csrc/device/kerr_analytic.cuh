@@ -71,6 +71,9 @@
 namespace bhan {
 
 using bhmino::inv_sqrt;
+using bhmino::qdiv;
+using bhmino::qrcp;
+using bhmino::qsqrt;
 
 // Carlson's R_F as one shared device call: inlined at each of its call sites
 // it made the tracer's code large enough that instruction fetch, not
@@ -88,21 +91,21 @@ using std::isnan;
 BHM_HD double carlson_rc(double x, double y) {
   double f = 1.0;
   if (y < 0.0) {
-    f = sqrt(x / (x - y));
+    f = qsqrt(qdiv(x, x - y));
     x = x - y;
     y = -y;
   }
-  if (x == 0.0) return f * 1.5707963267948966 / sqrt(y);
-  const double d = (y - x) / x;
+  if (x == 0.0) return qdiv(f * 1.5707963267948966, qsqrt(y));
+  const double d = qdiv(y - x, x);
   double g;
   if (fabs(d) < 1e-3) {
     g = 1.0 - d * (1.0 / 3.0 - d * (0.2 - d * (1.0 / 7.0 - d * (1.0 / 9.0 - d * (1.0 / 11.0)))));
   } else if (d > 0.0) {
-    const double sd = sqrt(d);
-    g = atan(sd) / sd;
+    const double sd = qsqrt(d);
+    g = qdiv(atan(sd), sd);
   } else {
-    const double sd = sqrt(-d);
-    g = atanh(sd) / sd;
+    const double sd = qsqrt(-d);
+    g = qdiv(atanh(sd), sd);
   }
   return f * g * inv_sqrt(x);
 }
@@ -123,11 +126,11 @@ BHA_CALL double carlson_rj(double x, double y, double z, double p) {
   if (x > y) { const double t = x; x = y; y = t; }
   if (y > z) { const double t = y; y = z; z = t; }
   if (x > y) { const double t = x; x = y; y = t; }
-  const double a = 1.0 / (y - p);
+  const double a = qdiv(1.0, y - p);
   const double b = a * (z - y) * (y - x);
   const double pt = y + b;
-  const double rho = x * z / y;
-  const double tau = p * pt / y;
+  const double rho = qdiv(x * z, y);
+  const double tau = qdiv(p * pt, y);
   return a * (b * carlson_rj_pos(x, y, z, pt) + 3.0 * (carlson_rc(rho, tau) - carlson_rf(x, y, z)));
 }
 
@@ -137,11 +140,12 @@ BHA_CALL void carlson_rj2(double x, double y, double z, double p1, double p2, do
   const double dxyz1 = (p1 - x) * (p1 - y) * (p1 - z), dxyz2 = (p2 - x) * (p2 - y) * (p2 - z);
   double s1 = 0.0, s2 = 0.0, fac = 1.0, f3 = 1.0;
   for (int it = 0; it < 60; ++it) {
-    const double sx = sqrt(x), sy = sqrt(y), sz = sqrt(z), sp1 = sqrt(p1), sp2 = sqrt(p2);
+    const double sx = qsqrt(x), sy = qsqrt(y), sz = qsqrt(z), sp1 = qsqrt(p1), sp2 = qsqrt(p2);
     const double lam = sx * sy + sy * sz + sz * sx;
     const double d1 = (sp1 + sx) * (sp1 + sy) * (sp1 + sz), d2 = (sp2 + sx) * (sp2 + sy) * (sp2 + sz);
-    s1 += fac * carlson_rc1(f3 * dxyz1 / (d1 * d1)) / d1;
-    s2 += fac * carlson_rc1(f3 * dxyz2 / (d2 * d2)) / d2;
+    const double i1 = qrcp(d1), i2 = qrcp(d2);
+    s1 += fac * carlson_rc1(f3 * dxyz1 * (i1 * i1)) * i1;
+    s2 += fac * carlson_rc1(f3 * dxyz2 * (i2 * i2)) * i2;
     fac *= 0.25;
     f3 *= 1.0 / 64.0;
     x = 0.25 * (x + lam);
@@ -150,13 +154,14 @@ BHA_CALL void carlson_rj2(double x, double y, double z, double p1, double p2, do
     p1 = 0.25 * (p1 + lam);
     p2 = 0.25 * (p2 + lam);
     const double A1 = (x + y + z + 2.0 * p1) * 0.2, A2 = (x + y + z + 2.0 * p2) * 0.2;
-    const double X1 = (A1 - x) / A1, Y1 = (A1 - y) / A1, Z1 = (A1 - z) / A1, P1 = (A1 - p1) / A1;
-    const double X2 = (A2 - x) / A2, Y2 = (A2 - y) / A2, Z2 = (A2 - z) / A2, P2 = (A2 - p2) / A2;
+    const double X1 = A1 - x, Y1 = A1 - y, Z1 = A1 - z, P1 = A1 - p1;
+    const double X2 = A2 - x, Y2 = A2 - y, Z2 = A2 - z, P2 = A2 - p2;
     const double e1 = fmax(fmax(fabs(X1), fabs(Y1)), fmax(fabs(Z1), fabs(P1)));
     const double e2 = fmax(fmax(fabs(X2), fabs(Y2)), fmax(fabs(Z2), fabs(P2)));
-    if (fmax(e1, e2) < 1e-3) {
-      o1 = 6.0 * s1 + fac * rj_series(X1, Y1, Z1, P1) * inv_sqrt(A1) / A1;
-      o2 = 6.0 * s2 + fac * rj_series(X2, Y2, Z2, P2) * inv_sqrt(A2) / A2;
+    if (e1 < 8e-3 * A1 && e2 < 8e-3 * A2) {
+      const double r1 = qrcp(A1), r2 = qrcp(A2);
+      o1 = 6.0 * s1 + fac * rj_series(X1 * r1, Y1 * r1, Z1 * r1, P1 * r1) * inv_sqrt(A1) * r1;
+      o2 = 6.0 * s2 + fac * rj_series(X2 * r2, Y2 * r2, Z2 * r2, P2 * r2) * inv_sqrt(A2) * r2;
       return;
     }
   }
@@ -175,7 +180,7 @@ BHA_CALL void sncndn(double u, double m1, double &sn, double &cn, double &dn) {
 #pragma unroll 1
   for (int k = 0; k < kMax; ++k) {
     em[k] = a;
-    emc = sqrt(emc);
+    emc = qsqrt(emc);
     en[k] = emc;
     c = 0.5 * (a + emc);
     if (fabs(a - emc) <= 1e-15 * a) {
@@ -190,30 +195,30 @@ BHA_CALL void sncndn(double u, double m1, double &sn, double &cn, double &dn) {
   cn = cos(v);
   dn = 1.0;
   if (sn != 0.0) {
-    double t = cn / sn, cc = c * t;
+    double t = qdiv(cn, sn), cc = c * t;
 #pragma unroll 1
     for (int k = n - 1; k >= 0; --k) {
       const double b = em[k];
       t *= cc;
       cc *= dn;
-      dn = (en[k] + t) / (b + t);
-      t = cc / b;
+      dn = qdiv(en[k] + t, b + t);
+      t = qdiv(cc, b);
     }
-    const double r = 1.0 / sqrt(cc * cc + 1.0);
+    const double r = inv_sqrt(cc * cc + 1.0);
     sn = sn >= 0.0 ? r : -r;
     cn = cc * sn;
   }
 }
 
 // sn, cn, dn(u | m) for m = 1 - m1 < 0 (m1 > 1): Abramowitz & Stegun 16.10.2-4,
-// sn(u | m) = sd(u sqrt(m1) | mu) / sqrt(m1), cn = cd, dn = nd, mu = 1 - 1 / m1.
+// sn(u | m) = sd(u qsqrt(m1) | mu) / qsqrt(m1), cn = cd, dn = nd, mu = 1 - 1 / m1.
 BHM_HD void sncndn_neg(double u, double m1, double &sn, double &cn, double &dn) {
-  const double r = sqrt(m1);
+  const double r = qsqrt(m1);
   double s, c, d;
-  sncndn(u * r, 1.0 / m1, s, c, d);
-  sn = s / (d * r);
-  cn = c / d;
-  dn = 1.0 / d;
+  sncndn(u * r, qdiv(1.0, m1), s, c, d);
+  dn = qdiv(1.0, d);
+  sn = qdiv(s, d * r);
+  cn = qdiv(c, d);
 }
 
 // Bulirsch's complete integral cel(kc, p, a, b) (mino_solve.cuh; p < 0 gives
@@ -221,7 +226,7 @@ BHM_HD void sncndn_neg(double u, double m1, double &sn, double &cn, double &dn) 
 BHA_CALL double bulirsch_cel(double kc, double p, double a, double b) { return bhmino::cel<double>(kc, p, a, b); }
 
 // The complete Q(n; pi/2 | m) = int_0^(pi/2) sin^2 / ((1 - n sin^2) dn) = cel(sqrt m1, 1 - n, 0, 1).
-BHM_HD double ellip_qc(double n, double m1) { return bulirsch_cel(sqrt(m1), 1.0 - n, 0.0, 1.0); }
+BHM_HD double ellip_qc(double n, double m1) { return bulirsch_cel(qsqrt(m1), 1.0 - n, 0.0, 1.0); }
 
 // Incomplete F(phi | m) for phi in [-pi/2, pi/2] from sin, cos (Carlson's form).
 BHM_HD double ellip_f(double s, double c, double m1) { return s * carlson_rf(c * c, c * c + m1 * s * s, 1.0); }
@@ -239,7 +244,7 @@ BHA_PCALL double ellip_q_sc(double n, double s, double c, double m1, double &qc)
 // The same with the complement nc = 1 - n given (1 - n s^2 = c^2 + nc s^2 with
 // no cancellation): the polar motion's n = z+ tends to 1 as lambda -> 0, and
 // 1 - z+ ~ lambda^2 drops below FP64 resolution when formed from z+.
-BHM_HD double ellip_qc_nc(double nc, double m1) { return bulirsch_cel(sqrt(m1), nc, 0.0, 1.0); }
+BHM_HD double ellip_qc_nc(double nc, double m1) { return bulirsch_cel(qsqrt(m1), nc, 0.0, 1.0); }
 BHM_HD double q_part_nc(double nc, double s, double c, double m1) {
   return s * s * s * carlson_rj(c * c, c * c + m1 * s * s, 1.0, c * c + nc * s * s) * (1.0 / 3.0);
 }
@@ -291,7 +296,7 @@ BHM_HD double newton_root(double p2, double p1, double p0, double r) {
     const double r2 = r * r;
     const double R = (r2 + p2) * r2 + p1 * r + p0;
     const double dR = 4.0 * r2 * r + 2.0 * p2 * r + p1;
-    const double dr = R / dR;
+    const double dr = qdiv(R, dR);
     r -= dr;
     if (fabs(dr) <= 1e-15 * fabs(r)) break;
   }
@@ -308,23 +313,24 @@ BHA_CALL bool ferrari_factor(double p2, double p1, double p0, double &al, double
   const double disc = 0.25 * Q * Q + P * P * P * (1.0 / 27.0);
   double t;
   if (disc < 0.0) {
-    const double rr = sqrt(-P * (1.0 / 3.0));
-    const double cc = fmax(-1.0, fmin(1.0, (-0.5 * Q) / (rr * rr * rr)));
+    const double rr = qsqrt(-P * (1.0 / 3.0));
+    const double cc = fmax(-1.0, fmin(1.0, qdiv(-0.5 * Q, rr * rr * rr)));
     t = 2.0 * rr * cos(acos(cc) * (1.0 / 3.0));
   } else {
-    const double sd = sqrt(disc);
+    const double sd = qsqrt(disc);
     t = cbrt(-0.5 * Q + sd) + cbrt(-0.5 * Q - sd);
   }
   double z = t - (2.0 / 3.0) * p2;
   for (int it = 0; it < 3; ++it) {
     const double f = ((z + 2.0 * p2) * z + (p2 * p2 - 4.0 * p0)) * z - p1 * p1;
     const double df = (3.0 * z + 4.0 * p2) * z + (p2 * p2 - 4.0 * p0);
-    if (df != 0.0) z -= f / df;
+    if (df != 0.0) z -= qdiv(f, df);
   }
   if (!(z > 0.0)) return false;
-  al = sqrt(z);
-  be = 0.5 * (p2 + z - p1 / al);
-  ga = 0.5 * (p2 + z + p1 / al);
+  al = qsqrt(z);
+  const double p1a = qdiv(p1, al);
+  be = 0.5 * (p2 + z - p1a);
+  ga = 0.5 * (p2 + z + p1a);
   return true;
 }
 
@@ -339,21 +345,21 @@ BHA_CALL int ferrari(double p2, double p1, double p0, double re[4], double &c, d
   const double d1 = z - 4.0 * be, d2 = z - 4.0 * ga;
   int n = 0;
   if (d1 >= 0.0) {
-    const double s = sqrt(d1);
+    const double s = qsqrt(d1);
     re[n++] = 0.5 * (-al - s);
     re[n++] = 0.5 * (-al + s);
   } else {
     c = -0.5 * al;
-    d = 0.5 * sqrt(-d1);
+    d = 0.5 * qsqrt(-d1);
     mod2 = be;
   }
   if (d2 >= 0.0) {
-    const double s = sqrt(d2);
+    const double s = qsqrt(d2);
     re[n++] = 0.5 * (al - s);
     re[n++] = 0.5 * (al + s);
   } else {
     c = 0.5 * al;
-    d = 0.5 * sqrt(-d2);
+    d = 0.5 * qsqrt(-d2);
     mod2 = ga;
   }
   for (int k = 0; k < n; ++k) re[k] = newton_root(p2, p1, p0, re[k]);
@@ -374,18 +380,19 @@ BHA_SCALL double x_of_r(const RadSol &q, double r, Amp &a) {
     const double A = q.A, B = q.B;
     const double num = A * (r - q.r1) - B * (r - q.r2);
     const double den = A * (r - q.r1) + B * (r - q.r2);
-    a.c = num / den;
-    a.s = 2.0 * sqrt(A * B * (r - q.r1) * (r - q.r2)) / den;
-    a.d = sqrt(a.c * a.c + q.m1 * a.s * a.s);
+    a.c = qdiv(num, den);
+    a.s = qdiv(2.0 * qsqrt(A * B * (r - q.r1) * (r - q.r2)), den);
+    a.d = qsqrt(a.c * a.c + q.m1 * a.s * a.s);
     const double F = ellip_f(a.s, fabs(a.c), q.m1);
     return (a.c < 0.0) ? 2.0 * carlson_rf(0.0, q.m1, 1.0) - F : F;
   }
   const double r31 = q.r3 - q.r1, r41 = q.r4 - q.r1, r43 = q.r4 - q.r3;
-  const double s2 = r31 * (r - q.r4) / (r41 * (r - q.r3));
-  const double c2 = r43 * (r - q.r1) / (r41 * (r - q.r3));
-  a.s = sqrt(s2);
-  a.c = sqrt(c2);
-  a.d = sqrt(c2 + q.m1 * s2);
+  const double dd = r41 * (r - q.r3);
+  const double s2 = qdiv(r31 * (r - q.r4), dd);
+  const double c2 = qdiv(r43 * (r - q.r1), dd);
+  a.s = qsqrt(s2);
+  a.c = qsqrt(c2);
+  a.d = qsqrt(c2 + q.m1 * s2);
   return a.s * carlson_rf(c2, c2 + q.m1 * s2, 1.0);
 }
 
@@ -410,13 +417,13 @@ BHA_SCALL RadSol radial(double p2, double p1, double p0, double r_plus, double r
   const double Rm = rm > r_plus ? (rm * rm + p2) * rm * rm + p1 * rm + p0 : 1.0;
   if (rm > r_plus && Rm < 0.0) {
     const double d2 = 12.0 * rm * rm + 2.0 * p2;
-    const double off = sqrt(-2.0 * Rm / fmax(d2, 1e-300));
+    const double off = qsqrt(qdiv(-2.0 * Rm, fmax(d2, 1e-290)));
     const double r4 = newton_root(p2, p1, p0, rm + off);
     if (!(r4 > r_hor) || !(r4 < r_obs) || !crosses) return q;
     const double r3 = newton_root(p2, p1, p0, rm - off);
     if (!(r3 < r4)) return q;
-    const double sm = -(r3 + r4), pr = p0 / (r3 * r4);
-    const double sq = sqrt(fmax(sm * sm - 4.0 * pr, 0.0));
+    const double sm = -(r3 + r4), pr = qdiv(p0, r3 * r4);
+    const double sq = qsqrt(fmax(sm * sm - 4.0 * pr, 0.0));
     q.r1 = 0.5 * (sm - sq);
     q.r2 = 0.5 * (sm + sq);
     q.r3 = r3;
@@ -442,7 +449,7 @@ BHA_SCALL RadSol radial(double p2, double p1, double p0, double r_plus, double r
       const double dd = mod2 - c * c;
       if (!(dd > 0.0) || !(q.r2 < r_hor)) return q;
       q.r3 = c;
-      q.r4 = sqrt(dd);
+      q.r4 = qsqrt(dd);
       q.type = kP2;
     } else {
       return q;
@@ -452,35 +459,35 @@ BHA_SCALL RadSol radial(double p2, double p1, double p0, double r_plus, double r
   if (q.type == kP2) {
     const double c_ = q.r3, d_ = q.r4;
     const double u2 = c_ - q.r2, u1 = c_ - q.r1, d2 = d_ * d_;
-    const double A = sqrt(u2 * u2 + d2), B = sqrt(u1 * u1 + d2);
+    const double A = qsqrt(u2 * u2 + d2), B = qsqrt(u1 * u1 + d2);
     const double r21 = q.r2 - q.r1;
     // 1 - m = r21^2 ((A - u2) + (B - u1)) ((A + u2) + (B + u1)) / ((A + B)^2 4 A B), each sum without cancellation
-    const double amu2 = u2 > 0.0 ? d2 / (A + u2) : A - u2;
-    const double bmu1 = u1 > 0.0 ? d2 / (B + u1) : B - u1;
-    const double apu2 = u2 > 0.0 ? A + u2 : d2 / (A - u2);
-    const double bpu1 = u1 > 0.0 ? B + u1 : d2 / (B - u1);
+    const double amu2 = u2 > 0.0 ? qdiv(d2, A + u2) : A - u2;
+    const double bmu1 = u1 > 0.0 ? qdiv(d2, B + u1) : B - u1;
+    const double apu2 = u2 > 0.0 ? A + u2 : qdiv(d2, A - u2);
+    const double bpu1 = u1 > 0.0 ? B + u1 : qdiv(d2, B - u1);
     q.A = A;
     q.B = B;
-    q.m1 = r21 * r21 * (amu2 + bmu1) * (apu2 + bpu1) / ((A + B) * (A + B) * 4.0 * A * B);
-    q.sc = sqrt(A * B);
+    q.m1 = qdiv(r21 * r21 * (amu2 + bmu1) * (apu2 + bpu1), (A + B) * (A + B) * 4.0 * A * B);
+    q.sc = qsqrt(A * B);
     q.X0 = x_of_r(q, r_obs, q.a0);
     q.dir = -1.0;
-    q.tau_end = (q.X0 - x_of_r(q, r_hor, a_h)) / q.sc;
+    q.tau_end = qdiv(q.X0 - x_of_r(q, r_hor, a_h), q.sc);
   } else {
     const double r31 = q.r3 - q.r1, r42 = q.r4 - q.r2, r21 = q.r2 - q.r1, r43 = q.r4 - q.r3;
-    q.m1 = r21 * r43 / (r31 * r42);
-    q.sc = 0.5 * sqrt(r31 * r42);
+    q.m1 = qdiv(r21 * r43, r31 * r42);
+    q.sc = 0.5 * qsqrt(r31 * r42);
     const double x_obs = x_of_r(q, r_obs, q.a0);
     if (q.type == kS) {  // X runs from -X(r_obs) through the turning point (X = 0) to X(r_esc)
       q.X0 = -x_obs;
       q.a0.s = -q.a0.s;
       q.dir = 1.0;
       q.X_end = x_of_r(q, r_esc, q.a_end);
-      q.tau_end = (x_obs + q.X_end) / q.sc;
+      q.tau_end = qdiv(x_obs + q.X_end, q.sc);
     } else {
       q.X0 = x_obs;
       q.dir = -1.0;
-      q.tau_end = (x_obs - x_of_r(q, r_hor, a_h)) / q.sc;
+      q.tau_end = qdiv(x_obs - x_of_r(q, r_hor, a_h), q.sc);
     }
   }
   return q;
@@ -491,10 +498,10 @@ BHM_HD double x_at(const RadSol &q, double tau) { return q.X0 + q.dir * q.sc * t
 // r from the amplitude at X (S, P4: sn; P2: cn).
 BHM_HD double r_of_amp(const RadSol &q, const Amp &a) {
   if (q.type == kP2)
-    return ((q.B * q.r2 - q.A * q.r1) + (q.B * q.r2 + q.A * q.r1) * a.c) / ((q.B - q.A) + (q.B + q.A) * a.c);
+    return qdiv((q.B * q.r2 - q.A * q.r1) + (q.B * q.r2 + q.A * q.r1) * a.c, (q.B - q.A) + (q.B + q.A) * a.c);
   const double s2 = a.s * a.s;
   const double r31 = q.r3 - q.r1, r41 = q.r4 - q.r1;
-  return (q.r4 * r31 - q.r3 * r41 * s2) / (r31 - r41 * s2);
+  return qdiv(q.r4 * r31 - q.r3 * r41 * s2, r31 - r41 * s2);
 }
 
 BHM_HD Amp amp_at(const RadSol &q, double X) {
@@ -524,14 +531,14 @@ struct JPole {
 };
 
 BHM_HD double p2_g(const JPole &J, const Amp &a) {
-  const double t = a.s / a.d;
-  if (J.Aq * J.Cq > 0.0) return atan(t * sqrt(J.Cq / J.Aq)) / sqrt(J.Aq * J.Cq);
-  const double p1 = sqrt(-J.Aq / J.Cq);
-  return log(fabs((t - p1) / (t + p1))) / (2.0 * p1 * J.Cq);
+  const double t = qdiv(a.s, a.d);
+  if (J.Aq * J.Cq > 0.0) return qdiv(atan(t * qsqrt(qdiv(J.Cq, J.Aq))), qsqrt(J.Aq * J.Cq));
+  const double p1 = qsqrt(qdiv(-J.Aq, J.Cq));
+  return qdiv(log(fabs(qdiv(t - p1, t + p1))), 2.0 * p1 * J.Cq);
 }
 
 BHM_HD double p2_r1(JPole &J, double m1, double X, const Amp &a) {
-  return (X + J.par * ellip_q_sc(J.par, a.s, a.c, m1, J.qc)) / J.Aq - J.al * p2_g(J, a);
+  return qdiv(X + J.par * ellip_q_sc(J.par, a.s, a.c, m1, J.qc), J.Aq) - J.al * p2_g(J, a);
 }
 
 BHA_PCALL void j_poles(const RadSol &q, double r_plus, double r_minus, JPole &jp, JPole &jm) {
@@ -544,28 +551,28 @@ BHA_PCALL void j_poles(const RadSol &q, double r_plus, double r_minus, JPole &jp
       const double A = q.A, B = q.B, r21 = q.r2 - q.r1;
       const double D0 = B * (q.r2 - rpm) - A * (q.r1 - rpm);
       const double D1 = B * (q.r2 - rpm) + A * (q.r1 - rpm);
-      J.al = D1 / D0;
+      J.al = qdiv(D1, D0);
       const double al2 = J.al * J.al;
-      J.par = al2 / (al2 - 1.0);
+      J.par = qdiv(al2, al2 - 1.0);
       J.Aq = 1.0 - al2;
       J.Cq = J.Aq * (1.0 - q.m1) + al2;
-      J.k1 = (B + A) / (D1 * q.sc);
-      J.k2 = -2.0 * A * B * r21 / (D1 * D0 * q.sc);
+      J.k1 = qdiv(B + A, D1 * q.sc);
+      J.k2 = qdiv(-2.0 * A * B * r21, D1 * D0 * q.sc);
       J.t0 = p2_r1(J, q.m1, q.X0, q.a0);
     } else {
       const double r31 = q.r3 - q.r1, r41 = q.r4 - q.r1;
-      J.par = r41 * (q.r3 - rpm) / (r31 * (q.r4 - rpm));
-      J.k1 = q.dir / ((q.r4 - rpm) * q.sc);
-      J.k2 = J.par - r41 / r31;
+      J.par = qdiv(r41 * (q.r3 - rpm), r31 * (q.r4 - rpm));
+      J.k1 = qdiv(q.dir, (q.r4 - rpm) * q.sc);
+      J.k2 = J.par - qdiv(r41, r31);
     }
   }
   if (q.type != kP2) ellip_q2_sc(jp.par, jm.par, q.a0.s, q.a0.c, q.m1, jp.t0, jm.t0);
 }
 
-// The integrand of Q: sin^2 / ((1 - n sin^2) sqrt(cos^2 + m1 sin^2)).
+// The integrand of Q: sin^2 / ((1 - n sin^2) qsqrt(cos^2 + m1 sin^2)).
 BHM_HD double q_integrand(double n, double m1, double ph) {
   const double s = sin(ph), c = cos(ph), s2 = s * s;
-  return s2 / ((1.0 - n * s2) * sqrt(c * c + m1 * s2));
+  return qdiv(s2, (1.0 - n * s2) * qsqrt(c * c + m1 * s2));
 }
 
 // S rays at the escape radius: the amplitude there differs little from the
@@ -610,16 +617,16 @@ BHA_PCALL void j_eval_escape(const RadSol &q, JPole &jp, JPole &jm, double &vp, 
 
 // ---- polar motion -------------------------------------------------------------------
 //
-// u = sqrt(z+) sin chi, Phi(chi) = F(chi | -mm / w) / sqrt(w) the Mino time
+// u = qsqrt(z+) sin chi, Phi(chi) = F(chi | -mm / w) / qsqrt(w) the Mino time
 // since chi = 0; the ray starts at Phi = phi_start and crosses the equator at
 // chi = j pi, i.e. at tau = j period - phi_start.
 
 struct PolSol {
   bool crosses;
-  double zp, w, mm, sz;  // U = (z+ - u^2)(a^2 u^2 + w), mm = a^2 z+, sz = sqrt(z+)
+  double zp, w, mm, sz;  // U = (z+ - u^2)(a^2 u^2 + w), mm = a^2 z+, sz = qsqrt(z+)
   double zc;             // 1 - z+, formed without cancellation
   double m1;             // complementary parameter of -mm / w
-  double sw;             // sqrt(w)
+  double sw;             // qsqrt(w)
   double phi_start;      // Phi at the observer [Mino time]
   double tau1, period;   // first crossing, time between crossings
   double s0, c0;         // chi at the observer: sin, cos (chi0 in (-pi/2, 3 pi/2); cos has the sign of du/dtau)
@@ -632,18 +639,18 @@ BHA_SCALL PolSol polar(double a2, double qTh, double lam, double u0, double pu0)
   t.crosses = c0 > 0.0;
   if (!t.crosses) return t;
   const double b2 = a2 - qTh;
-  const double sq = sqrt(b2 * b2 + 4.0 * a2 * c0);
-  t.zp = (b2 > 0.0) ? (b2 + sq) / (2.0 * a2) : 2.0 * c0 / (sq - b2);
-  t.zc = 2.0 * lam * lam / (a2 + qTh + sq);  // (a^2 + qTh)^2 - sq^2 = 4 a^2 lambda^2
-  t.w = c0 / t.zp;
+  const double sq = qsqrt(b2 * b2 + 4.0 * a2 * c0);
+  t.zp = (b2 > 0.0) ? qdiv(b2 + sq, 2.0 * a2) : qdiv(2.0 * c0, sq - b2);
+  t.zc = qdiv(2.0 * lam * lam, a2 + qTh + sq);  // (a^2 + qTh)^2 - sq^2 = 4 a^2 lambda^2
+  t.w = qdiv(c0, t.zp);
   t.mm = a2 * t.zp;
-  t.sz = sqrt(t.zp);
-  t.m1 = 1.0 + t.mm / t.w;
-  t.sw = sqrt(t.w);
-  const double s0 = fmax(-1.0, fmin(1.0, u0 / t.sz));
+  t.sz = qsqrt(t.zp);
+  t.m1 = 1.0 + qdiv(t.mm, t.w);
+  t.sw = qsqrt(t.w);
+  const double s0 = fmax(-1.0, fmin(1.0, qdiv(u0, t.sz)));
   // cos^2 chi_obs from U(u0) = pu0^2 = (z+ - u0^2)(a^2 u0^2 + w): exact where
   // 1 - s0^2 would cancel (an observer at a polar turning point, beta ~ 0)
-  const double c2 = pu0 * pu0 / ((a2 * u0 * u0 + t.w) * t.zp);
+  const double c2 = qdiv(pu0 * pu0, (a2 * u0 * u0 + t.w) * t.zp);
   const double phi_x = s0 * carlson_rf(t.w * c2, t.w + t.mm * s0 * s0, t.w);
   const double K = bhmino::quarter_period<double>(t.w, t.mm);
   t.phi_start = (pu0 >= 0.0) ? phi_x : 2.0 * K - phi_x;
@@ -651,7 +658,7 @@ BHA_SCALL PolSol polar(double a2, double qTh, double lam, double u0, double pu0)
   t.tau1 = ((pu0 * u0) < 0.0) ? fabs(phi_x) : 2.0 * K - fabs(phi_x);
   t.period = 2.0 * K;
   t.s0 = s0;
-  t.c0 = (pu0 >= 0.0 ? 1.0 : -1.0) * sqrt(c2);  // dchi/dtau > 0: cos chi has the sign of du/dtau
+  t.c0 = (pu0 >= 0.0 ? 1.0 : -1.0) * qsqrt(c2);  // dchi/dtau > 0: cos chi has the sign of du/dtau
   t.q0 = NAN;
   t.qc = NAN;
   return t;
@@ -663,7 +670,7 @@ BHM_HD void polar_q0(PolSol &t) {
 }
 
 // lambda int_0^tau dtau / (1 - u^2) at an equatorial crossing (chi = j pi,
-// Q(z+; j pi) = 2 j Q(pi/2)): lambda (tau + (z+ / sqrt(w)) (2 j Q_c - Q(chi0))).
+// Q(z+; j pi) = 2 j Q(pi/2)): lambda (tau + (z+ / qsqrt(w)) (2 j Q_c - Q(chi0))).
 // With 1 - z+ == 0 (lambda == 0, or lambda^2 below the smallest double) the
 // integral is its limit lambda -> 0 from the side of lambda's sign: a turn by
 // copysign(pi, lambda) at each pass over the pole (chi = pi/2 + j pi), so
@@ -677,27 +684,27 @@ BHM_HD double pole_turns(const PolSol &t, double lam, double tau) {
 BHA_PCALL double phi_theta_crossing(PolSol &t, double lam, double tau) {
   if (!(t.zc > 0.0)) return pole_turns(t, lam, tau);
   polar_q0(t);
-  const double j = rint((t.phi_start + tau) / t.period);
-  return lam * (tau + t.zp / t.sw * (2.0 * j * t.qc - t.q0));
+  const double j = rint(qdiv(t.phi_start + tau, t.period));
+  return lam * (tau + qdiv(t.zp, t.sw) * (2.0 * j * t.qc - t.q0));
 }
 
 // u, du/dtau and lambda int_0^tau dtau / (1 - u^2) at any tau.
 BHA_PCALL void polar_at(PolSol &t, double lam, double tau, double &u, double &pu, double &phi_th) {
   const double total = t.phi_start + tau;
-  const double j = floor(total / t.period);
+  const double j = floor(qdiv(total, t.period));
   double sa, ca, da;  // amplitude in [0, pi): sa >= 0
   sncndn_neg(t.sw * (total - j * t.period), t.m1, sa, ca, da);
   sa = fabs(sa);
   const double sg = fmod(j, 2.0) != 0.0 ? -1.0 : 1.0;
   u = sg * t.sz * sa;
-  pu = sg * t.sz * ca * sqrt(t.w + t.mm * sa * sa);
+  pu = sg * t.sz * ca * qsqrt(t.w + t.mm * sa * sa);
   if (!(t.zc > 0.0)) {
     phi_th = pole_turns(t, lam, tau);
     return;
   }
   polar_q0(t);
   const double q = 2.0 * j * t.qc + ellip_q_sc_nc(t.zc, sa, ca, t.m1, t.qc);
-  phi_th = lam * (tau + t.zp / t.sw * (q - t.q0));
+  phi_th = lam * (tau + qdiv(t.zp, t.sw) * (q - t.q0));
 }
 
 }  // namespace bhan

@@ -35,6 +35,7 @@
 #include <cmath>
 
 #ifdef __CUDACC__
+#include "ieee_fp64.cuh"
 #define BHM_HD __device__ __forceinline__
 #else
 #define BHM_HD inline
@@ -105,35 +106,63 @@ __constant__
 #endif
 constexpr int kGlUnroll = BHM_GL_UNROLL;
 
-// a / b: IEEE division in FP64 (the closed-form tracer's results stay those
-// of plain division); in FP32 on the device the 2-ulp __fdividef, ample for
-// elliptic integrals carried to FP32's ~1e-7.
+// a / b and sqrt(x): correctly rounded in FP64, on the device without a branch
+// (ieee_fp64.cuh: the solve's operands are far from the ends of the range); in
+// FP32 on the device the 2-ulp __fdividef, ample for elliptic integrals carried
+// to FP32's ~1e-7. qrcp: 1 / b to an ulp, for several quotients by one value.
 template <class T>
 BHM_HD T qdiv(T a, T b) {
 #ifdef __CUDA_ARCH__
-  if constexpr (sizeof(T) == 4) return __fdividef(a, b);
+  if constexpr (sizeof(T) == 4)
+    return __fdividef(a, b);
+  else
+    return bhk::div_rn(a, b);
 #endif
   return a / b;
 }
+template <class T>
+BHM_HD T qsqrt(T x) {
+#ifdef __CUDA_ARCH__
+  if constexpr (sizeof(T) == 8) {
+    const double s = bhk::sqrt_rn(x);
+    return x < 0.0 ? NAN : s;
+  }
+#endif
+  return sqrt(x);
+}
+BHM_HD double qrcp(double b) {
+#ifdef __CUDA_ARCH__
+  return bhk::rcp_near(b);
+#else
+  return 1.0 / b;
+#endif
+}
 
 // Carlson's symmetric integral R_F(x, y, z) = 1/2 int_0^inf dt / sqrt((t+x)(t+y)(t+z)),
-// x, y, z >= 0 with at most one zero.
+// x, y, z >= 0 with at most one zero. FP64 carries the expansion about the mean
+// to degree 7 (DLMF 19.36.1) and so stops a duplication or two earlier.
 template <class T>
 BHM_HD T carlson_rf(T x, T y, T z) {
-  const T tol = sizeof(T) == 4 ? T(3e-2) : T(1e-3);  // series error ~ tol^6
+  constexpr bool wide = sizeof(T) == 8;
+  const T tol = wide ? T(8e-3) : T(3e-2);  // series error ~ 0.02 tol^8, tol^6
   for (int it = 0; it < 60; ++it) {
-    const T sx = sqrt(x), sy = sqrt(y), sz = sqrt(z);
+    const T sx = qsqrt(x), sy = qsqrt(y), sz = qsqrt(z);
     const T lam = sx * sy + sy * sz + sz * sx;
     x = T(0.25) * (x + lam);
     y = T(0.25) * (y + lam);
     z = T(0.25) * (z + lam);
     const T A = (x + y + z) * T(1.0 / 3.0);
+    if constexpr (wide) {
+      if (!(fmax(fabs(x - A), fmax(fabs(y - A), fabs(z - A))) < tol * A)) continue;
+    }
     const T dx = T(1) - qdiv(x, A), dy = T(1) - qdiv(y, A);
     const T dz = -(dx + dy);
-    if (fmax(fabs(dx), fmax(fabs(dy), fabs(dz))) < tol) {
+    if (wide || fmax(fabs(dx), fmax(fabs(dy), fabs(dz))) < tol) {
       const T e2 = dx * dy - dz * dz, e3 = dx * dy * dz;
-      return (T(1) - T(0.1) * e2 + e3 * T(1.0 / 14.0) + e2 * e2 * T(1.0 / 24.0) - e2 * e3 * T(3.0 / 44.0)) *
-             inv_sqrt(A);
+      T f = T(1) - T(0.1) * e2 + e3 * T(1.0 / 14.0) + e2 * e2 * T(1.0 / 24.0) - e2 * e3 * T(3.0 / 44.0);
+      if constexpr (wide)
+        f += e3 * e3 * T(3.0 / 104.0) - e2 * e2 * e2 * T(5.0 / 208.0) + e2 * e2 * e3 * T(1.0 / 16.0);
+      return f * inv_sqrt(A);
     }
   }
   return T(NAN);
@@ -144,12 +173,13 @@ BHM_HD T carlson_rf(T x, T y, T z) {
 template <class T>
 BHM_HD T quarter_period(T w, T m) {
   const T eps = sizeof(T) == 4 ? T(1e-7) : T(1e-15);
-  T a = sqrt(w + m), g = sqrt(w);
+  T a = qsqrt(w + m), g = qsqrt(w);
   for (int it = 0; it < 12 && fabs(a - g) > eps * a; ++it) {
     const T an = T(0.5) * (a + g);
-    g = sqrt(a * g);
+    g = qsqrt(a * g);
     a = an;
   }
+  if constexpr (sizeof(T) == 8) return qdiv(T(1.5707963267948966), T(0.5) * (a + g));
   return T(1.5707963267948966) / (T(0.5) * (a + g));
 }
 
@@ -166,36 +196,42 @@ BHM_HD T rc1(T e) {
   if (fabs(e) < T(1e-3))
     return T(1) - e * (T(1.0 / 3.0) - e * (T(0.2) - e * (T(1.0 / 7.0) - e * (T(1.0 / 9.0) - e * T(1.0 / 11.0)))));
   if (e > T(0)) {
-    const T se = sqrt(e);
+    const T se = qsqrt(e);
     return qdiv(atan(se), se);
   }
-  const T se = sqrt(-e);
+  const T se = qsqrt(-e);
   return qdiv(atanh(se), se);
 }
 
-// The fifth-order expansion of R_J about the mean of its arguments.
+// The expansion of R_J about the mean of its arguments: degree 5 in FP32, 7 in
+// FP64 (DLMF 19.36.2).
 template <class T>
 BHM_HD T rj_series(T X, T Y, T Z, T P) {
   const T E2 = X * Y + X * Z + Y * Z - T(3) * P * P;
   const T E3 = X * Y * Z + T(2) * E2 * P + T(4) * P * P * P;
   const T E4 = (T(2) * X * Y * Z + E2 * P + T(3) * P * P * P) * P;
   const T E5 = X * Y * Z * P * P;
-  return T(1) - T(3.0 / 14.0) * E2 + E3 * T(1.0 / 6.0) + T(9.0 / 88.0) * E2 * E2 - T(3.0 / 22.0) * E4 -
-         T(9.0 / 52.0) * E2 * E3 + T(3.0 / 26.0) * E5;
+  const T f = T(1) - T(3.0 / 14.0) * E2 + E3 * T(1.0 / 6.0) + T(9.0 / 88.0) * E2 * E2 - T(3.0 / 22.0) * E4 -
+              T(9.0 / 52.0) * E2 * E3 + T(3.0 / 26.0) * E5;
+  if constexpr (sizeof(T) == 8)
+    return f - E2 * E2 * E2 * T(1.0 / 16.0) + E3 * E3 * T(3.0 / 40.0) + E2 * E4 * T(3.0 / 20.0) +
+           E2 * E2 * E3 * T(45.0 / 272.0) - (E3 * E4 + E2 * E5) * T(9.0 / 68.0);
+  return f;
 }
 
 // R_J(x, y, z, p) for p > 0 in Carlson's 1995 form: R_J = 4^-n A_n^-3/2 S +
 // 6 sum_m 4^-m R_C(1, 1 + e_m) / d_m, d_m = (sqrt p_m + sqrt x_m)(sqrt p_m + sqrt y_m)
 // (sqrt p_m + sqrt z_m), e_m = 4^-3m delta / d_m^2, delta = (p - x)(p - y)(p - z):
 // e_m falls by 64 per step, so all but the first terms take the series.
-// The series error is ~tol^6: 1e-3 in FP64, 3e-2 in FP32.
+// The series error is ~tol^8 in FP64 (tol 8e-3), tol^6 in FP32 (3e-2).
 template <class T>
 BHM_HD T rj_pos(T x, T y, T z, T p) {
-  const T tol = sizeof(T) == 4 ? T(3e-2) : T(1e-3);
+  constexpr bool wide = sizeof(T) == 8;
+  const T tol = wide ? T(8e-3) : T(3e-2);
   const T delta = (p - x) * (p - y) * (p - z);
   T sum = T(0), fac = T(1), f3 = T(1);
   for (int it = 0; it < 60; ++it) {
-    const T sx = sqrt(x), sy = sqrt(y), sz = sqrt(z), sp = sqrt(p);
+    const T sx = qsqrt(x), sy = qsqrt(y), sz = qsqrt(z), sp = qsqrt(p);
     const T lam = sx * sy + sy * sz + sz * sx;
     const T d = (sp + sx) * (sp + sy) * (sp + sz);
     sum += qdiv(fac * rc1<T>(qdiv(f3 * delta, d * d)), d);
@@ -206,8 +242,11 @@ BHM_HD T rj_pos(T x, T y, T z, T p) {
     z = T(0.25) * (z + lam);
     p = T(0.25) * (p + lam);
     const T A = (x + y + z + T(2) * p) * T(0.2);
+    if constexpr (wide) {
+      if (!(fmax(fmax(fabs(A - x), fabs(A - y)), fmax(fabs(A - z), fabs(A - p))) < tol * A)) continue;
+    }
     const T X = qdiv(A - x, A), Y = qdiv(A - y, A), Z = qdiv(A - z, A), P = qdiv(A - p, A);
-    if (fmax(fmax(fabs(X), fabs(Y)), fmax(fabs(Z), fabs(P))) < tol)
+    if (wide || fmax(fmax(fabs(X), fabs(Y)), fmax(fabs(Z), fabs(P))) < tol)
       return T(6) * sum + qdiv(fac * rj_series<T>(X, Y, Z, P) * inv_sqrt(A), A);
   }
   return T(NAN);
@@ -223,14 +262,14 @@ BHM_HD T cel(T kc, T p, T a, T b) {
   kc = fabs(kc);
   T e = kc, em = T(1);
   if (p > T(0)) {
-    p = sqrt(p);
+    p = qsqrt(p);
     b = qdiv(b, p);
   } else {
     T f = kc * kc, q = T(1) - f;
     const T g = T(1) - p;
     f -= p;
     q *= (b - a * p);
-    p = sqrt(qdiv(f, g));
+    p = qsqrt(qdiv(f, g));
     a = qdiv(a - b, g);
     b = -qdiv(q, g * g * p) + a * p;
   }
@@ -244,7 +283,7 @@ BHM_HD T cel(T kc, T p, T a, T b) {
     g = em;
     em += kc;
     if (fabs(g - kc) <= g * ca) break;
-    kc = sqrt(e);
+    kc = qsqrt(e);
     kc += kc;
     e = kc * em;
   }
@@ -293,18 +332,18 @@ BHM_HD Polar polar_motion(double a2, double qTh, double lam, double u0, double p
   const double c0 = qTh - lam * lam;  // U(0)
   if (!(c0 > 0.0)) return t;
   const double b2 = a2 - qTh;
-  const double sq = sqrt(b2 * b2 + 4.0 * a2 * c0);
-  t.zp = (b2 > 0.0) ? (b2 + sq) / (2.0 * a2) : 2.0 * c0 / (sq - b2);
-  t.zc = 2.0 * lam * lam / (a2 + qTh + sq);  // (a^2 + qTh)^2 - sq^2 = 4 a^2 lambda^2
-  t.w = c0 / t.zp;
+  const double sq = qsqrt(b2 * b2 + 4.0 * a2 * c0);
+  t.zp = (b2 > 0.0) ? qdiv(b2 + sq, 2.0 * a2) : qdiv(2.0 * c0, sq - b2);
+  t.zc = qdiv(2.0 * lam * lam, a2 + qTh + sq);  // (a^2 + qTh)^2 - sq^2 = 4 a^2 lambda^2
+  t.w = qdiv(c0, t.zp);
   t.mm = a2 * t.zp;
-  t.m1 = 1.0 + t.mm / t.w;
-  t.sw = sqrt(t.w);
-  t.sz = sqrt(t.zp);
-  t.s0 = fmax(-1.0, fmin(1.0, u0 / t.sz));
+  t.m1 = 1.0 + qdiv(t.mm, t.w);
+  t.sw = qsqrt(t.w);
+  t.sz = qsqrt(t.zp);
+  t.s0 = fmax(-1.0, fmin(1.0, qdiv(u0, t.sz)));
   // cos^2 chi0 = pu0^2 / ((a^2 u0^2 + w) z+) (U(u0) = pu0^2): no cancellation near |s0| = 1
-  const double c2 = fmin(1.0, pu0 * pu0 / ((a2 * u0 * u0 + t.w) * t.zp));
-  t.c0 = (pu0 >= 0.0 ? 1.0 : -1.0) * sqrt(c2);
+  const double c2 = fmin(1.0, qdiv(pu0 * pu0, (a2 * u0 * u0 + t.w) * t.zp));
+  t.c0 = (pu0 >= 0.0 ? 1.0 : -1.0) * qsqrt(c2);
   const double phi_x = (double)(T(t.s0) * carlson_rf<T>(T(t.w * c2), T(t.w + t.mm * t.s0 * t.s0), T(t.w)));
   t.K = (double)quarter_period<T>(T(t.w), T(t.mm));
   t.period = 2.0 * t.K;
@@ -313,7 +352,7 @@ BHM_HD Polar polar_motion(double a2, double qTh, double lam, double u0, double p
   t.tau1 = ((pu0 * u0) < 0.0) ? fabs(phi_x) : t.period - fabs(phi_x);
   t.crosses = true;
   if (az) {
-    t.qc = (double)cel<T>(T(sqrt(t.m1)), T(t.zc), T(0), T(1));
+    t.qc = (double)cel<T>(T(qsqrt(t.m1)), T(t.zc), T(0), T(1));
     const double qp = (double)q_part<T>(T(t.zc), T(fabs(t.s0)), T(fabs(t.c0)), T(t.m1));
     // chi0 in [-pi/2, pi/2] (c0 >= 0): Q odd in chi; else chi0 = pi - chi' (Q = 2 Q_c - Q(chi'))
     const double qs = t.s0 < 0.0 ? -qp : qp;
@@ -414,7 +453,7 @@ BHM_HD double largest_dR_root(double p2, double p1) {
   for (int it = 0; it < 2; ++it) {
     const double g = (r * r + p) * r + qq;
     const double dg = 3.0 * r * r + p;
-    if (dg != 0.0) r -= g / dg;
+    if (dg != 0.0) r -= qdiv(g, dg);
   }
   return r;
 }
@@ -596,12 +635,12 @@ BHM_HD Radial radial_motion(double a2, double a2_alam, double C, double r_obs, d
   if (q.r_min > 0.0 && q.R_min < 0.0) {
     // Largest root of R: Newton from the right on the convex branch.
     const double d2 = 12.0 * rm * rm + 2.0 * q.p2;
-    double r = rm + sqrt(-2.0 * q.R_min / fmax(d2, 1e-300));
+    double r = rm + qsqrt(qdiv(-2.0 * q.R_min, fmax(d2, 1e-290)));
     for (int it = 0; it < 100; ++it) {
       const double r2 = r * r;
       const double R = (r2 + q.p2) * r2 + q.p1 * r + q.p0;
       const double dR = 4.0 * r2 * r + 2.0 * q.p2 * r + q.p1;
-      const double dr = R / dR;
+      const double dr = qdiv(R, dR);
       r -= dr;
       if (fabs(dr) <= 1e-15 * r) break;
     }
