@@ -25,6 +25,7 @@
 
 #include <algorithm>
 
+#include "frame_source.cuh"
 #include "image_fp64.cuh"
 #include "launch.h"
 #include "mino_solve.cuh"
@@ -41,6 +42,17 @@ constexpr double kPanel = FAST ? 0.25 : 0.125;
 __device__ __forceinline__ void warp_count(unsigned *stats, int slot, bool pred) {
   const unsigned m = __ballot_sync(kFull, pred);
   if ((threadIdx.x & 31u) == 0 && m) atomicAdd(stats + slot, (unsigned)__popc(m));
+}
+
+// Pixel w of a chunk [p0, p1) of a frame in the order the refinement takes
+// them: the chunk's whole rows [b0, b1) in the tracers' 8 x 4 tiles, so that a
+// warp's rays are neighbours in both directions and take the same branches;
+// the pieces of rows at its ends as they come.
+struct ChunkRows {
+  long long p0, p1, b0, b1;
+};
+__device__ __forceinline__ long long chunk_pixel(const ChunkRows &c, long long w, int width) {
+  return w < c.b0 || w >= c.b1 ? w : c.b0 + bhsrc::tile_pixel(w - c.b0, width, c.b1 - c.b0);
 }
 
 // Resident 128-thread CTAs per SM the refinement is compiled for: 6 caps it
@@ -61,10 +73,11 @@ __global__ void __launch_bounds__(128, FAST ? BH_REFINE_MIN_CTAS : 2) k_surrogat
                                                           const float *__restrict__ head, float min_conf,
                                                           double band, int verify, int *__restrict__ list,
                                                           unsigned int *__restrict__ count,
-                                                          unsigned int *__restrict__ stats, long long p0,
-                                                          long long p1) {
-  const long long pix = p0 + (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  const bool live = pix < p1;
+                                                          unsigned int *__restrict__ stats,
+                                                          const __grid_constant__ ChunkRows chunk) {
+  const long long w = chunk.p0 + (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  const bool live = w < chunk.p1;
+  const long long pix = live ? chunk_pixel(chunk, w, p.width) : 0;
   int reason = 0;  // 0 accepted, 1 confidence, 2 critical band, 3 solve, 4 disagreement
   if (live) {
     const long long i = pix % p.width, j = pix / p.width;
@@ -188,9 +201,10 @@ __global__ void __launch_bounds__(BH_REFINE_THREADS, 1)
     k_surrogate_refine_phased(const __grid_constant__ BhkImageParams p, const __grid_constant__ BhkImageOut o,
                               const float *__restrict__ head, float min_conf, double band, int verify,
                               int *__restrict__ list, unsigned int *__restrict__ count,
-                              unsigned int *__restrict__ stats, long long p0, long long p1) {
-  const long long pix = p0 + (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  const bool live = pix < p1;
+                              unsigned int *__restrict__ stats, const __grid_constant__ ChunkRows chunk) {
+  const long long w = chunk.p0 + (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  const bool live = w < chunk.p1;
+  const long long pix = live ? chunk_pixel(chunk, w, p.width) : 0;
   int reason = 0;  // 0 accepted, 1 confidence, 2 critical band, 3 solve, 4 disagreement
   const double a = p.a;
   double lam = 0.0, qTh = 0.0, pu0 = 0.0;
@@ -357,6 +371,8 @@ extern "C" int bhk_surrogate_refine(const BhkImageParams *p, const BhkImageOut *
   p1 = p1 < p->n_pix ? p1 : p->n_pix;
   if (p1 <= p0) return 0;
   const unsigned blocks = (unsigned)((p1 - p0 + 127) / 128);
+  ChunkRows chunk{p0, p1, (p0 + p->width - 1) / p->width * p->width, p1 / p->width * p->width};
+  if (chunk.b1 < chunk.b0) chunk.b1 = chunk.b0;
   const bool phi = o->phi_hit != nullptr || o->phi_inf != nullptr;
 #if BH_REFINE_PHASED
   // With azimuths the phased kernel is faster (2048^2 frame, serialised:
@@ -365,24 +381,24 @@ extern "C" int bhk_surrogate_refine(const BhkImageParams *p, const BhkImageOut *
   if (!refine_fp64 && phi) {
     const unsigned pb = (unsigned)((p1 - p0 + BH_REFINE_THREADS - 1) / BH_REFINE_THREADS);
     k_surrogate_refine_phased<true, true><<<pb, BH_REFINE_THREADS, 0, s>>>(*p, *o, head, min_conf, band, verify,
-                                                                         list, count, stats, p0, p1);
+                                                                         list, count, stats, chunk);
     return cudaGetLastError() == cudaSuccess ? 0 : -1;
   }
 #endif
   if (refine_fp64) {
     if (phi)
       k_surrogate_refine<false, true><<<blocks, 128, 0, s>>>(*p, *o, head, min_conf, band, verify, list, count,
-                                                             stats, p0, p1);
+                                                             stats, chunk);
     else
       k_surrogate_refine<false, false><<<blocks, 128, 0, s>>>(*p, *o, head, min_conf, band, verify, list, count,
-                                                              stats, p0, p1);
+                                                              stats, chunk);
   } else {
     if (phi)
       k_surrogate_refine<true, true><<<blocks, 128, 0, s>>>(*p, *o, head, min_conf, band, verify, list, count,
-                                                            stats, p0, p1);
+                                                            stats, chunk);
     else
       k_surrogate_refine<true, false><<<blocks, 128, 0, s>>>(*p, *o, head, min_conf, band, verify, list, count,
-                                                             stats, p0, p1);
+                                                             stats, chunk);
   }
   return cudaGetLastError() == cudaSuccess ? 0 : -1;
 }

@@ -21,6 +21,7 @@
 #define BHA_INLINE_SOLUTION 1
 #endif
 
+#include "frame_source.cuh"
 #include "image_fp64.cuh"
 #include "kerr_analytic.cuh"
 #include "launch.h"
@@ -173,12 +174,12 @@ __device__ __forceinline__ bool trace_pixel(const BhkImageParams &p, const BhkIm
 }
 
 // Threads per CTA and resident CTAs per SM the closed form is compiled for:
-// one CTA per SM, whose warps the phases of trace_pixel keep together. 384
+// one CTA per SM, whose warps the phases of trace_pixel keep together: 384
 // threads at 168 registers (the solution structs in registers, a ~690-byte
-// frame) ran the 2048^2 a = 0.9, 60 deg frame in 4.06 ms with all outputs
-// and 1.61 ms with the disk fields, against 4.33 and 1.69 ms for 512
-// threads at 128 registers (1 KB frames that overflow L1); 320 threads
-// (168 registers, more spills) and 256 threads (246 registers) were slower.
+// frame). 2048^2 a = 0.9, 60 deg frame with all outputs / with the disk
+// fields, in row order: 2.07 / 0.99 ms; 512 threads at 128 registers 2.35 /
+// 1.15; two CTAs of 256 or 192 threads 2.34 / 1.09 and 2.15 / 0.95; without
+// the phases' barriers, 128-thread CTAs, 3.2 / 0.94.
 #ifndef BH_ANALYTIC_MIN_CTAS
 #define BH_ANALYTIC_MIN_CTAS 1
 #endif
@@ -193,8 +194,8 @@ __global__ void __launch_bounds__(BH_ANALYTIC_THREADS, BH_ANALYTIC_MIN_CTAS) k_t
   const long long stride = (long long)gridDim.x * blockDim.x;
   // every thread of the CTA takes the same trips through the phases' barriers
   for (long long base = (long long)blockIdx.x * blockDim.x; base < p.n_pix; base += stride) {
-    const long long pix = base + threadIdx.x;
-    const bool live = pix < p.n_pix;
+    const bool live = base + threadIdx.x < p.n_pix;
+    const long long pix = live ? bhsrc::tile_pixel(base + threadIdx.x, p.width, p.n_pix) : 0;
     if (!trace_pixel(p, o, pix, live) && live) list[atomicAdd(count, 1u)] = (int)pix;
   }
 }
