@@ -31,6 +31,13 @@ __device__ __forceinline__ unsigned long long globaltimer_ns() {
 // and in row order (before): 21.6, 3.27, 3.21 and 0.61 ms.
 constexpr int kHold = 64;
 
+// Steps between two looks at the warp's held lanes (times the launch's refill
+// interval). The votes cost a warp its lanes' reconvergence and some thirty
+// cycles of the step's latency each time: every step / every 8 or 32, one B200,
+// 64 x 48 RK4: mixed 2.07 / 1.31 ms, FP64 3.39 / 2.63; 64 x 48 DP45: mixed 0.24 /
+// 0.20, FP64 0.62 / 0.57; 48 uneven mixed frames 13.95 / 13.28.
+constexpr int kTurnsRk4 = 32, kTurnsDp45 = 8;
+
 // Lane states of the persistent tracers.
 enum : int { kEmpty = -1, kRun = -2, kCross = -3, kCrossStop = -4 };  // >= 0: ended with that class
 
@@ -56,12 +63,40 @@ __device__ __forceinline__ long long tile_pixel(long long w, int width, long lon
   return (long long)(r0 + y) * width + x;
 }
 
+// The same for a frame of one wave (every ray has a lane from the start), with
+// its tiles shuffled (a bijection of [0, 2^k) by two xor shifts and a product
+// with an odd number, repeated until it falls below the number of tiles): rays
+// that run long -- past the hole and out again, twice the others' RK4 steps --
+// are neighbours, and in order one SM got six such warps while most had none
+// (256^2 RK4: FP64 6.1 ms, shuffled 5.4; mixed 3.0 and 2.65).
+// Frames of several waves keep their order: there a warp takes new rays from
+// two tiles at a time, and neighbours stay together.
+__device__ __forceinline__ long long wave_pixel(long long w, const BhkImageParams &p) {
+  if (p.n_pix <= (long long)gridDim.x * blockDim.x) {
+    const unsigned T = (unsigned)(p.n_pix >> 5);
+    unsigned t = (unsigned)(w >> 5);
+    if (t < T && T > 1) {
+      const int k = 32 - __clz((int)(T - 1)), half = (k + 1) / 2;
+      const unsigned mask = (1u << k) - 1u;
+      do {
+        t ^= t >> half;
+        t = (t * 0x9E3779B1u) & mask;
+        t ^= t >> half;
+      } while (t >= T);
+      w = (long long)(t << 5 | (unsigned)(w & 31));
+    }
+  }
+  return tile_pixel(w, p.width, p.n_pix);
+}
+
+// WAVE: the order of wave_pixel (RK4, whose steps depend on where a ray ends).
+template <bool WAVE>
 struct SingleSrc {
   const BhkImageParams &p;
   const BhkImageOut &o;
   __device__ __forceinline__ long long total() const { return p.n_pix; }
   __device__ __forceinline__ int frame_of(long long w, long long &pix) const {
-    pix = tile_pixel(w, p.width, p.n_pix);
+    pix = WAVE ? wave_pixel(w, p) : tile_pixel(w, p.width, p.n_pix);
     return 0;
   }
   __device__ __forceinline__ const BhkImageParams &params(int) const { return p; }

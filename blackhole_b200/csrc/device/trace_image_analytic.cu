@@ -62,10 +62,12 @@ __device__ __forceinline__ double phi_radial(const BhkImageParams &p, const Ray 
 // The kernel's code is longer than the instruction cache holds, and warps at
 // different points of it kept evicting each other's instructions (47 % of
 // fetches hit); aligned by the barriers, the CTA's warps run each phase's
-// code at about the same time. Measured on the 2048^2 a = 0.9, 60 deg frame
-// with all outputs: 9.56 ms unaligned in 128-thread CTAs, 6.85 ms with one
-// barrier per pixel, 4.62 ms with that in 512-thread CTAs, 4.34 ms phased
-// in 512-thread CTAs (outputs bit-identical). Returns false when the closed
+// code at about the same time. The barriers' own cost is the wait for
+// a phase's slowest warp (the first stall, 4.2 of 9 cycles an issue), which
+// pixels taken in 8 x 4 tiles shorten. One B200, 2048^2 a = 0.9, 60 deg frame
+// with all outputs: 4.07 ms with CUDA's quotients and roots (a branch each),
+// 2.07 without them, 1.73 in tiles as well; 1279 x 721, three crossings: 1.88,
+// 0.94, 0.76 ms. Returns false when the closed
 // form does not cover the ray.
 __device__ __forceinline__ bool trace_pixel(const BhkImageParams &p, const BhkImageOut &o, long long pix,
                                             bool live) {

@@ -581,11 +581,12 @@ __device__ __forceinline__ void trace_loop(const Src &src, unsigned long long *_
   int st = bhsrc::kEmpty;
   bool exhausted = false;
   int waited = bhsrc::kHold;  // the first pass fills every lane
+  const int turns = refill * (INTEG == 0 ? bhsrc::kTurnsRk4 : bhsrc::kTurnsDp45);
   for (;;) {
     const unsigned running = __ballot_sync(kFull, st == bhsrc::kRun);
     const unsigned held = __ballot_sync(kFull, st != bhsrc::kRun && !(st == bhsrc::kEmpty && exhausted));
     if (held) {
-      waited += __popc(held) * refill;
+      waited += __popc(held) * turns;
       if (waited >= bhsrc::kHold || !running) {
         waited = 0;
         if (st == bhsrc::kCross || st == bhsrc::kCrossStop) {
@@ -625,7 +626,7 @@ __device__ __forceinline__ void trace_loop(const Src &src, unsigned long long *_
     } else if (!running) {
       break;
     }
-    for (int k = 0; k < refill; ++k)
+    for (int k = 0; k < turns; ++k)
       if (st == bhsrc::kRun)
         st = iterate<INTEG, tracks_closest<Src>::value, has_volume<Src>::value, DRIFT>(src.params(R.f), hs, R,
                                                                                     volume_of(src));
@@ -636,7 +637,7 @@ template <int INTEG, bool DRIFT>
 __global__ void __launch_bounds__(128, 4) k_trace_image_mixed(const __grid_constant__ BhkImageParams p,
                                                            const __grid_constant__ BhkImageOut o,
                                                            unsigned long long *__restrict__ counter, int refill) {
-  trace_loop<INTEG, DRIFT>(bhsrc::SingleSrc{p, o}, counter, refill);
+  trace_loop<INTEG, DRIFT>(bhsrc::SingleSrc<INTEG == 0>{p, o}, counter, refill);
 }
 
 template <int INTEG, bool DRIFT>
