@@ -12,26 +12,33 @@
 //
 // Here that is three launches instead of nineteen:
 //   k_post_rows : bright-pass fused into the four horizontal blurs. A tile of
-//                 32 rows x 128 columns (+ 32-column halos) in shared memory,
-//                 two rows side by side (pitch 193 pairs: 16 row pairs fall in
-//                 distinct banks); a thread has 8 outputs of a row pair. Each
-//                 output plane is staged in shared memory and stored by rows.
-//   k_post_cols : the four vertical blurs, summed in the reference's order
-//                 (r = 4, 8, 16, 32), and the composite; a thread has 8 rows
-//                 of two neighbouring columns; the planes of the next two
-//                 (channel, scale) jobs arrive by 16-byte cp.async meanwhile,
-//                 no more rows of them than the scale reaches.
-//   k_post_tone : the tone map into the caller's framebuffer.
+//                 16 rows x 64 columns (+ 32-column halos) in shared memory,
+//                 two rows side by side (pitch 129 pairs: a half-warp's 8 row
+//                 pairs x 2 runs fall in distinct banks); two warps a channel,
+//                 a thread has 8 outputs of a row pair and stores them from
+//                 its registers, a warp 128 bytes of a row. The framebuffer's
+//                 own channels leave as planes too.
+//   k_post_cols : the four vertical blurs of one channel, summed in the
+//                 reference's order (r = 4, 8, 16, 32), added to that
+//                 channel's plane; a thread has 8 rows of two neighbouring
+//                 columns; the next scale's plane arrives by 16-byte cp.async
+//                 meanwhile, no more rows of it than the scale reaches.
+//   k_post_tone : the tone map of the three planes into the caller's
+//                 framebuffer.
 // Both blurs multiply and add two values per instruction (fma.rn.f32x2, each
 // half rounded as the scalar one): issue slots, not the FP32 lanes, bound the
 // scalar version (79 and 68 % issue at 42 and 34 % of the FMA pipe). 1920 x
-// 1080, strength 0.5, per launch: rows 76 -> 61, columns 101 -> 54, tone (with
-// a 64-bit division per pixel) 30 -> 28 us (three powf, 84 % issue).
+// 1080, strength 0.5, per launch from a cold L2: rows 76 -> 61 us in pairs,
+// -> 52 in these tiles (1.15 waves of 32 x 128 tiles, all channels in turn,
+// became 2.8 waves of a third of the work); columns 101 -> 54 in pairs, -> 47
+// with a channel a CTA (2 CTAs of 256 threads at 126 registers became 7 of
+// 128); tone, without a 64-bit division per pixel, 30 -> 29 (three powf, 84 %
+// issue). The multiplications alone fill the FP32 pipe for 24 us a blur.
 // The horizontal results travel through 12 float planes (4 scales x RGB,
-// structure of arrays, rows padded to 64 columns); the composite goes to a
-// separate buffer because the tone map reads a neighbour's colour (below),
-// which an in-place pass would race on. Bytes per pixel: rows 16 in + 48 out,
-// cols 48 + 16 in + 16 out, tone 16 in + 16 out.
+// structure of arrays, rows padded to 64 columns), the composite through three
+// more: the tone map reads a neighbour's colour (below), which an in-place
+// pass would race on. Bytes per pixel: rows 16 in + 60 out, columns 60 in +
+// 12 out, tone 12 in + 16 out.
 //
 // The tone map's red and blue come from pixel (rx, ry) = (int(u w), int(v h))
 // with u = px / w, v = py / h rounded to float (cuda_postprocess.cu:165-176,
@@ -51,28 +58,26 @@ namespace {
 constexpr int kHalo = 32;  // the largest blur half-width
 constexpr int kRun = 8;    // outputs per thread along the blur direction
 
-// Rows pass tile.
-constexpr int kRowsY = 32;
-constexpr int kRowsX = 128;
+// Rows pass tile: two warps (of 64 columns) a channel.
+constexpr int kRowsY = 16;
+constexpr int kRowsX = 64;
 constexpr int kRowsW = kRowsX + 2 * kHalo;
 constexpr int kRowsPitch = kRowsW + 1;          // in row pairs
 constexpr int kRowPairs = kRowsY / 2;
-constexpr int kRowsThreads = kRowPairs * (kRowsX / kRun);  // 256
-constexpr int kOutPitch = kRowsX + 4;
-constexpr size_t kRowsSmem = sizeof(float2) * 3 * kRowPairs * kRowsPitch + sizeof(float) * kRowsY * kOutPitch;
+constexpr int kRowsLanes = kRowPairs * (kRowsX / kRun);  // threads of a channel
+constexpr int kRowsThreads = 3 * kRowsLanes;
 
 // Columns pass tile.
-constexpr int kColsX = 64;
+constexpr int kColsX = 32;
 constexpr int kColsY = 64;
 constexpr int kColsH = kColsY + 2 * kHalo;
-constexpr int kColsThreads = kColsX / 2 * (kColsY / kRun);  // 256
-constexpr int kColsRing = 3;
+constexpr int kColsThreads = kColsX / 2 * (kColsY / kRun);
 constexpr int kColsBuf = kColsH * kColsX;
-constexpr size_t kColsSmem = sizeof(float) * kColsRing * kColsBuf;
 
 // Floats between rows of a plane: whole tiles of columns, so that every row
 // starts on 256 bytes and the last tile reads within the plane.
-__host__ __device__ constexpr int plane_pitch(int w) { return (w + kColsX - 1) / kColsX * kColsX; }
+__host__ __device__ constexpr int plane_pitch(int w) { return (w + 63) / 64 * 64; }
+constexpr int kBase = 12;  // planes kBase + c: the framebuffer's channels, then the composite's
 
 // Scale index and offset of the normalized taps (2r + 1 each) of half-width R.
 __host__ __device__ constexpr int scale_of(int R) { return R == 4 ? 0 : R == 8 ? 1 : R == 16 ? 2 : 3; }
@@ -115,61 +120,68 @@ __device__ __forceinline__ void blur_run(const float2 *src, int stride, const fl
   }
 }
 
-__global__ void __launch_bounds__(kRowsThreads, 2) k_post_rows(const __grid_constant__ Taps2 taps,
-                                                             const float4 *__restrict__ fb, int w, int h,
-                                                             float threshold, float *__restrict__ planes) {
-  extern __shared__ float2 sm[];  // [3][kRowPairs][kRowsPitch] bright-pass, then [kRowsY][kOutPitch] one output plane
-  float *stage = reinterpret_cast<float *>(sm + 3 * kRowPairs * kRowsPitch);
+__global__ void __launch_bounds__(kRowsThreads, 5) k_post_rows(const __grid_constant__ Taps2 taps,
+                                                               const float4 *__restrict__ fb, int w, int h,
+                                                               float threshold, float *__restrict__ planes) {
+  __shared__ float2 sm[3 * kRowPairs * kRowsPitch];  // bright-pass
   const int x0 = blockIdx.x * kRowsX, y0 = blockIdx.y * kRowsY;
-  static_assert(kRowPairs * kRowsW % (4 * kRowsThreads) == 0, "whole load rounds");
+  const int pitch = plane_pitch(w);
+  const int64_t plane = (int64_t)h * pitch;
+  constexpr int kPairs = kRowPairs * kRowsW, kInFlight = 3;  // 6 pixels a thread
 #pragma unroll 1
-  for (int k0 = 0; k0 < kRowPairs * kRowsW; k0 += 4 * kRowsThreads) {  // 8 pixels in flight a thread
-    float4 v[4][2];
+  for (int k0 = 0; k0 < kPairs; k0 += kInFlight * kRowsThreads) {
+    float4 v[kInFlight][2];
 #pragma unroll
-    for (int k = 0; k < 4; ++k) {
+    for (int k = 0; k < kInFlight; ++k) {
       const int e = k0 + k * kRowsThreads + threadIdx.x, rp = e / kRowsW, col = e - rp * kRowsW;
       const int x = min(max(x0 - kHalo + col, 0), w - 1);
 #pragma unroll
       for (int i = 0; i < 2; ++i) {
         const int y = y0 + 2 * rp + i;
-        v[k][i] = y < h ? fb[(int64_t)y * w + x] : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        v[k][i] = e < kPairs && y < h ? fb[(int64_t)y * w + x] : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
       }
     }
 #pragma unroll
-    for (int k = 0; k < 4; ++k) {
+    for (int k = 0; k < kInFlight; ++k) {
       const int e = k0 + k * kRowsThreads + threadIdx.x, rp = e / kRowsW, col = e - rp * kRowsW;
+      if (e >= kPairs) continue;
       const float s0 = bright_scale(v[k][0], threshold), s1 = bright_scale(v[k][1], threshold);
       sm[(0 * kRowPairs + rp) * kRowsPitch + col] = make_float2(v[k][0].x * s0, v[k][1].x * s1);
       sm[(1 * kRowPairs + rp) * kRowsPitch + col] = make_float2(v[k][0].y * s0, v[k][1].y * s1);
       sm[(2 * kRowPairs + rp) * kRowsPitch + col] = make_float2(v[k][0].z * s0, v[k][1].z * s1);
+      const int x = x0 - kHalo + col;
+      if (col >= kHalo && col < kHalo + kRowsX && x < w) {
+#pragma unroll
+        for (int i = 0; i < 2; ++i) {
+          const int y = y0 + 2 * rp + i;
+          float *base = planes + kBase * plane + (int64_t)y * pitch + x;
+          if (y < h) base[0] = v[k][i].x, base[plane] = v[k][i].y, base[2 * plane] = v[k][i].z;
+        }
+      }
     }
   }
-  const int rp = threadIdx.x % kRowPairs, run = threadIdx.x / kRowPairs;
-  const int pitch = plane_pitch(w);
-  // Results leave through the stage, so that a warp stores 32 consecutive
-  // float4 of one row (the compute layout has a lane per row pair).
+  const int c = threadIdx.x / kRowsLanes, lane = threadIdx.x % kRowsLanes;
+  const int rp = lane % kRowPairs, run = lane / kRowPairs;
+  __syncthreads();
+  // A warp has 8 row pairs x 4 neighbouring runs: its stores fill whole 32-byte
+  // sectors, 128 bytes of a row at a time.
+  const int y = y0 + 2 * rp, x = x0 + run * kRun;
+  const float2 *src = sm + (c * kRowPairs + rp) * kRowsPitch + kHalo + run * kRun;
+  float *dst = planes + c * plane + (int64_t)y * pitch + x;
+  const bool top = x < pitch && y < h, low = x < pitch && y + 1 < h;
   auto scale = [&](auto rtag) {
     constexpr int R = decltype(rtag)::value, si = scale_of(R);
-#pragma unroll 1
-    for (int c = 0; c < 3; ++c) {
-      __syncthreads();  // bright-pass written / the previous plane copied out
-      float2 acc[kRun] = {};
-      blur_run<R>(sm + (c * kRowPairs + rp) * kRowsPitch + kHalo + run * kRun - R, 1, taps.w + tap_off(R), acc);
-      float4 *s0 = reinterpret_cast<float4 *>(stage + 2 * rp * kOutPitch + run * kRun);
-      float4 *s1 = reinterpret_cast<float4 *>(stage + (2 * rp + 1) * kOutPitch + run * kRun);
-      s0[0] = make_float4(acc[0].x, acc[1].x, acc[2].x, acc[3].x);
-      s0[1] = make_float4(acc[4].x, acc[5].x, acc[6].x, acc[7].x);
-      s1[0] = make_float4(acc[0].y, acc[1].y, acc[2].y, acc[3].y);
-      s1[1] = make_float4(acc[4].y, acc[5].y, acc[6].y, acc[7].y);
-      __syncthreads();
-      float *out = planes + (int64_t)(si * 3 + c) * h * pitch;
-#pragma unroll
-      for (int e = threadIdx.x; e < kRowsY * kRowsX / 4; e += kRowsThreads) {
-        const int row = e / (kRowsX / 4), col = 4 * (e % (kRowsX / 4));
-        if (y0 + row < h && x0 + col < pitch)
-          *reinterpret_cast<float4 *>(out + (int64_t)(y0 + row) * pitch + x0 + col) =
-              *reinterpret_cast<const float4 *>(stage + row * kOutPitch + col);
-      }
+    float2 acc[kRun] = {};
+    asm volatile("" ::: "memory");  // one scale's window at a time in registers
+    blur_run<R>(src - R, 1, taps.w + tap_off(R), acc);
+    float4 *out = reinterpret_cast<float4 *>(dst + 3 * si * plane);
+    if (top) {
+      out[0] = make_float4(acc[0].x, acc[1].x, acc[2].x, acc[3].x);
+      out[1] = make_float4(acc[4].x, acc[5].x, acc[6].x, acc[7].x);
+    }
+    if (low) {
+      out[pitch / 4] = make_float4(acc[0].y, acc[1].y, acc[2].y, acc[3].y);
+      out[pitch / 4 + 1] = make_float4(acc[4].y, acc[5].y, acc[6].y, acc[7].y);
     }
   };
   scale(std::integral_constant<int, 4>{});
@@ -178,14 +190,15 @@ __global__ void __launch_bounds__(kRowsThreads, 2) k_post_rows(const __grid_cons
   scale(std::integral_constant<int, 32>{});
 }
 
-// Rows y0 - R .. y0 + 63 + R (clamped) of one channel's plane of scale si,
-// columns x0 .. x0 + 63, into a shared buffer, by cp.async.
+// Rows y0 - R .. y0 + kColsY - 1 + R (clamped) of one channel's plane of scale
+// si, kColsX columns from x0, into a shared buffer, by cp.async.
 __device__ __forceinline__ void cols_fetch(float *buf, const float *__restrict__ planes, int c, int si, int x0,
                                            int y0, int pitch, int h) {
   const int R = 4 << si;
-  const float *src = planes + (int64_t)(si * 3 + c) * h * pitch + x0 + 4 * (threadIdx.x % 16);
-  float *dst = buf + 4 * (threadIdx.x % 16);
-  for (int row = threadIdx.x / 16; row < kColsY + 2 * R; row += kColsThreads / 16) {
+  constexpr int kVecs = kColsX / 4;
+  const float *src = planes + (int64_t)(si * 3 + c) * h * pitch + x0 + 4 * (threadIdx.x % kVecs);
+  float *dst = buf + 4 * (threadIdx.x % kVecs);
+  for (int row = threadIdx.x / kVecs; row < kColsY + 2 * R; row += kColsThreads / kVecs) {
     const int y = min(max(y0 - R + row, 0), h - 1);
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(
                      (unsigned)__cvta_generic_to_shared(dst + row * kColsX)),
@@ -194,61 +207,44 @@ __device__ __forceinline__ void cols_fetch(float *buf, const float *__restrict__
   }
 }
 
-__global__ void __launch_bounds__(kColsThreads, 2) k_post_cols(const __grid_constant__ Taps2 taps,
-                                                             const float *__restrict__ planes,
-                                                             const float4 *__restrict__ fb, int w, int h,
-                                                             float strength, float4 *__restrict__ out) {
-  extern __shared__ float cols_sm[];  // kColsRing buffers of [kColsH][kColsX]: job 4 c + si in buffer job % kColsRing
-  const int x0 = blockIdx.x * kColsX, y0 = blockIdx.y * kColsY;
-  const int lane = threadIdx.x & 31, grp = threadIdx.x >> 5;
+__global__ void __launch_bounds__(kColsThreads, 7) k_post_cols(const __grid_constant__ Taps2 taps,
+                                                               float *__restrict__ planes, int w, int h,
+                                                               float strength) {
+  extern __shared__ float cols_sm[];  // two buffers of [kColsH][kColsX]: scale si in buffer si % 2
+  const int x0 = blockIdx.x * kColsX, y0 = blockIdx.y * kColsY, c = blockIdx.z;
+  const int lane = threadIdx.x % (kColsX / 2), grp = threadIdx.x / (kColsX / 2);
   const int pitch = plane_pitch(w);
-  float2 tr[kRun], tg[kRun], tb[kRun];
-  auto fetch = [&](int job) {
-    if (job < 12) cols_fetch(cols_sm + (job % kColsRing) * kColsBuf, planes, job >> 2, job & 3, x0, y0, pitch, h);
+  auto fetch = [&](int si) {
+    if (si < 4) cols_fetch(cols_sm + (si % 2) * kColsBuf, planes, c, si, x0, y0, pitch, h);
     asm volatile("cp.async.commit_group;\n" ::: "memory");
   };
   fetch(0);
   fetch(1);
-#pragma unroll 1
-  for (int c = 0; c < 3; ++c) {
-    float2 tot[kRun] = {};
-    auto scale = [&](auto rtag) {
-      constexpr int R = decltype(rtag)::value, si = scale_of(R);
-      const int job = 4 * c + si;
-      asm volatile("cp.async.wait_group 1;\n" ::: "memory");  // this job landed, the next may be in flight
-      __syncthreads();                                         // ... for every warp, and buffer (job + 2) % 3 is free
-      fetch(job + 2);
-      const float2 *buf = reinterpret_cast<const float2 *>(cols_sm + (job % kColsRing) * kColsBuf);
-      float2 acc[kRun] = {};
-      blur_run<R>(buf + grp * kRun * (kColsX / 2) + lane, kColsX / 2, taps.w + tap_off(R), acc);
+  float2 tot[kRun] = {};
+  auto scale = [&](auto rtag) {
+    constexpr int R = decltype(rtag)::value, si = scale_of(R);
+    asm volatile("cp.async.wait_group 1;\n" ::: "memory");  // this scale landed, the next may be in flight
+    __syncthreads();
+    const float2 *buf = reinterpret_cast<const float2 *>(cols_sm + (si % 2) * kColsBuf);
+    float2 acc[kRun] = {};
+    blur_run<R>(buf + grp * kRun * (kColsX / 2) + lane, kColsX / 2, taps.w + tap_off(R), acc);
 #pragma unroll
-      for (int j = 0; j < kRun; ++j) tot[j].x += acc[j].x, tot[j].y += acc[j].y;
-    };
-    scale(std::integral_constant<int, 4>{});
-    scale(std::integral_constant<int, 8>{});
-    scale(std::integral_constant<int, 16>{});
-    scale(std::integral_constant<int, 32>{});
-#pragma unroll
-    for (int j = 0; j < kRun; ++j) {
-      if (c == 0) tr[j] = tot[j];
-      if (c == 1) tg[j] = tot[j];
-      if (c == 2) tb[j] = tot[j];
-    }
-  }
-  const int x = x0 + 2 * lane;
+    for (int j = 0; j < kRun; ++j) tot[j].x += acc[j].x, tot[j].y += acc[j].y;
+    if (si < 2) __syncthreads();  // every warp is done with the buffer
+    fetch(si + 2);
+  };
+  scale(std::integral_constant<int, 4>{});
+  scale(std::integral_constant<int, 8>{});
+  scale(std::integral_constant<int, 16>{});
+  scale(std::integral_constant<int, 32>{});
+  float *base = planes + (int64_t)(kBase + c) * h * pitch + x0 + 2 * lane;
 #pragma unroll
   for (int j = 0; j < kRun; ++j) {
     const int y = y0 + grp * kRun + j;
     if (y >= h) break;
-    const int64_t i = (int64_t)y * w + x;
-    if (x < w) {
-      const float4 b = fb[i];
-      out[i] = make_float4(b.x + tr[j].x * strength, b.y + tg[j].x * strength, b.z + tb[j].x * strength, 1.0f);
-    }
-    if (x + 1 < w) {
-      const float4 b = fb[i + 1];
-      out[i + 1] = make_float4(b.x + tr[j].y * strength, b.y + tg[j].y * strength, b.z + tb[j].y * strength, 1.0f);
-    }
+    float2 *p = reinterpret_cast<float2 *>(base + (int64_t)y * pitch);
+    const float2 b = *p;
+    *p = make_float2(b.x + tot[j].x * strength, b.y + tot[j].y * strength);
   }
 }
 
@@ -264,9 +260,17 @@ __device__ __forceinline__ float tone_channel(float x, float exposure, float vig
 }
 
 // A thread has one column of 4 rows, so that u and the column index are worked out once.
+// PLANAR: the composite is in three planes, otherwise a copy of the framebuffer.
 constexpr int kToneRows = 4;
-__global__ void __launch_bounds__(256) k_post_tone(const float4 *__restrict__ src, int w, int h, float exposure,
+template <bool PLANAR>
+__global__ void __launch_bounds__(256) k_post_tone(const float *__restrict__ src, int w, int h, float exposure,
                                                    float4 *__restrict__ fb) {
+  const int pitch = PLANAR ? plane_pitch(w) : w;
+  const int64_t plane = (int64_t)h * pitch;
+  auto at = [&](int y, int x, int c) {
+    const int64_t i = (int64_t)y * pitch + x;
+    return PLANAR ? src[c * plane + i] : src[4 * i + c];
+  };
   const int px = blockIdx.x * 64 + (threadIdx.x & 63);
   const int y0 = (blockIdx.y * 4 + (threadIdx.x >> 6)) * kToneRows;
   if (px >= w) return;
@@ -280,47 +284,40 @@ __global__ void __launch_bounds__(256) k_post_tone(const float4 *__restrict__ sr
     const int64_t i = (int64_t)py * w + px;
     const float v = __fdiv_rn((float)py, (float)h);
     const int ry = min(max((int)__fmul_rn(v, (float)h), 0), h - 1);
-    const float4 rb = src[(int64_t)ry * w + rx];
-    const float gch = src[i].y;
+    const float red = at(ry, rx, 0), gch = at(py, px, 1), blue = at(ry, rx, 2);
     const float dv = v - 0.5f;
     const float dist = sqrtf(du * du + dv * dv);
     const float vig = sqrtf(fmaxf(1.0f - dist * dist * 0.5f, 0.0f));
-    fb[i] = make_float4(tone_channel(rb.x, exposure, vig), tone_channel(gch, exposure, vig),
-                        tone_channel(rb.z, exposure, vig), 1.0f);
+    fb[i] = make_float4(tone_channel(red, exposure, vig), tone_channel(gch, exposure, vig),
+                        tone_channel(blue, exposure, vig), 1.0f);
   }
 }
 
 }  // namespace
 
-// 12 padded planes, then the composite (float4 per pixel; 256-byte aligned rows before it keep it aligned).
-extern "C" int64_t bhk_post_scratch_floats(int w, int h) {
-  return (int64_t)12 * plane_pitch(w) * h + (int64_t)4 * w * h;
-}
+// 15 padded planes, or a copy of the framebuffer where the bloom is off.
+extern "C" int64_t bhk_post_scratch_floats(int w, int h) { return (int64_t)(kBase + 3) * plane_pitch(w) * h; }
 
 extern "C" int bhk_post_process(float *fb, int w, int h, const BhkPostTaps *taps, float threshold, float strength,
                                 float exposure, float *scratch, void *stream) {
   if (w <= 0 || h <= 0) return 0;
   const cudaStream_t st = static_cast<cudaStream_t>(stream);
-  const int64_t n = (int64_t)w * h;
-  float *planes = scratch;
-  float4 *comp = reinterpret_cast<float4 *>(scratch + (int64_t)12 * plane_pitch(w) * h);
   float4 *f4 = reinterpret_cast<float4 *>(fb);
+  const dim3 gt((w + 63) / 64, (h + 4 * kToneRows - 1) / (4 * kToneRows));
   if (strength != 0.0f) {
-    if (cudaFuncSetAttribute(k_post_rows, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kRowsSmem) !=
-            cudaSuccess ||
-        cudaFuncSetAttribute(k_post_cols, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kColsSmem) !=
-            cudaSuccess)
+    constexpr int smem = sizeof(float) * 2 * kColsBuf;
+    if (cudaFuncSetAttribute(k_post_cols, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess)
       return -1;
     Taps2 t2;
     for (int i = 0; i < 124; ++i) t2.w[i] = make_float2(taps->w[i], taps->w[i]);
     const dim3 gr((w + kRowsX - 1) / kRowsX, (h + kRowsY - 1) / kRowsY);
-    k_post_rows<<<gr, kRowsThreads, kRowsSmem, st>>>(t2, f4, w, h, threshold, planes);
-    const dim3 gc((w + kColsX - 1) / kColsX, (h + kColsY - 1) / kColsY);
-    k_post_cols<<<gc, kColsThreads, kColsSmem, st>>>(t2, planes, f4, w, h, strength, comp);
-  } else if (cudaMemcpyAsync(comp, fb, sizeof(float4) * n, cudaMemcpyDeviceToDevice, st) != cudaSuccess) {
-    return -1;
+    k_post_rows<<<gr, kRowsThreads, 0, st>>>(t2, f4, w, h, threshold, scratch);
+    const dim3 gc((w + kColsX - 1) / kColsX, (h + kColsY - 1) / kColsY, 3);
+    k_post_cols<<<gc, kColsThreads, smem, st>>>(t2, scratch, w, h, strength);
+    k_post_tone<true><<<gt, 256, 0, st>>>(scratch + (int64_t)kBase * plane_pitch(w) * h, w, h, exposure, f4);
+  } else {
+    if (cudaMemcpyAsync(scratch, fb, sizeof(float4) * w * h, cudaMemcpyDeviceToDevice, st) != cudaSuccess) return -1;
+    k_post_tone<false><<<gt, 256, 0, st>>>(scratch, w, h, exposure, f4);
   }
-  const dim3 gt((w + 63) / 64, (h + 4 * kToneRows - 1) / (4 * kToneRows));
-  k_post_tone<<<gt, 256, 0, st>>>(comp, w, h, exposure, f4);
   return cudaGetLastError() == cudaSuccess ? 0 : -1;
 }
