@@ -27,10 +27,8 @@
 
 namespace bhk {
 
-// x < 0 (false for -0), on the integer pipe.
-__device__ __forceinline__ bool is_neg(double x) {
-  return (unsigned long long)__double_as_longlong(x) > 0x8000000000000000ull;
-}
+// The sign bit: x < 0 for every x but -0 (and NaN), on the integer pipe.
+__device__ __forceinline__ bool is_neg(double x) { return __double2hiint(x) < 0; }
 
 // 1 / b to 0.51 ulp, and a / b from it.
 __device__ __forceinline__ double rcp_near(double b) {
@@ -48,29 +46,27 @@ __device__ __forceinline__ double div_by(double a, double b, double y) {
 // a / b.
 __device__ __forceinline__ double div_rn(double a, double b) { return div_by(a, b, rcp_near(b)); }
 
-// a / 5 and a / 6: y is the rounded reciprocal itself.
-__device__ __forceinline__ double div_5(double a) {
-  constexpr double y = 1.0 / 5.0;
-  const double q = a * y;
-  return fma(fma(-5.0, q, a), y, q);
-}
-__device__ __forceinline__ double div_6(double a) {
-  constexpr double y = 1.0 / 6.0;
-  const double q = a * y;
-  return fma(fma(-6.0, q, a), y, q);
-}
+// a / 5 and a / 6, the reciprocal in two parts: a quotient by 5 or 3 lies a
+// tenth of an ulp or more from any midpoint of two doubles (a multiple of the
+// half ulp that is not 5 or 3 times a midpoint is one half ulp off at least),
+// and the sum before its one rounding is within 2^-50 ulp of it.
+__device__ __forceinline__ double div_5(double a) { return fma(a, 1.0 / 5.0, a * -0x1.999999999999ap-57); }
+__device__ __forceinline__ double div_6(double a) { return fma(a, 1.0 / 6.0, a * 0x1.5555555555555p-57); }
 
-// sqrt(x) for x > 1e-290; a smaller x (0 and NaN among them) is returned as
-// it is: the callers compare the root with bounds that all such values, and
-// their roots, lie on the same side of.
+// sqrt(x) for x > 1e-290; a smaller x (0 among them) is returned as it is: the
+// callers compare the root with bounds that all such values, and their roots,
+// lie on the same side of. The compare is of the high words. Root and half
+// reciprocal are refined side by side (R. E. Goldschmidt's scheme), a chain of
+// seven dependent operations.
 __device__ __forceinline__ double sqrt_rn(double x) {
   double y;
   asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
-  const double e = fma(-(x * y), y, 1.0);
-  y = fma(y, fma(0.375, e, 0.5) * e, y);
-  const double g = x * y;
-  const double s = fma(fma(-g, g, x), 0.5 * y, g);
-  return x > 1e-290 ? s : x;
+  const double g0 = x * y, h0 = 0.5 * y;
+  const double e = fma(-g0, y, 1.0);
+  const double t = fma(0.375, e, 0.5) * e;
+  const double g = fma(g0, t, g0);
+  const double s = fma(fma(-g, g, x), fma(h0, t, h0), g);
+  return __double2hiint(x) > 0x03cfffff ? s : x;
 }
 
 }  // namespace bhk

@@ -38,7 +38,9 @@ __device__ __forceinline__ Yd rhs(const Yd &y, const RayC &c) {
   const double A = (rr + c.a2) - (c.a * c.lam);
   const double D = fma(-2.0, r, rr) + c.a2;
   const double u2 = u * u;
-  const double s2 = dmax_(1.0 - u2, 1e-12);
+  // max(1 - u^2, 1e-12) by the high words: near 1e-12 the values of 1 - u^2 are
+  // multiples of 2^-53 and none of them shares a high word with 1e-12
+  const double c2 = 1.0 - u2, s2 = __double2hiint(c2) > 0x3d719799 ? c2 : 1e-12;
   Yd d;
   d.r = y.pr;
   d.u = y.pu;
@@ -96,21 +98,25 @@ constexpr double kProjTau = 1e-6;
 // removed, |eta(state) - eta| / (|q_Th| + a^2) with eta(state) - eta =
 // (p_u^2 - U(u)) / (1 - u^2), where the polar momentum was projected (0 near
 // a polar turning point); otherwise 0, and the division is skipped.
+//
+// Without branches, here and in step_factor: a step's chain of dependent
+// operations (8 cycles each) is what a small frame waits for, and a branch
+// keeps the two roots, and the step control, from running beside each other.
+// One B200, one warp an SM quarter: an RK4 step 519 -> 391 ns, a DP45 step
+// 1590 -> 1500 ns. 256^2 RK4 5.47 -> 4.64 ms, 64 x 48 DP45 0.58 -> 0.53, 640 x
+// 360 DP45 2.83 -> 2.66 ms.
 __device__ __forceinline__ double project(Yd &y, const RayC &c, bool want_drift = false) {
   const double Rv = pot_R(y.r, c);
   const double r2 = y.r * y.r;
-  if (Rv > kProjTau * (r2 * r2)) {
-    const double m = sqrt_rn(Rv);
-    y.pr = is_neg(y.pr) ? -m : m;
-  }
+  const double mr = copysign(sqrt_rn(Rv), y.pr);
+  y.pr = Rv > kProjTau * (r2 * r2) ? mr : y.pr;
   const double Uv = pot_U(y.u, c);
   const double scale = fabs(c.qTh) + (c.a * c.a);
+  const bool on = Uv > kProjTau * scale;
   double drift = 0.0;
-  if (Uv > kProjTau * scale) {
-    if (want_drift) drift = fabs((y.pu * y.pu) - Uv) / ((1.0 - (y.u * y.u)) * scale);
-    const double m = sqrt_rn(Uv);
-    y.pu = is_neg(y.pu) ? -m : m;
-  }
+  if (want_drift && on) drift = fabs((y.pu * y.pu) - Uv) / ((1.0 - (y.u * y.u)) * scale);
+  const double mu = copysign(sqrt_rn(Uv), y.pu);
+  y.pu = on ? mu : y.pu;
   return drift;
 }
 
@@ -241,10 +247,11 @@ __device__ __forceinline__ double inv_fifth_root(double x) {
 // [0.1, 2] after acceptance, [0.1, 1] after rejection).
 __device__ __forceinline__ double step_factor(double err, bool accepted) {
   const double hi = accepted ? 2.0 : 1.0;
-  if (!(err < 1e300)) return 0.1;
-  if (!(err > 0.0)) return hi;
   const double f = 0.9 * inv_fifth_root(err);
-  return (f < 0.1) ? 0.1 : ((hi < f) ? hi : f);
+  const double g = (f < 0.1) ? 0.1 : ((hi < f) ? hi : f);
+  // by its high word (err has no sign): 0 takes the upper bound, 1e300, infinity and NaN the lower
+  const unsigned w = (unsigned)__double2hiint(err);
+  return w >= 0x7e37e43cu ? 0.1 : (w == 0u ? hi : g);
 }
 
 // Keplerian prograde emitter (Bardeen, Press & Teukolsky 1972):

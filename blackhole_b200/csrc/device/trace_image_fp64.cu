@@ -29,8 +29,8 @@ constexpr unsigned kFull = 0xffffffffu;
 struct RayFp64 {
   RayC c;
   Yd y;
-  Yd k1;        // DP45: FSAL stage of y
-  double h;     // DP45: next trial step
+  Yd k1;        // rhs(y); DP45: its FSAL stage
+  double h;     // next step; DP45: next trial step
   double inten;
   long long pix;
   int f;  // frame of the current ray (batch launches)
@@ -39,6 +39,13 @@ struct RayFp64 {
   int ncross;
   double drift;  // largest Carter-constant residual the projection removed
 };
+
+// RK4's step at y, DP45's first trial step.
+__device__ __forceinline__ double mino_step(const BhkImageParams &p, const Yd &y) {
+  const double hh = p.step_coeff * dmin_(y.r, p.step_rcap);
+  const double sigma = (y.r * y.r) + ((p.a2 * y.u) * y.u);
+  return div_rn(hh, sigma);
+}
 
 __device__ __forceinline__ void init_ray(const BhkImageParams &p, long long pix, RayFp64 &R) {
   const long long i = pix % p.width, j = pix / p.width;
@@ -55,8 +62,8 @@ __device__ __forceinline__ void init_ray(const BhkImageParams &p, long long pix,
   R.y.u = p.cos_o;
   R.y.phi = 0.0;
   const double Rv = pot_R(R.y.r, R.c);
-  R.y.pr = -sqrt((Rv < 0.0) ? 0.0 : Rv);
-  R.y.pu = beta * p.sin_o;
+  R.y.pr = 0.0 - sqrt((Rv < 0.0) ? 0.0 : Rv);  // no -0, which is_neg takes for negative
+  R.y.pu = beta * p.sin_o + 0.0;
   R.steps = 0;
   R.attempts = 0;
   R.ncross = 0;
@@ -64,12 +71,8 @@ __device__ __forceinline__ void init_ray(const BhkImageParams &p, long long pix,
   R.pix = pix;
   project(R.y, R.c);  // idempotent from here on (see iterate)
   R.drift = 0.0;
-  if (p.integrator == 1) {
-    const double hh = p.step_coeff * dmin_(R.y.r, p.step_rcap);
-    const double sigma = (R.y.r * R.y.r) + ((p.a2 * R.y.u) * R.y.u);
-    R.h = hh / sigma;
-    R.k1 = rhs(R.y, R.c);
-  }
+  R.h = mino_step(p, R.y);
+  R.k1 = rhs(R.y, R.c);
 }
 
 // The step in which a lane's ray crosses u = 0, y0 -> y1 (y1 before the
@@ -158,19 +161,17 @@ __device__ __forceinline__ int iterate(const BhkImageParams &p, HeldSteps &hs, R
     if (R.steps >= p.max_steps) return 3;
     if (R.y.r <= p.r_hor) return 0;
     if (R.y.r >= p.r_esc) return 2;
-    const double hh = p.step_coeff * dmin_(R.y.r, p.step_rcap);
-    const double sigma = (R.y.r * R.y.r) + ((p.a2 * R.y.u) * R.y.u);
-    const double h = div_rn(hh, sigma);
-    const Yd k0 = rhs(R.y, R.c);
-    Yd yn = rk4(R.y, h, R.c, k0);
+    Yd yn = rk4(R.y, R.h, R.c, R.k1);
     ++R.steps;
     const bool cross = (R.y.u * yn.u) < 0.0;
-    if (cross) hold_step(hs, R.y, k0, yn, rhs(yn, R.c), h);
+    if (cross) hold_step(hs, R.y, R.k1, yn, rhs(yn, R.c), R.h);
     if (DRIFT)
       R.drift = dmax_(R.drift, project(yn, R.c, true));
     else
       project(yn, R.c);
     R.y = yn;
+    R.h = mino_step(p, yn);  // beside the projection's roots, which the step and the accelerations do not need
+    R.k1 = rhs(yn, R.c);
     return cross ? bhsrc::kCross : bhsrc::kRun;
   } else {
     const long long max_attempts = 4LL * p.max_steps + 64;
