@@ -69,4 +69,17 @@ __device__ __forceinline__ double sqrt_rn(double x) {
   return __double2hiint(x) > 0x03cfffff ? s : x;
 }
 
+// The FP32 root, the same way; 0 is its own root, arguments below 1e-30 are
+// scaled by an even power of two. All 2^31 floats checked against sqrtf.
+__device__ __forceinline__ float sqrt_rn_f(float x) {
+  const bool tiny = x < 1e-30f;
+  const float v = tiny ? x * 0x1p100f : x;
+  float y;
+  asm("rsqrt.approx.f32 %0, %1;" : "=f"(y) : "f"(v));
+  const float g = v * y;
+  float s = fmaf(fmaf(-g, g, v), 0.5f * y, g);
+  s = tiny ? s * 0x1p-50f : s;
+  return x == 0.0f || x == INFINITY ? x : s;
+}
+
 }  // namespace bhk

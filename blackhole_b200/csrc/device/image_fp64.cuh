@@ -257,21 +257,22 @@ __device__ __forceinline__ double step_factor(double err, bool accepted) {
 // Keplerian prograde emitter (Bardeen, Press & Teukolsky 1972):
 // g = sqrt(x^3 (x^3 - 3x + 2a)) / (x^3 + a - lambda), x = sqrt(r).
 __device__ __forceinline__ double disk_g(double r, double a, double lam) {
-  const double x = sqrt(r);
+  const double x = sqrt_rn(r);
   const double x3 = (x * x) * x;
   const double v = x3 * ((x3 - (3.0 * x)) + (2.0 * a));
-  if (v <= 0.0) return 0.0;
-  return sqrt(v) / ((x3 + a) - lam);
+  // where the orbit is timelike (v > 0), 1 - Omega lambda > 0 for every photon
+  const double g = div_rn(sqrt_rn(v), (x3 + a) - lam);
+  return (v <= 0.0) ? 0.0 : g;
 }
 
 // NovikovThorneDisk::normalizedFlux (src/physics/novikov_thorne.h:170-190)
 // with its scene constants r_isco and flux(1.5 r_isco) precomputed.
 __device__ __forceinline__ double nt_flux(double r, double r_isco, double flux_peak) {
   if (r < r_isco) return 0.0;
-  const double t = 1.0 - sqrt(r_isco / r);
+  const double t = 1.0 - sqrt_rn(div_rn(r_isco, r));
   const double fR = (0.0 < t) ? t : 0.0;
-  const double flux = fR / ((r * r) * r);
-  const double v = flux / flux_peak;
+  const double flux = div_rn(fR, (r * r) * r);
+  const double v = div_rn(flux, flux_peak);
   return (v < 1.0) ? v : 1.0;
 }
 

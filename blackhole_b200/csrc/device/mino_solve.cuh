@@ -126,10 +126,21 @@ BHM_HD T qsqrt(T x) {
   if constexpr (sizeof(T) == 8) {
     const double s = bhk::sqrt_rn(x);
     return x < 0.0 ? NAN : s;
+  } else {
+    return bhk::sqrt_rn_f(x);
   }
 #endif
   return sqrt(x);
 }
+// sin and cos of one angle.
+BHM_HD void sin_cos(float x, float& s, float& c) {
+#ifdef __CUDA_ARCH__
+  sincosf(x, &s, &c);
+#else
+  s = sin(x), c = cos(x);
+#endif
+}
+BHM_HD void sin_cos(double x, double& s, double& c) { s = sin(x), c = cos(x); }
 BHM_HD double qrcp(double b) {
 #ifdef __CUDA_ARCH__
   return bhk::rcp_near(b);
@@ -373,8 +384,8 @@ BHM_HD double pole_passes(const Polar& t, double tau) {
 // -0 continue the two sides, which agree modulo 2 pi.
 BHM_HD double phi_theta_crossing(const Polar& t, double lam, double tau) {
   if (!(t.zc > 0.0)) return copysign(3.141592653589793, lam) * pole_passes(t, tau);
-  const double j = rint((t.phi_start + tau) / t.period);
-  return lam * (tau + t.zp / t.sw * (2.0 * j * t.qc - t.q0));
+  const double j = rint(qdiv(t.phi_start + tau, t.period));
+  return lam * (tau + qdiv(t.zp, t.sw) * (2.0 * j * t.qc - t.q0));
 }
 
 // u = cos theta reached at Mino time tau (the ray must cross the equator:
@@ -384,36 +395,38 @@ BHM_HD double phi_theta_crossing(const Polar& t, double lam, double tau) {
 template <class T = double>
 BHM_HD double polar_at(const Polar& t, double lam, double tau, bool az, double& phi_th) {
   const double total = t.phi_start + tau;
-  const double n = floor(total / t.period);
+  const double n = floor(qdiv(total, t.period));
   double rem = total - n * t.period;  // in [0, 2K)
   const bool second = rem > t.K;
   if (second) rem = t.period - rem;   // chi' -> pi - chi' has the same sine
   // Phi(chi') = rem on [0, pi/2]: bracketed Newton.
   const T wT = T(t.w), mT = T(t.mm), remT = T(rem);
-  T lo = T(0), hi = T(1.5707963267948966), chi = T(rem * sqrt(t.w + 0.5 * t.mm));
+  T lo = T(0), hi = T(1.5707963267948966), chi = T(rem * qsqrt(t.w + 0.5 * t.mm));
   chi = fmin(fmax(chi, lo), hi);
   const T tol = sizeof(T) == 4 ? T(2e-7) : T(1e-15);
   for (int it = 0; it < 60; ++it) {
-    const T s = sin(chi), c = cos(chi);
+    T s, c;
+    sin_cos(chi, s, c);
     const T f = s * carlson_rf<T>(wT * c * c, wT + mT * s * s, wT) - remT;
     if (f < T(0)) lo = chi; else hi = chi;
-    T nc = chi - f * sqrt(wT + mT * s * s);
+    T nc = chi - f * qsqrt(wT + mT * s * s);
     if (!(nc > lo && nc < hi)) nc = T(0.5) * (lo + hi);
     const T step = nc - chi;
     chi = nc;
     if (fabs(step) < tol) break;
   }
-  const T s = sin(chi), c = cos(chi);
+  T s, c;
+  sin_cos(chi, s, c);
   if (az) {
     if (!(t.zc > 0.0)) {
       phi_th = copysign(3.141592653589793, lam) * pole_passes(t, tau);
     } else {
       const double qp = (double)q_part<T>(T(t.zc), s, c, T(t.m1));
       const double q = 2.0 * n * t.qc + (second ? 2.0 * t.qc - qp : qp);
-      phi_th = lam * (tau + t.zp / t.sw * (q - t.q0));
+      phi_th = lam * (tau + qdiv(t.zp, t.sw) * (q - t.q0));
     }
   }
-  const double sgn = (fmod(n, 2.0) != 0.0) ? -1.0 : 1.0;
+  const double sgn = n != 2.0 * floor(0.5 * n) ? -1.0 : 1.0;
   return sgn * t.sz * (double)s;
 }
 
@@ -521,7 +534,7 @@ BHM_HD float phi_weight_f(const RadialF& q, float x) {
 #endif
 }
 
-BHM_HD double radius_of(const Radial& q, double v) { return q.kind == 1 ? 1.0 / (q.x_tp - v * v) : 1.0 / v; }
+BHM_HD double radius_of(const Radial& q, double v) { return qdiv(1.0, q.kind == 1 ? q.x_tp - v * v : v); }
 
 // Mino time and, with PHI, the radial azimuth integral over an interval of v.
 struct TauPhi {
@@ -548,7 +561,7 @@ BHM_HD TauPhi integrate2(const Radial& q, double v0, double v1, double hmax) {
   }
   int n = (int)ceil(fabs(len) / hmax);
   n = n < 1 ? 1 : (n > 64 ? 64 : n);
-  const double h = len / n;
+  const double h = qdiv(len, (double)n);
   double sum = 0.0, sump = 0.0;
   for (int p = 0; p < n; ++p) {
     const double c = v0 + (p + 0.5) * h, hh = 0.5 * h;
@@ -591,7 +604,7 @@ BHM_HD TauPhi integrate_f2(const RadialF& q, double v0, double v1, double hmax) 
   }
   int n = (int)ceil(fabs(len) / hmax);
   n = n < 1 ? 1 : (n > 64 ? 64 : n);
-  const double h = len / n;
+  const double h = qdiv(len, (double)n);
   double sum = 0.0, sump = 0.0;
   for (int p = 0; p < n; ++p) {
     const float c = (float)(v0 + (p + 0.5) * h), hh = (float)(0.5 * h);
@@ -646,7 +659,7 @@ BHM_HD Radial radial_motion(double a2, double a2_alam, double C, double r_obs, d
     }
     if (!(r > r_hor) || !(r < r_obs)) return q;  // turning point inside the horizon cut or beyond the observer
     q.kind = 1;
-    q.x_tp = 1.0 / r;
+    q.x_tp = qdiv(1.0, r);
     // P(x) = (x - x_tp) Q(x) (synthetic division, remainder dropped); P / (x_tp - x) = -Q.
     const double b3 = q.p0;
     const double b2 = q.p1 + q.x_tp * b3;
@@ -656,12 +669,12 @@ BHM_HD Radial radial_motion(double a2, double a2_alam, double C, double r_obs, d
     q.q2 = -b2;
     q.q1 = -b1;
     q.q0 = -b0;
-    q.v_obs = -sqrt(q.x_tp - 1.0 / r_obs);
-    q.v_end = sqrt(q.x_tp - 1.0 / r_esc);
+    q.v_obs = -qsqrt(q.x_tp - qdiv(1.0, r_obs));
+    q.v_end = qsqrt(q.x_tp - qdiv(1.0, r_esc));
   } else {
     q.kind = 0;
-    q.v_obs = 1.0 / r_obs;
-    q.v_end = 1.0 / r_hor;
+    q.v_obs = qdiv(1.0, r_obs);
+    q.v_end = qdiv(1.0, r_hor);
   }
   return q;
 }
@@ -712,7 +725,7 @@ BHM_HD int solve_tau(const Quad<FAST, KIND, PHI>& Q, double T, double lo, double
       hi = v;
       end_known = true;
     }
-    double vn = v + (T - tv) / Q.at(v);
+    double vn = v + qdiv(T - tv, Q.at(v));
     if (!(vn < hi) && !end_known) {
       const double t_hi = tv + Q.integ(v, hi, hmax);
       if (t_hi < T) {
@@ -765,11 +778,11 @@ BHM_HD void crossing_loop(const Radial& q, const Polar& th, double r_in, double 
   double seed_v[2] = {NAN, NAN};
   if (r_seed > 0.0) {
     if (KIND == 1) {
-      const double s = sqrt(fmax(0.0, q.x_tp - 1.0 / r_seed));
+      const double s = qsqrt(fmax(0.0, q.x_tp - qdiv(1.0, r_seed)));
       seed_v[0] = -s;
       seed_v[1] = s;
     } else {
-      seed_v[0] = 1.0 / r_seed;
+      seed_v[0] = qdiv(1.0, r_seed);
     }
   }
   double lo = q.v_obs, tlo = 0.0, plo = 0.0;
@@ -866,7 +879,7 @@ BHM_HD double critical_distance(double r_min, double R_min, double a, double lam
   const double dR_deta = -D;
   const double gx = -dR_dlam * sin_o + dR_deta * 2.0 * alpha * cos_o * cos_o;
   const double gy = dR_deta * 2.0 * beta;
-  return fabs(R_min) / fmax(sqrt(gx * gx + gy * gy), 1e-300);
+  return qdiv(fabs(R_min), fmax(qsqrt(gx * gx + gy * gy), 1e-290));
 }
 
 }  // namespace bhmino
