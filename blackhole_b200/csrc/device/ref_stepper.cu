@@ -57,6 +57,31 @@ __device__ __forceinline__ Pot potentials(double r, double theta, double mass, d
   return p;
 }
 
+// sin^2 and cos^2 of |x| < 2^10. The angle less the nearest multiple of pi / 2,
+// which is taken in two parts, as r + rl; Taylor's series on |r| <= pi / 4 to
+// r^17 and r^16, summed in pairs (G. Estrin's scheme); sine and cosine within
+// 0.83 ulp each (2e7 arguments). CUDA's sincos has a branch for large arguments:
+// four calls a step keep its stages in blocks of their own, and the polar motion
+// is the step's longest chain.
+__device__ __forceinline__ void sin2_cos2(double x, double &s2, double &c2) {
+  const double t = fma(x, 0x1.45f306dc9c883p-1, 0x1.8p52);  // 2 / pi
+  const bool odd = __double2loint(t) & 1;
+  const double k = t - 0x1.8p52;
+  constexpr double hi = 0x1.921fb54442d18p0, lo = 0x1.1a62633145c07p-54;  // pi / 2
+  const double r1 = fma(-k, hi, x), r = fma(-k, lo, r1), rl = fma(-k, lo, r1 - r);
+  const double z = r * r, z2 = z * z, z4 = z2 * z2;
+  const double S = fma(fma(fma(1 / 355687428096000.0, z, -1 / 1307674368000.0), z2,
+                           fma(1 / 6227020800.0, z, -1 / 39916800.0)),
+                       z4, fma(fma(1 / 362880.0, z, -1 / 5040.0), z2, fma(1 / 120.0, z, -1 / 6.0)));
+  const double C = fma(fma(1 / 20922789888000.0, z2, fma(-1 / 87178291200.0, z, 1 / 479001600.0)), z4,
+                       fma(fma(-1 / 3628800.0, z, 1 / 40320.0), z2, fma(-1 / 720.0, z, 1 / 24.0)));
+  const double w = fma(-0.5, z, 1.0), e = fma(-0.5, z, 1.0 - w);
+  const double s = r + fma(r * z, S, rl * w), c = w + fma(z2, C, fma(-r, rl, e));
+  const double ss = s * s, cc = c * c;
+  s2 = odd ? cc : ss;
+  c2 = odd ? ss : cc;
+}
+
 // kerrMinoDerivatives (kerr.cpp:40-66). The reference recomputes the full
 // potentials (including the unused derivatives) and sin(theta) twice; the
 // values that feed the result are identical here.
@@ -65,10 +90,16 @@ __device__ __forceinline__ Dv mino_derivs(const St &s, double mass, double a, co
   const double r = s.r;
   const double rr = r * r;
   const double aa = a * a;
-  double sinTheta, cosTheta;
-  sincos(s.theta, &sinTheta, &cosTheta);
-  const double sin2 = mx(sinTheta * sinTheta, 1e-12);
-  const double cos2 = cosTheta * cosTheta;
+  double sin2, cos2;
+  if (fabs(s.theta) < 1024.0) {
+    sin2_cos2(s.theta, sin2, cos2);
+  } else {
+    double sinTheta, cosTheta;
+    sincos(s.theta, &sinTheta, &cosTheta);
+    sin2 = sinTheta * sinTheta;
+    cos2 = cosTheta * cosTheta;
+  }
+  sin2 = mx(sin2, 1e-12);
   const double delta = rr - (2.0 * mGeom * r) + aa;
   const double aFactor = ((rr + aa) * c.e) - (a * c.lz);
   const double lzMinusAe = c.lz - (a * c.e);
@@ -118,13 +149,16 @@ __device__ __noinline__ St step_mino_any(const St &state, double mass, double a,
 
 // ---- the same step with the branch-free quotients and roots (ieee_fp64.cuh) -------
 //
-// The same operations on the same values in the same order, so the same bits:
+// The same operations on the same values in the same order, so the same bits
+// (both take sin^2 and cos^2 from sin2_cos2):
 //   * the quotients by sin^2 share one reciprocal, those by Delta another;
 //   * products with 2 are exact, so fma(2, x, y) rounds as y + 2 x;
 //   * the first stage's potentials are those the trace loop tests for sign
 //     flips (kerr.cpp evaluates them twice).
 // It is bound by one ray's chain of FP64 operations: 4096 rays of up to 1500
-// steps take 4.53 ms with the operators and 1.60 ms here (one B200; 300,000 rays of 1000 steps: 14.3 and 8.7 ms).
+// steps take 4.53 ms with the operators, 1.56 ms without their branches and
+// 1.45 ms with sin2_cos2 in place of sincos as well (one B200; 300,000 rays of
+// 1000 steps: 14.3, 8.7 and 8.4 ms).
 // Operands must stay far from the ends of the exponent range: consts_ok() once
 // per ray, r and the stages' potentials per step; a step that fails is redone
 // by step_mino_any.
@@ -162,38 +196,52 @@ __device__ __forceinline__ bool consts_ok(const Geo &g, double dlam) {
          zero_or_in(g.lz, -200, 200) && zero_or_in(g.q, -400, 400) && zero_or_in(dlam, -200, 66);
 }
 
+// max(x, 1e-12), by the bits.
+__device__ __forceinline__ double at_least_tiny(double x) {
+  return __double_as_longlong(x) < __double_as_longlong(1e-12) ? 1e-12 : x;
+}
+
 // What a stage needs at (r, theta), before the signs.
 struct Raw {
-  double R, Th, y2, yd, A, rr, sin2, delta;
+  double R, Th, y2, yd, A, rr, sin2, delta, theta;
 };
 
 __device__ __forceinline__ Raw raw_at(double r, double theta, const Geo &g) {
   Raw w;
-  double sinTheta, cosTheta;
-  sincos(theta, &sinTheta, &cosTheta);
+  double sin2, cos2;
+  sin2_cos2(theta, sin2, cos2);
+  w.theta = theta;
   w.rr = r * r;
-  w.sin2 = mx(sinTheta * sinTheta, 1e-12);
+  w.sin2 = at_least_tiny(sin2);
   const double delta = w.rr - (g.twoM * r) + g.aa;
   w.A = ((w.rr + g.aa) * g.e) - g.alz;
   w.R = (w.A * w.A) - (delta * g.lzae2);
   w.y2 = bhk::rcp_near(w.sin2);
-  w.Th = g.q + (g.kTh * (cosTheta * cosTheta)) - bhk::div_by(g.lz2, w.sin2, w.y2);
-  w.delta = mx(delta, 1e-12);
+  w.Th = g.q + (g.kTh * cos2) - bhk::div_by(g.lz2, w.sin2, w.y2);
+  w.delta = at_least_tiny(delta);
   w.yd = bhk::rcp_near(w.delta);
   return w;
 }
 
 // |R| and |Theta| finite and below 2^860: no product of the stage overflowed.
+// The angle within sin2_cos2's range.
 __device__ __forceinline__ bool raw_ok(const Raw &w) {
   return (__double2hiint(w.R) & 0x7fffffff) < ((1023 + 860) << 20) &&
-         (__double2hiint(w.Th) & 0x7fffffff) < ((1023 + 860) << 20);
+         (__double2hiint(w.Th) & 0x7fffffff) < ((1023 + 860) << 20) &&
+         (__double2hiint(w.theta) & 0x7fffffff) < ((1023 + 10) << 20);
+}
+
+// sqrt(max(x, 0)).
+__device__ __forceinline__ double root_of_positive(double x) {
+  const double s = bhk::sqrt_rn(x);
+  return __double2hiint(x) < 0 ? 0.0 : s;
 }
 
 template <bool TIME>
 __device__ __forceinline__ Dv rates(const Raw &w, double signR, double signTheta, const Geo &g) {
   Dv d;
-  d.dr = signR * bhk::sqrt_rn(mx(w.R, 0.0));
-  d.dtheta = signTheta * bhk::sqrt_rn(mx(w.Th, 0.0));
+  d.dr = signR * root_of_positive(w.R);
+  d.dtheta = signTheta * root_of_positive(w.Th);
   d.dphi = bhk::div_by(g.lz, w.sin2, w.y2) - g.ae + bhk::div_by(g.a * w.A, w.delta, w.yd);
   d.dt = TIME ? bhk::div_by((w.rr + g.aa) * w.A, w.delta, w.yd) + (g.a * (g.lz - (g.ae * w.sin2))) : 0.0;
   return d;
