@@ -251,6 +251,11 @@ __host__ __device__ inline MediumF medium_f(const BhkRtParams &q) {
 }
 
 #ifdef __CUDACC__
+// Issue slots bound a transfer, most of them its samples': fmodf and eight
+// 64-bit indices here took 5 % of the 512^2 frame (2.84 -> 2.70 ms), and eight
+// 64-bit addresses again (2.58 -> 2.45). Off, the type of a byte offset into
+// the cells, is 32 bits up to 2^28 cells.
+template <class Off>
 __device__ __forceinline__ bool sample_f(const MediumF &q, float r, float u, float phi, float &n, float &th,
                                          float &b) {
   if (!(r >= q.r_min && r <= q.r_max)) return false;
@@ -264,13 +269,13 @@ __device__ __forceinline__ bool sample_f(const MediumF &q, float r, float u, flo
   const float fp = phi * (0.15915494309f * (float)q.n_ph);
   const float fl = floorf(fp);
   const float tp = fp - fl;
-  // fmodf and eight 64-bit indices here took 5 % of the 512^2 transfer (2.84 -> 2.70 ms)
   int k0 = (int)fl - q.n_ph * (int)floorf(fl * q.inv_n_ph);  // the rounded quotient is off by one at most
   k0 += k0 < 0 ? q.n_ph : (k0 >= q.n_ph ? -q.n_ph : 0);
   k0 = min(max(k0, 0), q.n_ph - 1);  // an azimuth that is no number
   const int k1 = (k0 + 1 == q.n_ph) ? 0 : k0 + 1;
-  const float4 *c00 = q.cells + ((long long)i0 * q.n_th + j0) * q.n_ph;
-  const long long row = (long long)q.n_th * q.n_ph;
+  const char *cells = reinterpret_cast<const char *>(q.cells);
+  const Off c00 = ((Off)i0 * (Off)q.n_th + (Off)j0) * (Off)q.n_ph * 16u, row = (Off)q.n_th * (Off)q.n_ph * 16u,
+            col = (Off)q.n_ph * 16u, o0 = c00 + (Off)k0 * 16u, o1 = c00 + (Off)k1 * 16u;
   float a0 = 0.0f, a1 = 0.0f, a2 = 0.0f;
 #pragma unroll
   for (int di = 0; di < 2; ++di)
@@ -279,7 +284,8 @@ __device__ __forceinline__ bool sample_f(const MediumF &q, float r, float u, flo
 #pragma unroll
       for (int dk = 0; dk < 2; ++dk) {
         const float w = (di ? tr : 1.0f - tr) * (dj ? tt : 1.0f - tt) * (dk ? tp : 1.0f - tp);
-        const float4 v = __ldg(c00 + (di ? row : 0) + (dj ? q.n_ph : 0) + (dk ? k1 : k0));
+        const float4 v =
+            __ldg(reinterpret_cast<const float4 *>(cells + ((dk ? o1 : o0) + (di ? row : 0u) + (dj ? col : 0u))));
         a0 = fmaf(w, v.x, a0);
         a1 = fmaf(w, v.y, a1);
         a2 = fmaf(w, v.z, a2);

@@ -690,15 +690,22 @@ __device__ __forceinline__ int rt_count_f(const bhrt::MediumF &q, float a2, cons
   return (int)fminf(fmaxf(ceilf(__fdividef(sig_m * h, q.ds_max)), 1.0f), 64.0f);
 }
 
+// What every sample of a launch shares: the horizons and the azimuth's a G(r).
+struct RtShared {
+  float rp, rmn, gscale, g_obs;
+};
+__device__ __forceinline__ RtShared rt_shared(const BhkImageParams &p) {
+  const float a = (float)p.a, rp = (float)p.r_plus, rmn = (float)p.r_minus, ro = (float)p.r_obs;
+  return RtShared{rp, rmn, a == 0.0f ? 0.0f : __fdividef(a, rp - rmn), __fdividef(ro - rmn, ro - rp)};
+}
+
 // Sample m of ns of the step y0 -> y1: e^(ln S), the fraction absorbed and the
 // optical depth (all zero outside the medium).
-__device__ __forceinline__ bool rt_sample_f(const BhkImageParams &p, const bhrt::MediumF &q, float a, float a2,
+template <class Off>
+__device__ __forceinline__ bool rt_sample_f(const RtShared &c, const bhrt::MediumF &q, float a, float a2,
                                             float lam, const Yf &y0, const Yf &k0, const Yf &y1, const Yf &k1,
                                             float h, float ns, int m, float &src, float &om, float &ts) {
   const float dt = __fdividef(h, ns);
-  const float rp = (float)p.r_plus, rmn = (float)p.r_minus, ro = (float)p.r_obs;
-  const float gscale = a == 0.0f ? 0.0f : __fdividef(a, rp - rmn);
-  const float g_obs = __fdividef(ro - rmn, ro - rp);
   const float t = __fdividef((float)m + 0.5f, ns);
   const float t2 = t * t, t3 = t2 * t;
   const float h00 = 2.0f * t3 - 3.0f * t2 + 1.0f, h10 = t3 - 2.0f * t2 + t;
@@ -706,10 +713,10 @@ __device__ __forceinline__ bool rt_sample_f(const BhkImageParams &p, const bhrt:
   const float r = h00 * y0.r + h10 * h * k0.r + h01 * y1.r + h11 * h * k1.r;
   const float u = h00 * y0.u + h10 * h * k0.u + h01 * y1.u + h11 * h * k1.u;
   const float psi = h00 * y0.phi + h10 * h * k0.phi + h01 * y1.phi + h11 * h * k1.phi;
-  const float phi = psi + gscale * __logf(__fdividef(r - rp, r - rmn) * g_obs);  // phi = psi + a (G(r) - G(r_obs))
+  const float phi = psi + c.gscale * __logf(__fdividef(r - c.rp, r - c.rmn) * c.g_obs);  // psi + a (G(r) - G(r_obs))
   float n, th, b;
   src = 0.0f, om = 0.0f, ts = 0.0f;
-  if (!bhrt::sample_f(q, r, u, phi, n, th, b)) return false;
+  if (!bhrt::sample_f<Off>(q, r, u, phi, n, th, b)) return false;
   const float g = bhrt::redshift_f(a, r, u, lam);
   float ln_alpha, ln_s;
   if (!bhrt::ln_emission_f(q, n, th, b, g, ln_alpha, ln_s)) return false;
@@ -724,12 +731,14 @@ __device__ __forceinline__ bool rt_sample_f(const BhkImageParams &p, const bhrt:
 // ray: neighbours (8 x 4 tiles) reach the medium together, so their samples
 // do too. New rays only when all 32 have ended -- filled lane by lane, the
 // 512^2 frame took 3.0 to 4.0 ms, its lanes at different depths, against 2.74.
+template <class Off>
 __global__ void __launch_bounds__(128) k_trace_rt_mixed(const __grid_constant__ BhkImageParams p,
                                                         const __grid_constant__ bhrt::MediumF q,
                                                         double *__restrict__ i_nu, double *__restrict__ tau_out,
                                                         int *__restrict__ cls_out, int *__restrict__ steps_out,
                                                         unsigned long long *__restrict__ counter) {
   const unsigned lane = threadIdx.x & 31u;
+  const RtShared sh = rt_shared(p);
   for (;;) {
     unsigned long long base = 0;
     if (lane == 0) base = atomicAdd(counter, 32ull);
@@ -769,7 +778,7 @@ __global__ void __launch_bounds__(128) k_trace_rt_mixed(const __grid_constant__ 
         const int nsub = rt_count_f(q, R.c.a2, y0, k0, R.y, d.k7, h);
         for (int m = 0; m < nsub; ++m) {
           float src, om, ts;
-          if (!rt_sample_f(p, q, R.c.a, R.c.a2, R.c.lam, y0, k0, R.y, d.k7, h, (float)nsub, m, src, om, ts)) continue;
+          if (!rt_sample_f<Off>(sh, q, R.c.a, R.c.a2, R.c.lam, y0, k0, R.y, d.k7, h, (float)nsub, m, src, om, ts)) continue;
           I += (double)(T * src * om);
           T *= 1.0f - om;
           tau += (double)ts;
@@ -802,6 +811,7 @@ __global__ void __launch_bounds__(128) k_trace_rt_mixed(const __grid_constant__ 
 // 0.39 / 0.48 / 0.73 / 1.25 ms against 0.96 / 0.88 / 1.03 / 1.38; past one wave
 // the plain loop is the faster (320^2: 1.77 against 1.47 ms, 512^2: 3.6 against
 // 2.6), since 32 full lanes need no search for their samples.
+template <class Off>
 __global__ void __launch_bounds__(128) k_trace_rt_mixed_few(const __grid_constant__ BhkImageParams p,
                                                             const __grid_constant__ bhrt::MediumF q,
                                                             double *__restrict__ i_nu, double *__restrict__ tau_out,
@@ -811,6 +821,7 @@ __global__ void __launch_bounds__(128) k_trace_rt_mixed_few(const __grid_constan
   bhrt::WarpSamples<float> &w = warps[threadIdx.x >> 5];
   const int lane = threadIdx.x & 31;
   const float a = (float)p.a, a2 = (float)(p.a * p.a);
+  const RtShared sh = rt_shared(p);
   for (;;) {
     unsigned long long base = 0;
     if (lane == 0) base = atomicAdd(counter, (unsigned long long)slots);
@@ -872,7 +883,7 @@ __global__ void __launch_bounds__(128) k_trace_rt_mixed_few(const __grid_constan
             const Yf k0{w.step[1][l], w.step[5][l], w.step[9][l], 0.0f, 0.0f};
             const Yf y1{w.step[2][l], w.step[6][l], w.step[10][l], 0.0f, 0.0f};
             const Yf k1{w.step[3][l], w.step[7][l], w.step[11][l], 0.0f, 0.0f};
-            rt_sample_f(p, q, a, a2, w.step[14][l], y0, k0, y1, k1, w.step[12][l], w.step[13][l], m, w.res[0][slot],
+            rt_sample_f<Off>(sh, q, a, a2, w.step[14][l], y0, k0, y1, k1, w.step[12][l], w.step[13][l], m, w.res[0][slot],
                         w.res[1][slot], w.res[2][slot]);
           },
           [&](int slot) {
@@ -894,27 +905,36 @@ __global__ void __launch_bounds__(128) k_trace_rt_mixed_few(const __grid_constan
 
 }  // namespace bhm
 
-extern "C" int bhk_trace_rt_mixed(const BhkImageParams *p, const BhkRtParams *q, double *i_nu, double *tau,
-                                  int32_t *cls, int32_t *steps, unsigned long long *counter, void *stream) {
-  cudaStream_t s = static_cast<cudaStream_t>(stream);
-  if (cudaMemsetAsync(counter, 0, sizeof(unsigned long long), s) != cudaSuccess) return -1;
+// Off: the type of a byte offset into the medium.
+template <class Off>
+static int trace_rt_mixed(const BhkImageParams *p, const bhrt::MediumF &m, double *i_nu, double *tau, int32_t *cls,
+                          int32_t *steps, unsigned long long *counter, cudaStream_t s) {
   int dev = 0, sms = 0, per_sm = 0;
   if (cudaGetDevice(&dev) != cudaSuccess ||
       cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess ||
-      cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, bhm::k_trace_rt_mixed, 128, 0) != cudaSuccess)
+      cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, bhm::k_trace_rt_mixed<Off>, 128, 0) != cudaSuccess)
     return -1;
-  const bhrt::MediumF m = bhrt::medium_f(*q);
   if (p->n_pix <= 128LL * sms * per_sm) {  // one wave
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, bhm::k_trace_rt_mixed_few, 128, 0) != cudaSuccess)
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, bhm::k_trace_rt_mixed_few<Off>, 128, 0) != cudaSuccess)
       return -1;
     const bhrt::Slots L = bhrt::slots_for(p->n_pix, (long long)sms * per_sm);
-    bhm::k_trace_rt_mixed_few<<<L.grid, 128, 0, s>>>(*p, m, i_nu, tau, cls, steps, counter, L.slots);
+    bhm::k_trace_rt_mixed_few<Off><<<L.grid, 128, 0, s>>>(*p, m, i_nu, tau, cls, steps, counter, L.slots);
     return cudaGetLastError() == cudaSuccess ? 0 : -1;
   }
   const long long need = (p->n_pix + 127) / 128;
   const int grid = (int)(need < (long long)sms * per_sm ? need : (long long)sms * per_sm);
-  bhm::k_trace_rt_mixed<<<grid > 0 ? grid : 1, 128, 0, s>>>(*p, m, i_nu, tau, cls, steps, counter);
+  bhm::k_trace_rt_mixed<Off><<<grid > 0 ? grid : 1, 128, 0, s>>>(*p, m, i_nu, tau, cls, steps, counter);
   return cudaGetLastError() == cudaSuccess ? 0 : -1;
+}
+
+extern "C" int bhk_trace_rt_mixed(const BhkImageParams *p, const BhkRtParams *q, double *i_nu, double *tau,
+                                  int32_t *cls, int32_t *steps, unsigned long long *counter, void *stream) {
+  cudaStream_t s = static_cast<cudaStream_t>(stream);
+  if (cudaMemsetAsync(counter, 0, sizeof(unsigned long long), s) != cudaSuccess) return -1;
+  const bhrt::MediumF m = bhrt::medium_f(*q);
+  const bool narrow = (unsigned long long)m.n_r * (unsigned long long)m.n_th <= (1ull << 28) / (unsigned)m.n_ph;
+  return narrow ? trace_rt_mixed<unsigned>(p, m, i_nu, tau, cls, steps, counter, s)
+                : trace_rt_mixed<unsigned long long>(p, m, i_nu, tau, cls, steps, counter, s);
 }
 
 extern "C" int bhk_trace_image_mixed(const BhkImageParams *p, const BhkImageOut *o, unsigned long long *counter,
