@@ -267,9 +267,11 @@ __global__ void __launch_bounds__(256) k_post_tone(const float *__restrict__ src
                                                    float4 *__restrict__ fb) {
   const int pitch = PLANAR ? plane_pitch(w) : w;
   const int64_t plane = (int64_t)h * pitch;
-  auto at = [&](int y, int x, int c) {
-    const int64_t i = (int64_t)y * pitch + x;
-    return PLANAR ? src[c * plane + i] : src[4 * i + c];
+  // red and blue of one pixel
+  auto red_blue = [&](int64_t i) {
+    if (PLANAR) return make_float2(src[i], src[2 * plane + i]);
+    const float4 v = reinterpret_cast<const float4 *>(src)[i];
+    return make_float2(v.x, v.z);
   };
   const int px = blockIdx.x * 64 + (threadIdx.x & 63);
   const int y0 = (blockIdx.y * 4 + (threadIdx.x >> 6)) * kToneRows;
@@ -284,12 +286,14 @@ __global__ void __launch_bounds__(256) k_post_tone(const float *__restrict__ src
     const int64_t i = (int64_t)py * w + px;
     const float v = __fdiv_rn((float)py, (float)h);
     const int ry = min(max((int)__fmul_rn(v, (float)h), 0), h - 1);
-    const float red = at(ry, rx, 0), gch = at(py, px, 1), blue = at(ry, rx, 2);
+    const float2 rb = red_blue((int64_t)ry * pitch + rx);
+    const int64_t g = (int64_t)py * pitch + px;
+    const float gch = PLANAR ? src[plane + g] : src[4 * g + 1];
     const float dv = v - 0.5f;
     const float dist = sqrtf(du * du + dv * dv);
     const float vig = sqrtf(fmaxf(1.0f - dist * dist * 0.5f, 0.0f));
-    fb[i] = make_float4(tone_channel(red, exposure, vig), tone_channel(gch, exposure, vig),
-                        tone_channel(blue, exposure, vig), 1.0f);
+    fb[i] = make_float4(tone_channel(rb.x, exposure, vig), tone_channel(gch, exposure, vig),
+                        tone_channel(rb.y, exposure, vig), 1.0f);
   }
 }
 
