@@ -181,7 +181,7 @@ __device__ __forceinline__ F2 mul2(F2 a, F2 b) {
 // The step's arithmetic in pairs, (r, u) and (p_r, p_u): r' = p_r and u' = p_u, so
 // a stage's momenta pair is its position derivative pair, and psi, which no
 // right-hand side reads, stays a scalar quadrature. Issue slots bound the mixed
-// tracers (70 % issue, no pipe above half): 48 uneven frames 15.3 -> 14.2 ms,
+// tracers (70 % issue, no pipe above half): 48 uneven frames 15.3 -> 14.4 ms,
 // the 1920 x 1080 camera frame 1.86 -> 1.75 ms (one B200), same bits.
 __device__ __forceinline__ DPf dp45(const Yf &y, float h, const RayCf &c, const Yf &k1, float rtol, float atol,
                                     bool want_err) {

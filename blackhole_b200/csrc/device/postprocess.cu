@@ -48,12 +48,16 @@
 // mapping.
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <cstdint>
 #include <type_traits>
 
 #include "launch.h"
 
 namespace {
+
+// Rows of tiles in a grid's second dimension; taller images take the third.
+constexpr unsigned kMaxY = 65535;
 
 constexpr int kHalo = 32;  // the largest blur half-width
 constexpr int kRun = 8;    // outputs per thread along the blur direction
@@ -124,7 +128,7 @@ __global__ void __launch_bounds__(kRowsThreads, 5) k_post_rows(const __grid_cons
                                                                const float4 *__restrict__ fb, int w, int h,
                                                                float threshold, float *__restrict__ planes) {
   __shared__ float2 sm[3 * kRowPairs * kRowsPitch];  // bright-pass
-  const int x0 = blockIdx.x * kRowsX, y0 = blockIdx.y * kRowsY;
+  const int x0 = blockIdx.x * kRowsX, y0 = (blockIdx.y + kMaxY * blockIdx.z) * kRowsY;
   const int pitch = plane_pitch(w);
   const int64_t plane = (int64_t)h * pitch;
   constexpr int kPairs = kRowPairs * kRowsW, kInFlight = 3;  // 6 pixels a thread
@@ -211,7 +215,7 @@ __global__ void __launch_bounds__(kColsThreads, 7) k_post_cols(const __grid_cons
                                                                float *__restrict__ planes, int w, int h,
                                                                float strength) {
   extern __shared__ float cols_sm[];  // two buffers of [kColsH][kColsX]: scale si in buffer si % 2
-  const int x0 = blockIdx.x * kColsX, y0 = blockIdx.y * kColsY, c = blockIdx.z;
+  const int x0 = blockIdx.x * kColsX, y0 = (blockIdx.y + kMaxY * (blockIdx.z / 3)) * kColsY, c = blockIdx.z % 3;
   const int lane = threadIdx.x % (kColsX / 2), grp = threadIdx.x / (kColsX / 2);
   const int pitch = plane_pitch(w);
   auto fetch = [&](int si) {
@@ -259,10 +263,13 @@ __device__ __forceinline__ float tone_channel(float x, float exposure, float vig
   return powf(fmaxf(aces((x * exposure) * vignette), 0.0f), 1.0f / 2.2f);
 }
 
-// A thread has one column of 4 rows, so that u and the column index are worked out once.
+// A thread has one column of ROWS rows, so that u and the column index are
+// worked out once: 4 (1920 x 1080: 30 -> 28 us), but 1 where one wave of threads
+// holds the image and a thread's own chain of powf is the time (100 x 60 with
+// bloom: 44 and 41 us a call).
 // PLANAR: the composite is in three planes, otherwise a copy of the framebuffer.
-constexpr int kToneRows = 4;
-template <bool PLANAR>
+constexpr int kToneWave = 148 * 2048;
+template <bool PLANAR, int ROWS>
 __global__ void __launch_bounds__(256) k_post_tone(const float *__restrict__ src, int w, int h, float exposure,
                                                    float4 *__restrict__ fb) {
   const int pitch = PLANAR ? plane_pitch(w) : w;
@@ -274,13 +281,13 @@ __global__ void __launch_bounds__(256) k_post_tone(const float *__restrict__ src
     return make_float2(v.x, v.z);
   };
   const int px = blockIdx.x * 64 + (threadIdx.x & 63);
-  const int y0 = (blockIdx.y * 4 + (threadIdx.x >> 6)) * kToneRows;
+  const int y0 = ((blockIdx.y + kMaxY * blockIdx.z) * 4 + (threadIdx.x >> 6)) * ROWS;
   if (px >= w) return;
   const float u = __fdiv_rn((float)px, (float)w);
   const int rx = min(max((int)__fmul_rn(u, (float)w), 0), w - 1);
   const float du = u - 0.5f;
 #pragma unroll
-  for (int k = 0; k < kToneRows; ++k) {
+  for (int k = 0; k < ROWS; ++k) {
     const int py = y0 + k;
     if (py >= h) break;
     const int64_t i = (int64_t)py * w + px;
@@ -307,21 +314,29 @@ extern "C" int bhk_post_process(float *fb, int w, int h, const BhkPostTaps *taps
   if (w <= 0 || h <= 0) return 0;
   const cudaStream_t st = static_cast<cudaStream_t>(stream);
   float4 *f4 = reinterpret_cast<float4 *>(fb);
-  const dim3 gt((w + 63) / 64, (h + 4 * kToneRows - 1) / (4 * kToneRows));
+  auto tiles = [&](unsigned tx, unsigned ty, unsigned channels) {
+    const unsigned rows = ((unsigned)h + ty - 1) / ty;
+    return dim3(((unsigned)w + tx - 1) / tx, std::min(rows, kMaxY), (rows + kMaxY - 1) / kMaxY * channels);
+  };
+  auto tone = [&](auto planar, const float *src) {
+    constexpr bool kPlanar = decltype(planar)::value;
+    if ((int64_t)w * h <= kToneWave)
+      k_post_tone<kPlanar, 1><<<tiles(64, 4, 1), 256, 0, st>>>(src, w, h, exposure, f4);
+    else
+      k_post_tone<kPlanar, 4><<<tiles(64, 16, 1), 256, 0, st>>>(src, w, h, exposure, f4);
+  };
   if (strength != 0.0f) {
     constexpr int smem = sizeof(float) * 2 * kColsBuf;
     if (cudaFuncSetAttribute(k_post_cols, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess)
       return -1;
     Taps2 t2;
     for (int i = 0; i < 124; ++i) t2.w[i] = make_float2(taps->w[i], taps->w[i]);
-    const dim3 gr((w + kRowsX - 1) / kRowsX, (h + kRowsY - 1) / kRowsY);
-    k_post_rows<<<gr, kRowsThreads, 0, st>>>(t2, f4, w, h, threshold, scratch);
-    const dim3 gc((w + kColsX - 1) / kColsX, (h + kColsY - 1) / kColsY, 3);
-    k_post_cols<<<gc, kColsThreads, smem, st>>>(t2, scratch, w, h, strength);
-    k_post_tone<true><<<gt, 256, 0, st>>>(scratch + (int64_t)kBase * plane_pitch(w) * h, w, h, exposure, f4);
+    k_post_rows<<<tiles(kRowsX, kRowsY, 1), kRowsThreads, 0, st>>>(t2, f4, w, h, threshold, scratch);
+    k_post_cols<<<tiles(kColsX, kColsY, 3), kColsThreads, smem, st>>>(t2, scratch, w, h, strength);
+    tone(std::true_type{}, scratch + (int64_t)kBase * plane_pitch(w) * h);
   } else {
     if (cudaMemcpyAsync(scratch, fb, sizeof(float4) * w * h, cudaMemcpyDeviceToDevice, st) != cudaSuccess) return -1;
-    k_post_tone<false><<<gt, 256, 0, st>>>(scratch, w, h, exposure, f4);
+    tone(std::false_type{}, scratch);
   }
   return cudaGetLastError() == cudaSuccess ? 0 : -1;
 }
