@@ -728,7 +728,7 @@ def run_analytic(args, rank: int, world: int, dist):
                               "speedup_vs_fp64_plain": ms64 / ms_d},
     }
     # Outputs are the only HBM traffic (no inputs): the roofline below is the
-    # HBM one, far from binding; the kernel is bound by instruction fetch
+    # HBM one, far from binding; the kernel is bound by FP64 latency
     # (profiles/k_trace_image_analytic_disk1_512.md).
     out_bytes = sum(t.numel() * t.element_size() for t in outs.values())
     peaks = json.loads((ROOT / "MEASURED_PEAKS.json").read_text()) if (ROOT / "MEASURED_PEAKS.json").exists() else {}
@@ -738,7 +738,7 @@ def run_analytic(args, rank: int, world: int, dist):
                 "frac": achieved / (peak or 6650.0), "traffic": None, "kernel": "k_trace_image_analytic",
                 "bytes_per_launch": out_bytes,
                 "peak_source": "MEASURED_PEAKS.json hbm_gbs (of measured)" if peak else "fallback 6.65 TB/s",
-                "note": "algorithmic bytes = the outputs written; the kernel is bound by instruction fetch, not HBM"}
+                "note": "algorithmic bytes = the outputs written; the kernel is bound by FP64 latency and its phase barriers, not HBM"}
     e2e = None
     if rank == 0:
         fields = ("cls", "n_cross", "r_hit", "g", "flux", "intensity")
