@@ -15,8 +15,10 @@
 // the result is the correctly rounded one unless the exact value lies that
 // close to the midpoint of two doubles. They serve operands whose quotient
 // and remainder stay in the normal range (|a|, |b| in 1e-290 .. 1e300, or a
-// = 0); beyond it a quotient is NaN or 0, which the step controller rejects
-// like the overflow it stands for.
+// = 0). Beyond it a quotient may be NaN or 0 where the operator's is not: a / b
+// with an infinite a or b, or a zero or subnormal b, is NaN, and the root of
+// infinity is NaN. The step controller rejects that like the overflow it stands
+// for; elsewhere the callers keep such operands out.
 //
 // What it bought (one B200, outputs bit for bit the same): the FP64 pipe was
 // 57 % busy in a DP45 frame, "wait" (fixed latency) the first stall. 640 x 360

@@ -177,13 +177,15 @@ __device__ __forceinline__ void synchrotron(const BhkRtParams &q, double n, doub
   if (!(n > 0.0 && theta_e > 0.0 && b > 0.0 && nu_e > 0.0)) return;
   const double nu_b = (kE / (kTwoPi * kMe * kC)) * b;
   const double nu_s = 1.5 * nu_b * theta_e * theta_e;
-  const double lx = log(bhk::div_rn(nu_e, nu_s));
+  // an infinite Theta_e or |B| (div_rn wants finite operands) is the table's lower end, as x = 0 is
+  const double lx = nu_s < INFINITY ? log(bhk::div_rn(nu_e, nu_s)) : -INFINITY;
   if (lx > q.lx1) return;  // beyond the table: exp(-1.89 x^(1/3)) below any use
   const double lt = log(theta_e);
   double ft = (lt - q.lt0) * q.lt_scale;
   double fx = (lx - q.lx0) * q.lx_scale;
-  ft = ft < 0.0 ? 0.0 : (ft > (double)(q.n_lt - 1) ? (double)(q.n_lt - 1) : ft);
-  fx = fx < 0.0 ? 0.0 : (fx > (double)(q.n_lx - 1) ? (double)(q.n_lx - 1) : fx);
+  // a coordinate that is no number takes node 0 too: as an integer it would be INT_MIN
+  ft = ft > 0.0 ? (ft > (double)(q.n_lt - 1) ? (double)(q.n_lt - 1) : ft) : 0.0;
+  fx = fx > 0.0 ? (fx > (double)(q.n_lx - 1) ? (double)(q.n_lx - 1) : fx) : 0.0;
   int i0 = (int)floor(ft), k0 = (int)floor(fx);
   i0 = i0 > q.n_lt - 2 ? q.n_lt - 2 : i0;
   k0 = k0 > q.n_lx - 2 ? q.n_lx - 2 : k0;

@@ -333,7 +333,7 @@ __device__ __forceinline__ void rt_sample(const BhkImageParams &p, const BhkRtPa
     if (g > 0.0) {
       double j, al;
       bhrt::synchrotron(q, n, th, b, div_rn(q.nu, g), j, al);
-      const double jo = g * g * j, ao = div_rn(al, g);
+      const double jo = g * g * j, ao = al < INFINITY ? div_rn(al, g) : al;  // div_rn wants finite operands
       const double ds = dl * q.length_cm;
       ts = ao * ds;
       om = (ts < 1.0e-4) ? ts * (1.0 - 0.5 * ts) : -expm1(-ts);
