@@ -9,6 +9,7 @@
 #pragma once
 
 #include "launch.h"
+#include "tile_order.h"
 
 namespace bhsrc {
 
@@ -41,29 +42,7 @@ constexpr int kTurnsRk4 = 32, kTurnsDp45 = 8;
 // Lane states of the persistent tracers.
 enum : int { kEmpty = -1, kRun = -2, kCross = -3, kCrossStop = -4 };  // >= 0: ended with that class
 
-// Pixel w of a frame in the order the tracers take them: bands of 4 rows, in
-// a band 8 x 4 tiles, so that a warp's 32 rays are neighbours in both
-// directions and reach the disk, the hole or the sky at about the same step.
-__device__ __forceinline__ long long tile_pixel(long long w, int width, long long n_pix) {
-  if (n_pix > 0x7fffffffLL) return w;
-  const unsigned W = (unsigned)width, n = (unsigned)n_pix, q = (unsigned)w;
-  const unsigned band = q / (4u * W), r0 = 4u * band;
-  const unsigned in = q - r0 * W, rows = min(4u, n / W - r0);
-  const unsigned tiled = (W & ~7u) * rows;
-  unsigned x, y;
-  if (in < tiled) {
-    const unsigned t = in / (8u * rows), i = in - t * 8u * rows;
-    x = 8u * t + (i & 7u);
-    y = i >> 3;
-  } else {
-    const unsigned rest = W & 7u, i = in - tiled;
-    y = i / rest;
-    x = (W & ~7u) + i - y * rest;
-  }
-  return (long long)(r0 + y) * width + x;
-}
-
-// The same for a frame of one wave (every ray has a lane from the start), with
+// tile_pixel for a frame of one wave (every ray has a lane from the start), with
 // its tiles shuffled (a bijection of [0, 2^k) by two xor shifts and a product
 // with an odd number, repeated until it falls below the number of tiles): rays
 // that run long -- past the hole and out again, twice the others' RK4 steps --
