@@ -49,6 +49,7 @@ static_assert(sizeof(CUtensorMap) == 128 && kMaps <= 24, "BhsTrainPlan::maps");
 struct PassArgs {
   const float* in;
   const float* targets;
+  int targets16;  // targets start on 16 bytes
   const float* params;
   __nv_bfloat16* dout;
   float* y[3];
@@ -355,11 +356,16 @@ __global__ void __launch_bounds__(kPassThreads, 1)
       if (!ok) break;
       float t[BHS_TARGETS];
       if (hf == 0) {
-        const float4* tp = reinterpret_cast<const float4*>(A.targets) + row * 4;
+        if (A.targets16) {
+          const float4* tp = reinterpret_cast<const float4*>(A.targets) + row * 4;
 #pragma unroll
-        for (int i = 0; i < 4; ++i) {
-          const float4 f = tp[i];
-          t[4 * i] = f.x, t[4 * i + 1] = f.y, t[4 * i + 2] = f.z, t[4 * i + 3] = f.w;
+          for (int i = 0; i < 4; ++i) {
+            const float4 f = tp[i];
+            t[4 * i] = f.x, t[4 * i + 1] = f.y, t[4 * i + 2] = f.z, t[4 * i + 3] = f.w;
+          }
+        } else {
+#pragma unroll
+          for (int i = 0; i < BHS_TARGETS; ++i) t[i] = A.targets[row * BHS_TARGETS + i];
         }
       }
       wait_acc();
@@ -683,6 +689,7 @@ extern "C" int bhs_launch_train(const BhsTrainBuffers* b, const BhsTrainPlan* pl
   PassArgs p{};
   p.in = inputs;
   p.targets = targets;
+  p.targets16 = (reinterpret_cast<uintptr_t>(targets) & 15u) == 0 ? 1 : 0;
   p.params = b->params;
   p.dout = b->dout;
   for (int i = 0; i < 3; ++i) p.y[i] = b->y[i];

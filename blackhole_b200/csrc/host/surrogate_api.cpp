@@ -135,6 +135,8 @@ int forward_backward(BH_Surrogate *s, const float *inputs, const float *targets,
   if (B <= 0 || B > s->max_batch || B % 128 != 0)
     return fail_msg("surrogate: batch %lld must be a positive multiple of 128 up to %lld", static_cast<long long>(B),
                     static_cast<long long>(s->max_batch));
+  if ((reinterpret_cast<uintptr_t>(inputs) & 15u) != 0)
+    return fail_msg("surrogate: training inputs must start on 16 bytes (a row is read at once)");
   if (s->plan.batch != B) {
     s->plan.batch = 0;
     if (bhs_train_plan(&s->tr, B, &s->plan) != 0) return fail_msg("surrogate: tensor maps of the training batch failed");

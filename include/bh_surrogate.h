@@ -71,7 +71,9 @@ int bh_surrogate_forward(BH_Surrogate* s, const float* inputs, int64_t n, float*
 /* Loss gradient w.r.t. every parameter (FP32, bh_surrogate_param_count()
  * values) for one batch; loss4 (4 floats, may be NULL) receives the sums of
  * cross entropy, squared regression error, correctly classified rows and
- * classified rows. Parameters are not changed. */
+ * classified rows. Parameters are not changed. inputs starts on 16 bytes (a
+ * row is read at once; -1 otherwise, here and in bh_surrogate_train_step),
+ * targets on 4 like any float array. */
 int bh_surrogate_gradients(BH_Surrogate* s, const float* inputs, const float* targets, int64_t batch,
                            float* grad, float* loss4, void* stream);
 
