@@ -120,6 +120,13 @@ __device__ __forceinline__ void row_loss(const float (&o)[BHS_HEAD], const float
 // product after an epilogue starts on the 64-column chunks that are done.
 // Product 5 goes beside layer 3's pre-activations, which its epilogue still
 // needs: product 6 alone waits for all of that epilogue.
+//
+// An operand set is read by a product and copied to HBM, both of which see
+// its chunks' `ready` phases; the epilogue completes a chunk's next phase only
+// after both have passed the last one (acc_full and `stored` follow it). Set 5
+// has no copy and set 9 no product, so they have barriers of their own
+// (dout_ready, out_ready): on the shared ones a reader that does not wait for
+// them could fall two phases behind, which looks like none.
 __device__ __forceinline__ int set_chunks(int s) { return s == 0 ? 3 : (s == 5 ? 1 : 4); }
 __device__ __forceinline__ uint32_t acc_col(int s) { return (0x14Au >> s) & 1u ? 256u : 0u; }  // s = 1, 3, 6, 8
 
@@ -132,14 +139,16 @@ __global__ void __launch_bounds__(kPassThreads, 1)
   const uint32_t ring = act + 4u * kChunk;
   float* sb = reinterpret_cast<float*>(smem_raw + pad + 4 * kChunk + kWRing * kWStage);
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem_raw + pad + 4 * kChunk + kWRing * kWStage + kBiases * 4 + 64);
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 2 * kWRing + 7);
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 2 * kWRing + 12);
   const uint32_t b0 = umma::smem_u32(bars);
   auto full = [&](int i) { return b0 + 8u * i; };
   auto empty = [&](int i) { return b0 + 8u * (kWRing + i); };
-  auto ready = [&](int c) { return b0 + 8u * (2 * kWRing + c); };  // chunk c of an operand set is written
+  auto ready = [&](int c) { return b0 + 8u * (2 * kWRing + c); };  // chunk c of operand sets 0..4, 6..8 is written
   const uint32_t acc_full = b0 + 8u * (2 * kWRing + 4);
   const uint32_t stored = b0 + 8u * (2 * kWRing + 5);  // the operand set has been read by its copy to HBM
   const uint32_t drained = b0 + 8u * (2 * kWRing + 6);
+  const uint32_t dout_ready = b0 + 8u * (2 * kWRing + 7);               // set 5 (one chunk) is written
+  auto out_ready = [&](int c) { return b0 + 8u * (2 * kWRing + 8 + c); };  // chunk c of set 9 is written
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int64_t tiles = A.B / kTile;
 
@@ -148,7 +157,11 @@ __global__ void __launch_bounds__(kPassThreads, 1)
       umma::mbar_init(full(i), 1);
       umma::mbar_init(empty(i), 1);
     }
-    for (int c = 0; c < 4; ++c) umma::mbar_init(ready(c), kEpiWarps);
+    for (int c = 0; c < 4; ++c) {
+      umma::mbar_init(ready(c), kEpiWarps);
+      umma::mbar_init(out_ready(c), kEpiWarps);
+    }
+    umma::mbar_init(dout_ready, kEpiWarps);
     umma::mbar_init(acc_full, 1);
     umma::mbar_init(stored, 1);
     umma::mbar_init(drained, 1);
@@ -190,23 +203,26 @@ __global__ void __launch_bounds__(kPassThreads, 1)
     }
   } else if (warp == 1) {
     if (lane == 0) {  // MMA issuer
-      uint32_t it = 0, seen[4] = {0u, 0u, 0u, 0u};
+      uint32_t it = 0, seen[4] = {0u, 0u, 0u, 0u}, tiles_seen = 0;
       bool ok = true;
-      auto wait_ready = [&](int c) {
-        if (ok && !umma::mbar_wait(ready(c), seen[c] & 1u, A.wait_ns)) {
+      auto wait_on = [&](uint32_t bar, uint32_t phases) {
+        if (ok && !umma::mbar_wait(bar, phases & 1u, A.wait_ns)) {
           atomicExch(A.err, kErrMma);
           ok = false;
         }
-        ++seen[c];
       };
-      for (int64_t tile = blockIdx.x; ok && tile < tiles; tile += gridDim.x) {
+      auto wait_ready = [&](int c) { wait_on(ready(c), seen[c]++); };
+      for (int64_t tile = blockIdx.x; ok && tile < tiles; tile += gridDim.x, ++tiles_seen) {
         for (int s = 0; ok && s < 9; ++s) {
           const uint32_t idesc = umma::idesc_bf16_f32(kTile, s == 4 ? BHS_HEAD : BHS_HIDDEN);
           const uint32_t d = tmem + acc_col(s);
           if (s == 6)
             for (int c = 0; c < 4; ++c) wait_ready(c);
           for (int c = 0; ok && c < set_chunks(s); ++c, ++it) {
-            if (s != 6) wait_ready(c);
+            if (s == 5)
+              wait_on(dout_ready, tiles_seen);
+            else if (s != 6)
+              wait_ready(c);
             const int st = (int)(it % kWRing);
             if (ok && !umma::mbar_wait(full(st), (it / kWRing) & 1, A.wait_ns)) {
               atomicExch(A.err, kErrMma);
@@ -225,31 +241,30 @@ __global__ void __launch_bounds__(kPassThreads, 1)
           }
           if (ok) umma::mma_commit(acc_full);
         }
-        for (int c = 0; c < 4; ++c) wait_ready(c);  // set 9: no product, but its phases count
       }
       umma::mma_commit(drained);
       umma::mbar_wait(drained, 0, kDrainNs);
     }
   } else if (warp == 2) {
     if (lane == 0) {  // copies each operand set to HBM as its chunks are written
-      uint32_t seen[4] = {0u, 0u, 0u, 0u};
+      uint32_t seen[4] = {0u, 0u, 0u, 0u}, tiles_seen = 0;
       bool ok = true;
-      for (int64_t tile = blockIdx.x; ok && tile < tiles; tile += gridDim.x)
+      for (int64_t tile = blockIdx.x; ok && tile < tiles; tile += gridDim.x, ++tiles_seen)
         for (int s = 0; ok && s < 10; ++s) {
+          if (s == 5) continue;  // dout is written to HBM by the epilogue itself
           const CUtensorMap* map = s == 0 ? &M.m[kMapF] : (s < 5 ? &M.m[kMapH + s - 1] : &M.m[kMapDY + 9 - s]);
           for (int c = 0; c < set_chunks(s); ++c) {
-            if (!umma::mbar_wait(ready(c), seen[c] & 1u, A.wait_ns)) {
+            if (!umma::mbar_wait(s == 9 ? out_ready(c) : ready(c), (s == 9 ? tiles_seen : seen[c]++) & 1u,
+                                 A.wait_ns)) {
               atomicExch(A.err, kErrDone);
               ok = false;
               break;
             }
-            ++seen[c];
-            if (s == 5) continue;
             for (int half = 0; half < 2; ++half)
               tma_store_2d(map, act + (uint32_t)c * kChunk + (uint32_t)half * (kChunk / 2), c * kBK,
                            (int)(tile * kTile) + 64 * half);
           }
-          if (!ok || s == 5) continue;
+          if (!ok) continue;
           bulk_commit();
           bulk_wait_read();
           umma::mbar_arrive(stored);
@@ -263,12 +278,13 @@ __global__ void __launch_bounds__(kPassThreads, 1)
     const uint32_t tacc = tmem + ((uint32_t)(q * 32) << 16);
     uint32_t acc_seen = 0, stores = 0, stores_seen = 0;
     bool ok = true;
-    auto chunk_done = [&](int c) {  // one arrival a warp: an arrival is an atomic on one word
+    auto arrive_on = [&](uint32_t bar) {  // one arrival a warp: an arrival is an atomic on one word
       umma::fence_async_smem();
       umma::tc_fence_before();
       __syncwarp();
-      if (lane == 0) umma::mbar_arrive(ready(c));
+      if (lane == 0) umma::mbar_arrive(bar);
     };
+    auto chunk_done = [&](int c) { arrive_on(ready(c)); };
     // the copy of the last set has read the tile's buffer
     auto wait_stored = [&]() {
       if (stores == stores_seen) return;
@@ -397,7 +413,7 @@ __global__ void __launch_bounds__(kPassThreads, 1)
           if (lane == 0 && v != 0.0f) atomicAdd(A.loss + i, v);
         }
       }
-      chunk_done(0);
+      arrive_on(dout_ready);
       for (int s = 5; s < 9; ++s) {  // dY_l = (dY_(l+1) W_(l+1)) * SiLU'(Y_l)
         const int l = 8 - s;
         const float4* ys = l < 3 ? reinterpret_cast<const float4*>(A.y[l]) + tile * (kTile * BHS_HIDDEN / 4) : nullptr;
@@ -432,7 +448,7 @@ __global__ void __launch_bounds__(kPassThreads, 1)
 #pragma unroll
           for (int i = 0; i < 16; ++i) v[i] *= silu_grad(y[i]);
           put16(c, v);
-          chunk_done(c);
+          arrive_on(s == 8 ? out_ready(c) : ready(c));
           const float s1 = column_sum(c, 2 * hf);
           if (lane < 16) bias_out[l * BHS_HIDDEN + col + lane] = s1;
         }
