@@ -297,7 +297,7 @@ __device__ __forceinline__ int rt_count(const BhkImageParams &p, const BhkRtPara
   if (rlow > q.r_max) return 0;
   double ns = ceil(div_rn(sig_m * h, q.ds_max));
   ns = ns < 1.0 ? 1.0 : (ns > 64.0 ? 64.0 : ns);
-  return (int)ns;
+  return ns > 0.0 ? (int)ns : 0;  // no number: none, as an integer it would be INT_MIN in the warp's sum
 }
 
 using RtWarp = bhrt::WarpSamples<double>;

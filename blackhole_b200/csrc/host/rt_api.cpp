@@ -3,6 +3,7 @@
 // radiative-transfer image.
 #include <cuda_runtime_api.h>
 
+#include <algorithm>
 #include <cmath>
 #include <vector>
 
@@ -116,6 +117,9 @@ int bh_kerr_trace_rt(const BH_KerrScene *scene, const BH_GrmhdGrid *grid, const 
   bh_rt_defaults(&r);
   if (rt) r = *rt;
   if (!(r.nu_hz > 0.0 && r.length_cm > 0.0 && r.ds_max > 0.0)) return bhh_fail("bh_kerr_trace_rt: bad transfer parameters");
+  if (grid->n_r < 2 || grid->n_theta < 2 || grid->n_phi < 1)
+    return bhh_fail("bh_kerr_trace_rt: the grid needs >= 2 nodes in r and theta and >= 1 in phi");
+  if (lut->n_theta < 2 || lut->n_x < 2) return bhh_fail("bh_kerr_trace_rt: the emission table needs >= 2 nodes per axis");
   BH_KerrScene sc = *scene;
   const bool mixed = scene->precision == BH_PRECISION_MIXED;
   sc.precision = BH_PRECISION_FP64;  // launch shape of the FP64 kernel; the mixed one sizes its own grid
@@ -144,7 +148,9 @@ int bh_kerr_trace_rt(const BH_KerrScene *scene, const BH_GrmhdGrid *grid, const 
   q.lx_scale = (q.n_lx - 1) / (q.lx1 - q.lx0);
   q.nu = r.nu_hz;
   q.length_cm = r.length_cm;
-  q.ds_max = r.ds_max;
+  // A step has 1 to 64 samples: beyond these bounds the number is one of the two
+  // for every step, and the kernels' quotients want finite, normal divisors.
+  q.ds_max = std::clamp(r.ds_max, 1e-290, 1e290);
   q.min_transmit = r.min_transmit;
   unsigned long long *counter = nullptr;
   if (bhh_work_counter(&counter) != 0) return -1;

@@ -31,7 +31,8 @@ extern "C" {
 /* Device grid of float4 (n_e [cm^-3], Theta_e, |B| [G], 0), index
  * (i_r * n_theta + i_theta) * n_phi + i_phi. Nodes: r_i = r_min (r_max /
  * r_min)^(i / (n_r - 1)); theta_j = (j + 1/2) pi / n_theta; phi_k = 2 pi k /
- * n_phi (periodic). Trilinear interpolation; no emission outside [r_min, r_max]. */
+ * n_phi (periodic). Trilinear interpolation; no emission outside [r_min, r_max].
+ * At least 2 nodes in r and theta and 1 in phi (bh_kerr_trace_rt: else -1). */
 typedef struct BH_GrmhdGrid {
     const void *cells;
     int32_t n_r, n_theta, n_phi, reserved;
