@@ -629,8 +629,10 @@ BHM_HD double integrate_f(const RadialF& q, double v0, double v1, double hmax) {
 }
 
 // Radial set-up. C = K of the tracer (q_R + (lambda - a)^2); a2_alam = a^2 - a lambda.
+// x_obs, x_hor, x_esc: 1 / r of the observer, the horizon cut and the escape
+// radius from the host, where the reciprocal of an infinite radius is 0.
 BHM_HD Radial radial_motion(double a2, double a2_alam, double C, double r_obs, double r_plus, double r_hor,
-                            double r_esc) {
+                            double x_obs, double x_hor, double x_esc) {
   Radial q{};
   q.p2 = 2.0 * a2_alam - C;
   q.p1 = 2.0 * C;
@@ -669,12 +671,12 @@ BHM_HD Radial radial_motion(double a2, double a2_alam, double C, double r_obs, d
     q.q2 = -b2;
     q.q1 = -b1;
     q.q0 = -b0;
-    q.v_obs = -qsqrt(q.x_tp - qdiv(1.0, r_obs));
-    q.v_end = qsqrt(q.x_tp - qdiv(1.0, r_esc));
+    q.v_obs = -qsqrt(q.x_tp - x_obs);
+    q.v_end = qsqrt(q.x_tp - x_esc);
   } else {
     q.kind = 0;
-    q.v_obs = qdiv(1.0, r_obs);
-    q.v_end = qdiv(1.0, r_hor);
+    q.v_obs = x_obs;
+    q.v_end = x_hor;
   }
   return q;
 }
@@ -776,7 +778,7 @@ BHM_HD void crossing_loop(const Radial& q, const Polar& th, double r_in, double 
                           int max_hits, double hmax, Crossings& c) {
   const Quad<FAST, KIND, PHI> Q{q, to_f32(q)};
   double seed_v[2] = {NAN, NAN};
-  if (r_seed > 0.0) {
+  if (r_seed > 0.0 && r_seed < INFINITY) {
     if (KIND == 1) {
       const double s = qsqrt(fmax(0.0, q.x_tp - qdiv(1.0, r_seed)));
       seed_v[0] = -s;

@@ -101,7 +101,7 @@ __global__ void __launch_bounds__(128, FAST ? BH_REFINE_MIN_CTAS : 2) k_surrogat
     if (!(conf >= min_conf)) {
       reason = 1;
     } else {
-      bhmino::Radial q = bhmino::radial_motion(p.a2, p.a2 - a * lam, C, p.r_obs, p.r_plus, p.r_hor, p.r_esc);
+      bhmino::Radial q = bhmino::radial_motion(p.a2, p.a2 - a * lam, C, p.r_obs, p.r_plus, p.r_hor, p.inv_r_obs, p.inv_r_hor, p.inv_r_esc);
       if (PHI) bhmino::set_azimuth(q, a, lam);
       const double d = bhmino::critical_distance(q.r_min, q.R_min, a, lam, p.form == 1, p.sin_o, p.cos_o, alpha,
                                                  beta);
@@ -232,7 +232,7 @@ __global__ void __launch_bounds__(BH_REFINE_THREADS, 1)
     if (!(conf >= min_conf)) {
       reason = 1;
     } else {
-      q = bhmino::radial_motion(p.a2, p.a2 - a * lam, C, p.r_obs, p.r_plus, p.r_hor, p.r_esc);
+      q = bhmino::radial_motion(p.a2, p.a2 - a * lam, C, p.r_obs, p.r_plus, p.r_hor, p.inv_r_obs, p.inv_r_hor, p.inv_r_esc);
       if (PHI) bhmino::set_azimuth(q, a, lam);
       const double d = bhmino::critical_distance(q.r_min, q.R_min, a, lam, p.form == 1, p.sin_o, p.cos_o, alpha,
                                                  beta);
