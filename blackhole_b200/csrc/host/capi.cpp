@@ -166,8 +166,11 @@ static BhkImageParams make_params(const BH_KerrScene *s) {
   p.dbeta = (s->beta_max - s->beta_min) / double(s->height);
   p.step_coeff = s->step_coeff;
   p.step_rcap = s->step_rcap;
-  p.rtol = s->rtol;
-  p.atol = s->atol;
+  // The error's divisors, atol + rtol |y|, stay finite and normal (the kernels'
+  // quotients want that): beyond these bounds every error is as good as 0, or atol
+  // decides where a component is exactly 0 only. FP32 copies are unchanged (inf, 0).
+  p.rtol = std::min(s->rtol, 1e100);
+  p.atol = std::clamp(s->atol, 1e-290, 1e300);
   p.nt_isco = k.nt_isco;
   p.nt_flux_peak = k.nt_flux_peak;
   p.n_pix = int64_t(s->width) * s->height;
