@@ -286,7 +286,7 @@ int bhk_legacy_disk_texture(double a, double r_isco, double r_out, double nt_flu
 typedef struct BhkPostTaps {
   float w[124];
 } BhkPostTaps;
-int64_t bhk_post_scratch_floats(int w, int h);
+int64_t bhk_post_scratch_floats(int w, int h, float strength);
 int bhk_post_process(float *fb, int w, int h, const BhkPostTaps *taps, float threshold, float strength,
                      float exposure, float *scratch, void *stream);
 

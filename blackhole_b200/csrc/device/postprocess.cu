@@ -78,9 +78,16 @@ constexpr int kColsH = kColsY + 2 * kHalo;
 constexpr int kColsThreads = kColsX / 2 * (kColsY / kRun);
 constexpr int kColsBuf = kColsH * kColsX;
 
-// Floats between rows of a plane: whole tiles of columns, so that every row
-// starts on 256 bytes and the last tile reads within the plane.
-__host__ __device__ constexpr int plane_pitch(int w) { return (w + 63) / 64 * 64; }
+// Floats between rows of a plane: whole tiles of 64 columns, so that every row
+// starts on 256 bytes, where 15 such planes take no more than 16 floats a
+// pixel; narrower images the widest padding of 32, 16, 8 or 4 floats (a 16-byte
+// copy) that does, and 4 where none does (some below 42 columns). At 64 for all, a
+// column of 50 million rows would take 192 GB.
+constexpr int plane_pitch(int w) {
+  int pad = 64;
+  while (pad > 4 && 15ll * ((w + (pad - 1ll)) / pad * pad) > 16ll * w) pad /= 2;
+  return (w + pad - 1) / pad * pad;
+}
 constexpr int kBase = 12;  // planes kBase + c: the framebuffer's channels, then the composite's
 
 // Scale index and offset of the normalized taps (2r + 1 each) of half-width R.
@@ -125,11 +132,10 @@ __device__ __forceinline__ void blur_run(const float2 *src, int stride, const fl
 }
 
 __global__ void __launch_bounds__(kRowsThreads, 5) k_post_rows(const __grid_constant__ Taps2 taps,
-                                                               const float4 *__restrict__ fb, int w, int h,
+                                                               const float4 *__restrict__ fb, int w, int h, int pitch,
                                                                float threshold, float *__restrict__ planes) {
   __shared__ float2 sm[3 * kRowPairs * kRowsPitch];  // bright-pass
   const int x0 = blockIdx.x * kRowsX, y0 = (blockIdx.y + kMaxY * blockIdx.z) * kRowsY;
-  const int pitch = plane_pitch(w);
   const int64_t plane = (int64_t)h * pitch;
   constexpr int kPairs = kRowPairs * kRowsW, kInFlight = 3;  // 6 pixels a thread
 #pragma unroll 1
@@ -172,21 +178,17 @@ __global__ void __launch_bounds__(kRowsThreads, 5) k_post_rows(const __grid_cons
   const int y = y0 + 2 * rp, x = x0 + run * kRun;
   const float2 *src = sm + (c * kRowPairs + rp) * kRowsPitch + kHalo + run * kRun;
   float *dst = planes + c * plane + (int64_t)y * pitch + x;
-  const bool top = x < pitch && y < h, low = x < pitch && y + 1 < h;
+  const bool left = x < pitch, right = x + 4 < pitch, top = y < h, low = y + 1 < h;
   auto scale = [&](auto rtag) {
     constexpr int R = decltype(rtag)::value, si = scale_of(R);
     float2 acc[kRun] = {};
     asm volatile("" ::: "memory");  // one scale's window at a time in registers
     blur_run<R>(src - R, 1, taps.w + tap_off(R), acc);
     float4 *out = reinterpret_cast<float4 *>(dst + 3 * si * plane);
-    if (top) {
-      out[0] = make_float4(acc[0].x, acc[1].x, acc[2].x, acc[3].x);
-      out[1] = make_float4(acc[4].x, acc[5].x, acc[6].x, acc[7].x);
-    }
-    if (low) {
-      out[pitch / 4] = make_float4(acc[0].y, acc[1].y, acc[2].y, acc[3].y);
-      out[pitch / 4 + 1] = make_float4(acc[4].y, acc[5].y, acc[6].y, acc[7].y);
-    }
+    if (left && top) out[0] = make_float4(acc[0].x, acc[1].x, acc[2].x, acc[3].x);
+    if (right && top) out[1] = make_float4(acc[4].x, acc[5].x, acc[6].x, acc[7].x);
+    if (left && low) out[pitch / 4] = make_float4(acc[0].y, acc[1].y, acc[2].y, acc[3].y);
+    if (right && low) out[pitch / 4 + 1] = make_float4(acc[4].y, acc[5].y, acc[6].y, acc[7].y);
   };
   scale(std::integral_constant<int, 4>{});
   scale(std::integral_constant<int, 8>{});
@@ -195,13 +197,15 @@ __global__ void __launch_bounds__(kRowsThreads, 5) k_post_rows(const __grid_cons
 }
 
 // Rows y0 - R .. y0 + kColsY - 1 + R (clamped) of one channel's plane of scale
-// si, kColsX columns from x0, into a shared buffer, by cp.async.
+// si, kColsX columns from x0 (those inside the plane), into a shared buffer, by
+// cp.async.
 __device__ __forceinline__ void cols_fetch(float *buf, const float *__restrict__ planes, int c, int si, int x0,
                                            int y0, int pitch, int h) {
   const int R = 4 << si;
   constexpr int kVecs = kColsX / 4;
   const float *src = planes + (int64_t)(si * 3 + c) * h * pitch + x0 + 4 * (threadIdx.x % kVecs);
   float *dst = buf + 4 * (threadIdx.x % kVecs);
+  if (x0 + 4 * (int)(threadIdx.x % kVecs) >= pitch) return;
   for (int row = threadIdx.x / kVecs; row < kColsY + 2 * R; row += kColsThreads / kVecs) {
     const int y = min(max(y0 - R + row, 0), h - 1);
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(
@@ -212,12 +216,11 @@ __device__ __forceinline__ void cols_fetch(float *buf, const float *__restrict__
 }
 
 __global__ void __launch_bounds__(kColsThreads, 7) k_post_cols(const __grid_constant__ Taps2 taps,
-                                                               float *__restrict__ planes, int w, int h,
+                                                               float *__restrict__ planes, int h, int pitch,
                                                                float strength) {
   extern __shared__ float cols_sm[];  // two buffers of [kColsH][kColsX]: scale si in buffer si % 2
   const int x0 = blockIdx.x * kColsX, y0 = (blockIdx.y + kMaxY * (blockIdx.z / 3)) * kColsY, c = blockIdx.z % 3;
   const int lane = threadIdx.x % (kColsX / 2), grp = threadIdx.x / (kColsX / 2);
-  const int pitch = plane_pitch(w);
   auto fetch = [&](int si) {
     if (si < 4) cols_fetch(cols_sm + (si % 2) * kColsBuf, planes, c, si, x0, y0, pitch, h);
     asm volatile("cp.async.commit_group;\n" ::: "memory");
@@ -241,6 +244,7 @@ __global__ void __launch_bounds__(kColsThreads, 7) k_post_cols(const __grid_cons
   scale(std::integral_constant<int, 8>{});
   scale(std::integral_constant<int, 16>{});
   scale(std::integral_constant<int, 32>{});
+  if (x0 + 2 * lane >= pitch) return;
   float *base = planes + (int64_t)(kBase + c) * h * pitch + x0 + 2 * lane;
 #pragma unroll
   for (int j = 0; j < kRun; ++j) {
@@ -270,9 +274,8 @@ __device__ __forceinline__ float tone_channel(float x, float exposure, float vig
 // PLANAR: the composite is in three planes, otherwise a copy of the framebuffer.
 constexpr int kToneWave = 148 * 2048;
 template <bool PLANAR, int ROWS>
-__global__ void __launch_bounds__(256) k_post_tone(const float *__restrict__ src, int w, int h, float exposure,
+__global__ void __launch_bounds__(256) k_post_tone(const float *__restrict__ src, int w, int h, int pitch, float exposure,
                                                    float4 *__restrict__ fb) {
-  const int pitch = PLANAR ? plane_pitch(w) : w;
   const int64_t plane = (int64_t)h * pitch;
   // red and blue of one pixel
   auto red_blue = [&](int64_t i) {
@@ -281,15 +284,15 @@ __global__ void __launch_bounds__(256) k_post_tone(const float *__restrict__ src
     return make_float2(v.x, v.z);
   };
   const int px = blockIdx.x * 64 + (threadIdx.x & 63);
-  const int y0 = ((blockIdx.y + kMaxY * blockIdx.z) * 4 + (threadIdx.x >> 6)) * ROWS;
+  const unsigned y0 = ((blockIdx.y + kMaxY * blockIdx.z) * 4 + (threadIdx.x >> 6)) * ROWS;  // passes 2^31 by a slice
   if (px >= w) return;
   const float u = __fdiv_rn((float)px, (float)w);
   const int rx = min(max((int)__fmul_rn(u, (float)w), 0), w - 1);
   const float du = u - 0.5f;
 #pragma unroll
   for (int k = 0; k < ROWS; ++k) {
-    const int py = y0 + k;
-    if (py >= h) break;
+    if (y0 + k >= (unsigned)h) break;
+    const int py = (int)(y0 + k);
     const int64_t i = (int64_t)py * w + px;
     const float v = __fdiv_rn((float)py, (float)h);
     const int ry = min(max((int)__fmul_rn(v, (float)h), 0), h - 1);
@@ -306,8 +309,13 @@ __global__ void __launch_bounds__(256) k_post_tone(const float *__restrict__ src
 
 }  // namespace
 
-// 15 padded planes, or a copy of the framebuffer where the bloom is off.
-extern "C" int64_t bhk_post_scratch_floats(int w, int h) { return (int64_t)(kBase + 3) * plane_pitch(w) * h; }
+// 15 padded planes, or a copy of the framebuffer where the bloom is off; -1: the
+// image is too wide for the blurs' 32-bit columns.
+extern "C" int64_t bhk_post_scratch_floats(int w, int h, float strength) {
+  if (strength == 0.0f) return (int64_t)4 * w * h;
+  if (w > INT32_MAX - 2 * kRowsX) return -1;
+  return (int64_t)(kBase + 3) * plane_pitch(w) * h;
+}
 
 extern "C" int bhk_post_process(float *fb, int w, int h, const BhkPostTaps *taps, float threshold, float strength,
                                 float exposure, float *scratch, void *stream) {
@@ -318,12 +326,14 @@ extern "C" int bhk_post_process(float *fb, int w, int h, const BhkPostTaps *taps
     const unsigned rows = ((unsigned)h + ty - 1) / ty;
     return dim3(((unsigned)w + tx - 1) / tx, std::min(rows, kMaxY), (rows + kMaxY - 1) / kMaxY * channels);
   };
+  const int pitch = strength != 0.0f ? plane_pitch(w) : 0;
   auto tone = [&](auto planar, const float *src) {
     constexpr bool kPlanar = decltype(planar)::value;
+    const int row = kPlanar ? pitch : w;
     if ((int64_t)w * h <= kToneWave)
-      k_post_tone<kPlanar, 1><<<tiles(64, 4, 1), 256, 0, st>>>(src, w, h, exposure, f4);
+      k_post_tone<kPlanar, 1><<<tiles(64, 4, 1), 256, 0, st>>>(src, w, h, row, exposure, f4);
     else
-      k_post_tone<kPlanar, 4><<<tiles(64, 16, 1), 256, 0, st>>>(src, w, h, exposure, f4);
+      k_post_tone<kPlanar, 4><<<tiles(64, 16, 1), 256, 0, st>>>(src, w, h, row, exposure, f4);
   };
   if (strength != 0.0f) {
     constexpr int smem = sizeof(float) * 2 * kColsBuf;
@@ -331,9 +341,9 @@ extern "C" int bhk_post_process(float *fb, int w, int h, const BhkPostTaps *taps
       return -1;
     Taps2 t2;
     for (int i = 0; i < 124; ++i) t2.w[i] = make_float2(taps->w[i], taps->w[i]);
-    k_post_rows<<<tiles(kRowsX, kRowsY, 1), kRowsThreads, 0, st>>>(t2, f4, w, h, threshold, scratch);
-    k_post_cols<<<tiles(kColsX, kColsY, 3), kColsThreads, smem, st>>>(t2, scratch, w, h, strength);
-    tone(std::true_type{}, scratch + (int64_t)kBase * plane_pitch(w) * h);
+    k_post_rows<<<tiles(kRowsX, kRowsY, 1), kRowsThreads, 0, st>>>(t2, f4, w, h, pitch, threshold, scratch);
+    k_post_cols<<<tiles(kColsX, kColsY, 3), kColsThreads, smem, st>>>(t2, scratch, h, pitch, strength);
+    tone(std::true_type{}, scratch + (int64_t)kBase * pitch * h);
   } else {
     if (cudaMemcpyAsync(scratch, fb, sizeof(float4) * w * h, cudaMemcpyDeviceToDevice, st) != cudaSuccess) return -1;
     tone(std::false_type{}, scratch);

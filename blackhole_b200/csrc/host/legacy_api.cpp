@@ -516,7 +516,8 @@ int postprocess_locked(float *fb, int w, int h, float threshold, float strength,
   if ((int64_t)w * h > (int64_t(1) << 31)) return fail_msg("postprocess: image exceeds 2^31 pixels");
   Scratch *sc = nullptr;
   if (scratch(0, &sc) != 0) return -1;
-  const int64_t need = bhk_post_scratch_floats(w, h);
+  const int64_t need = bhk_post_scratch_floats(w, h, strength);
+  if (need < 0) return fail_msg("postprocess: bloom of an image %d pixels wide", w);
   if (need > sc->post_cap) {
     if (sc->post) cudaFree(sc->post);
     sc->post = nullptr;
