@@ -4,11 +4,12 @@
 //   k_kerr_step_mino   <- physics::kerrStepMino         (src/physics/kerr.cpp:99-134)
 //   k_kerr_trace_rays  <- physics::KerrRaytracer::trace (src/physics/raytracer.h:324-378)
 //
-// First-order Mino-time form with sign flips, CGS units, exactly the
-// reference's expression order; compiled with -fmad=false so every FP64
-// operation rounds once as on the CPU. The only device/host difference left
-// is CUDA's sin/cos against glibc's (at most an ulp or two). One thread per
-// state; inputs and outputs are structure-of-arrays.
+// First-order Mino-time form with sign flips, CGS units, the reference's
+// expression order; compiled with -fmad=false so every FP64 operation rounds
+// once as on the CPU. What differs from the host is sin^2 and cos^2, by an ulp
+// or two: the potentials take them from CUDA's sincos, the steps and the trace's
+// sign test from sin2_cos2 below. One thread per state; inputs and outputs are
+// structure-of-arrays.
 #include <cuda_runtime.h>
 
 #include "ieee_fp64.cuh"
@@ -82,10 +83,11 @@ __device__ __forceinline__ void sin2_cos2(double x, double &s2, double &c2) {
   c2 = odd ? ss : cc;
 }
 
-// kerrMinoDerivatives (kerr.cpp:40-66). The reference recomputes the full
-// potentials (including the unused derivatives) and sin(theta) twice; the
-// values that feed the result are identical here.
-__device__ __forceinline__ Dv mino_derivs(const St &s, double mass, double a, const Cs &c) {
+// What a step's derivatives and the trace's sign test need of a state.
+struct Stage {
+  double rr, sin2, delta, aFactor, rPot, thetaPot;
+};
+__device__ __forceinline__ Stage stage_at(const St &s, double mass, double a, const Cs &c) {
   const double mGeom = kG * mass / kC2;
   const double r = s.r;
   const double rr = r * r;
@@ -105,14 +107,23 @@ __device__ __forceinline__ Dv mino_derivs(const St &s, double mass, double a, co
   const double lzMinusAe = c.lz - (a * c.e);
   const double rPotRaw = (aFactor * aFactor) - (delta * (c.q + (lzMinusAe * lzMinusAe)));
   const double thetaPotRaw = c.q + (aa * c.e * c.e * cos2) - (c.lz * c.lz / sin2);
-  const double rPot = mx(rPotRaw, 0.0);
-  const double thetaPot = mx(thetaPotRaw, 0.0);
-  const double deltaSafe = mx(delta, 1e-12);
+  return Stage{rr, sin2, delta, aFactor, rPotRaw, thetaPotRaw};
+}
+
+// kerrMinoDerivatives (kerr.cpp:40-66). The reference recomputes the full
+// potentials (including the unused derivatives) and sin(theta) twice; the
+// values that feed the result are identical here.
+__device__ __forceinline__ Dv mino_derivs(const St &s, double mass, double a, const Cs &c) {
+  const Stage w = stage_at(s, mass, a, c);
+  const double aa = a * a;
+  const double rPot = mx(w.rPot, 0.0);
+  const double thetaPot = mx(w.thetaPot, 0.0);
+  const double deltaSafe = mx(w.delta, 1e-12);
   Dv d;
   d.dr = s.signR * sqrt(rPot);
   d.dtheta = s.signTheta * sqrt(thetaPot);
-  d.dphi = (c.lz / sin2) - (a * c.e) + (a * aFactor / deltaSafe);
-  d.dt = (((rr + aa) * aFactor) / deltaSafe) + (a * (c.lz - (a * c.e * sin2)));
+  d.dphi = (c.lz / w.sin2) - (a * c.e) + (a * w.aFactor / deltaSafe);
+  d.dt = (((w.rr + aa) * w.aFactor) / deltaSafe) + (a * (c.lz - (a * c.e * w.sin2)));
   return d;
 }
 
@@ -150,7 +161,7 @@ __device__ __noinline__ St step_mino_any(const St &state, double mass, double a,
 // ---- the same step with the branch-free quotients and roots (ieee_fp64.cuh) -------
 //
 // The same operations on the same values in the same order, so the same bits
-// (both take sin^2 and cos^2 from sin2_cos2):
+// (both take sin^2 and cos^2 from sin2_cos2, for the sign test too):
 //   * the quotients by sin^2 share one reciprocal, those by Delta another;
 //   * products with 2 are exact, so fma(2, x, y) rounds as y + 2 x;
 //   * the first stage's potentials are those the trace loop tests for sign
@@ -339,10 +350,10 @@ __global__ void k_kerr_trace_rays(int64_t n, BhkStateSoA init, BhkConstsSoA c, d
         next = step_mino_fast<false>(next, w, g, step, ok);
       }
       if (!ok) {
-        const Pot p = potentials(state.r, state.theta, mass, a, cs);
+        const Stage w = stage_at(state, mass, a, cs);
         next = state;
-        if (p.rPot < 0.0) next.signR = -next.signR;
-        if (p.thetaPot < 0.0) next.signTheta = -next.signTheta;
+        if (w.rPot < 0.0) next.signR = -next.signR;
+        if (w.thetaPot < 0.0) next.signTheta = -next.signTheta;
         next = step_mino_any(next, mass, a, cs, step);
       }
       state = next;
