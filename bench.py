@@ -906,6 +906,15 @@ def cpu_reference(workload: str, budget_s: float, seed: int = 7):
                       f"{el:.1f} s wall on {threads} threads (oracle/_ref: reference kerrPotentials)"}
 
 
+def cpu_baseline(rt_inputs, workload: str, budget_s: float):
+    """The CPU figure beside the GPU's, or None (with a word on stderr) where its library is not built."""
+    try:
+        return cpu_reference_rt(rt_inputs, budget_s) if rt_inputs is not None else cpu_reference(workload, budget_s)
+    except FileNotFoundError as e:
+        print(f"bench.py: no CPU baseline: {e}", file=sys.stderr)
+        return None
+
+
 def reference_gpu_kernel() -> dict:
     """The reference's own FP32 render kernel (geodesicTraceFp32, variant 0 of
     its bh_launch_geodesic_kernel; oracle/_ref/libbh_ref_render.so, compiled
@@ -1013,7 +1022,11 @@ def main():
     if args.impl == "reference":
         if rank != 0:
             return
-        cb = cpu_reference(args.workload, args.cpu_budget)
+        try:
+            cb = cpu_reference(args.workload, args.cpu_budget)
+        except FileNotFoundError as e:
+            print(json.dumps({"impl": "reference", "unavailable": str(e)}))
+            return
         line = {"metric": METRIC, "value": cb["value"], "unit": UNIT, "n_gpus": args.gpus, "steps": args.steps,
                 "warmup": args.warmup, "ms_per_step": None, "higher_is_better": True, "scaling": "weak",
                 "vs_baseline": None, "dtype": "f64", "data": "synthetic", "config": config, "impl": "reference",
@@ -1051,8 +1064,7 @@ def main():
             res["extra"]["legacy_render"] = lr
         cb = None
         if world == 1 and args.cpu_budget > 0:
-            cb = cpu_reference_rt(res["cpu_inputs"], args.cpu_budget) if wl.get("rt") else \
-                cpu_reference(args.workload, args.cpu_budget)
+            cb = cpu_baseline(res["cpu_inputs"] if wl.get("rt") else None, args.workload, args.cpu_budget)
         line = {"metric": METRIC, "value": res["value"], "unit": UNIT, "n_gpus": world, "steps": args.steps,
                 "warmup": args.warmup, "ms_per_step": res["ms_per_step"], "higher_is_better": True,
                 "scaling": "weak", "vs_baseline": None,
