@@ -33,18 +33,6 @@ __device__ __forceinline__ void store_f32x16(float* dst, const float (&h)[16]) {
   for (int q = 0; q < 4; ++q) p[q] = make_float4(h[4 * q], h[4 * q + 1], h[4 * q + 2], h[4 * q + 3]);
 }
 
-// ---- epilogues: (row, first column, 16 accumulator values, split index) ---
-
-struct EpiF32 {
-  float* C;
-  int64_t M;
-  int N;
-  __device__ void operator()(int64_t row, int col, const float (&v)[16], int split) const {
-    if (row >= M) return;
-    store_f32x16(C + ((int64_t)split * M + row) * N + col, v);
-  }
-};
-
 __device__ __forceinline__ void tmem_ld16(uint32_t taddr, float (&v)[16]) {
   uint32_t r[16];
   asm volatile(
@@ -60,11 +48,11 @@ __device__ __forceinline__ void tmem_ld16(uint32_t taddr, float (&v)[16]) {
   for (int i = 0; i < 16; ++i) v[i] = __uint_as_float(r[i]);
 }
 
-// One 128 x BN output tile per CTA; blockIdx = (M tile, N tile, K split).
-template <int BN, class Epi>
+// One 128 x BN output tile per CTA; blockIdx = (M tile, N tile).
+template <int BN>
 __global__ void __launch_bounds__(128, 1)
   k_gemm_bf16(const __grid_constant__ CUtensorMap ta, const __grid_constant__ CUtensorMap tb, int K,
-        int kchunks_per_split, Epi epi, int* err, uint64_t wait_ns) {
+        float* __restrict__ C, int64_t M, int N, int* err, uint64_t wait_ns) {
   using Cfg = GemmCfg<BN>;
   extern __shared__ uint8_t smem_raw[];
   const uint32_t raw = umma::smem_u32(smem_raw);
@@ -82,9 +70,7 @@ __global__ void __launch_bounds__(128, 1)
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int m0 = blockIdx.x * kBM, n0 = blockIdx.y * BN;
-  const int total = (K + kBK - 1) / kBK;
-  const int c0 = blockIdx.z * kchunks_per_split;
-  const int nch = max(0, min(total, c0 + kchunks_per_split) - c0);
+  const int nch = (K + kBK - 1) / kBK;
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < kStages; ++s) {
@@ -114,7 +100,7 @@ __global__ void __launch_bounds__(128, 1)
         break;
       }
       umma::mbar_arrive_expect_tx(full(s), Cfg::kStage);
-      const int kx = (c0 + i) * kBK;
+      const int kx = i * kBK;
       umma::tma_load_2d(sA(s), &ta, full(s), kx, m0);
       umma::tma_load_2d(sB(s), &tb, full(s), kx, n0);
       issued = i + 1;
@@ -154,11 +140,11 @@ __global__ void __launch_bounds__(128, 1)
   for (int j = 0; j < BN / 16; ++j) {
     float v[16];
     tmem_ld16(taddr + 16u * j, v);
-    if (!ok || nch == 0) {
+    if (!ok) {
 #pragma unroll
       for (int i = 0; i < 16; ++i) v[i] = 0.0f;
     }
-    epi(row, n0 + 16 * j, v, (int)blockIdx.z);
+    if (row < M) store_f32x16(C + row * N + n0 + 16 * j, v);
   }
   umma::tc_fence_before();
   __syncthreads();
@@ -593,8 +579,8 @@ __global__ void k_grid_inputs(double spin, double ct, double a0, double da, doub
 
 // ---- host side: tensor maps and launchers -----------------------------------
 
-template <int BN, class Epi>
-int launch_tile(const BhsGemm* g, const Epi& epi, int* err, cudaStream_t st) {
+template <int BN>
+int launch_bn(const BhsGemm* g, int* err, cudaStream_t st) {
   using Cfg = GemmCfg<BN>;
   CUtensorMap ta, tb;
   if (!make_map(&ta, g->A, g->M, g->K, g->lda, kBM) || !make_map(&tb, g->B, g->N, g->K, g->ldb, BN)) {
@@ -603,22 +589,15 @@ int launch_tile(const BhsGemm* g, const Epi& epi, int* err, cudaStream_t st) {
   }
   static bool attr_set = false;  // per template instance
   if (!attr_set) {
-    if (cudaFuncSetAttribute(k_gemm_bf16<BN, Epi>, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::kSmem) !=
+    if (cudaFuncSetAttribute(k_gemm_bf16<BN>, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::kSmem) !=
       cudaSuccess)
       return -1;
     attr_set = true;
   }
-  const int total = (g->K + kBK - 1) / kBK;
-  const int kcps = g->kchunks_per_split > 0 ? g->kchunks_per_split : total;
-  const int splits = (total + kcps - 1) / kcps;
-  const dim3 grid((unsigned)((g->M + kBM - 1) / kBM), (unsigned)(g->N / BN), (unsigned)splits);
-  k_gemm_bf16<BN, Epi><<<grid, 128, Cfg::kSmem, st>>>(ta, tb, g->K, kcps, epi, err, g->wait_ns);
+  const dim3 grid((unsigned)((g->M + kBM - 1) / kBM), (unsigned)(g->N / BN));
+  k_gemm_bf16<BN><<<grid, 128, Cfg::kSmem, st>>>(ta, tb, g->K, static_cast<float*>(g->out), g->M, g->N, err,
+                                                 g->wait_ns);
   return cudaGetLastError() == cudaSuccess ? 0 : -1;
-}
-
-template <int BN>
-int launch_bn(const BhsGemm* g, int* err, cudaStream_t st) {
-  return launch_tile<BN>(g, EpiF32{static_cast<float*>(g->out), g->M, g->N}, err, st);
 }
 
 int blocks_for(int64_t n, int threads) { return (int)((n + threads - 1) / threads); }

@@ -46,15 +46,13 @@ static inline int64_t bhs_bias_offset(int l) {
 }
 static inline int64_t bhs_param_count(void) { return bhs_weight_offset(BHS_LAYERS); }
 
-// BF16 GEMM C = A * B^T (A [M][K], B [N][K], both K-major), C FP32
-// [split][M][N]: split-K partial sums.
+// BF16 GEMM C = A * B^T (A [M][K], B [N][K], both K-major), C FP32 [M][N].
 typedef struct BhsGemm {
   const void* A;  // BF16 [M][lda]
   const void* B;  // BF16 [N][ldb]
   int64_t M;
   int N, K;
   int lda, ldb;
-  int kchunks_per_split;  // 64-wide K chunks per split (0 = all)
   void* out;
   uint64_t wait_ns;       // limit of each wait on another warp (>= 1)
 } BhsGemm;
