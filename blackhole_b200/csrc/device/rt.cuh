@@ -179,7 +179,8 @@ __device__ __forceinline__ void synchrotron(const BhkRtParams &q, double n, doub
   const double nu_s = 1.5 * nu_b * theta_e * theta_e;
   // an infinite Theta_e or |B| (div_rn wants finite operands) is the table's lower end, as x = 0 is
   const double lx = nu_s < INFINITY ? log(bhk::div_rn(nu_e, nu_s)) : -INFINITY;
-  if (lx > q.lx1) return;  // beyond the table: exp(-1.89 x^(1/3)) below any use
+  // beyond the table: exp(-1.89 x^(1/3)) below any use; a quotient past the range is no number
+  if (!(lx <= q.lx1)) return;
   const double lt = log(theta_e);
   double ft = (lt - q.lt0) * q.lt_scale;
   double fx = (lx - q.lx0) * q.lx_scale;
