@@ -272,7 +272,6 @@ __device__ __forceinline__ float tone_channel(float x, float exposure, float vig
 // holds the image and a thread's own chain of powf is the time (100 x 60 with
 // bloom: 44 and 41 us a call).
 // PLANAR: the composite is in three planes, otherwise a copy of the framebuffer.
-constexpr int kToneWave = 148 * 2048;
 template <bool PLANAR, int ROWS>
 __global__ void __launch_bounds__(256) k_post_tone(const float *__restrict__ src, int w, int h, int pitch, float exposure,
                                                    float4 *__restrict__ fb) {
@@ -326,11 +325,17 @@ extern "C" int bhk_post_process(float *fb, int w, int h, const BhkPostTaps *taps
     const unsigned rows = ((unsigned)h + ty - 1) / ty;
     return dim3(((unsigned)w + tx - 1) / tx, std::min(rows, kMaxY), (rows + kMaxY - 1) / kMaxY * channels);
   };
+  int dev = 0, sms = 0, per_sm = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess ||
+      cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess ||
+      cudaDeviceGetAttribute(&per_sm, cudaDevAttrMaxThreadsPerMultiProcessor, dev) != cudaSuccess)
+    return -1;
+  const int64_t wave = (int64_t)sms * per_sm;
   const int pitch = strength != 0.0f ? plane_pitch(w) : 0;
   auto tone = [&](auto planar, const float *src) {
     constexpr bool kPlanar = decltype(planar)::value;
     const int row = kPlanar ? pitch : w;
-    if ((int64_t)w * h <= kToneWave)
+    if ((int64_t)w * h <= wave)
       k_post_tone<kPlanar, 1><<<tiles(64, 4, 1), 256, 0, st>>>(src, w, h, row, exposure, f4);
     else
       k_post_tone<kPlanar, 4><<<tiles(64, 16, 1), 256, 0, st>>>(src, w, h, row, exposure, f4);
