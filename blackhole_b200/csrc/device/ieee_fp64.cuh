@@ -72,7 +72,8 @@ __device__ __forceinline__ double sqrt_rn(double x) {
 }
 
 // The FP32 root, the same way; 0 is its own root, arguments below 1e-30 are
-// scaled by an even power of two. All 2^31 floats checked against sqrtf.
+// scaled by an even power of two. tests/test_gpu_exact_ops.py: equal to sqrtf at all
+// 2^31 floats.
 __device__ __forceinline__ float sqrt_rn_f(float x) {
   const bool tiny = x < 1e-30f;
   const float v = tiny ? x * 0x1p100f : x;

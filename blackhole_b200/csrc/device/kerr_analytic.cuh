@@ -211,7 +211,7 @@ BHA_CALL void sncndn(double u, double m1, double &sn, double &cn, double &dn) {
 }
 
 // sn, cn, dn(u | m) for m = 1 - m1 < 0 (m1 > 1): Abramowitz & Stegun 16.10.2-4,
-// sn(u | m) = sd(u qsqrt(m1) | mu) / qsqrt(m1), cn = cd, dn = nd, mu = 1 - 1 / m1.
+// sn(u | m) = sd(u sqrt(m1) | mu) / sqrt(m1), cn = cd, dn = nd, mu = 1 - 1 / m1.
 BHM_HD void sncndn_neg(double u, double m1, double &sn, double &cn, double &dn) {
   const double r = qsqrt(m1);
   double s, c, d;
@@ -569,7 +569,7 @@ BHA_PCALL void j_poles(const RadSol &q, double r_plus, double r_minus, JPole &jp
   if (q.type != kP2) ellip_q2_sc(jp.par, jm.par, q.a0.s, q.a0.c, q.m1, jp.t0, jm.t0);
 }
 
-// The integrand of Q: sin^2 / ((1 - n sin^2) qsqrt(cos^2 + m1 sin^2)).
+// The integrand of Q: sin^2 / ((1 - n sin^2) sqrt(cos^2 + m1 sin^2)).
 BHM_HD double q_integrand(double n, double m1, double ph) {
   const double s = sin(ph), c = cos(ph), s2 = s * s;
   return qdiv(s2, (1.0 - n * s2) * qsqrt(c * c + m1 * s2));
@@ -617,16 +617,16 @@ BHA_PCALL void j_eval_escape(const RadSol &q, JPole &jp, JPole &jm, double &vp, 
 
 // ---- polar motion -------------------------------------------------------------------
 //
-// u = qsqrt(z+) sin chi, Phi(chi) = F(chi | -mm / w) / qsqrt(w) the Mino time
+// u = sqrt(z+) sin chi, Phi(chi) = F(chi | -mm / w) / sqrt(w) the Mino time
 // since chi = 0; the ray starts at Phi = phi_start and crosses the equator at
 // chi = j pi, i.e. at tau = j period - phi_start.
 
 struct PolSol {
   bool crosses;
-  double zp, w, mm, sz;  // U = (z+ - u^2)(a^2 u^2 + w), mm = a^2 z+, sz = qsqrt(z+)
+  double zp, w, mm, sz;  // U = (z+ - u^2)(a^2 u^2 + w), mm = a^2 z+, sz = sqrt(z+)
   double zc;             // 1 - z+, formed without cancellation
   double m1;             // complementary parameter of -mm / w
-  double sw;             // qsqrt(w)
+  double sw;             // sqrt(w)
   double phi_start;      // Phi at the observer [Mino time]
   double tau1, period;   // first crossing, time between crossings
   double s0, c0;         // chi at the observer: sin, cos (chi0 in (-pi/2, 3 pi/2); cos has the sign of du/dtau)
@@ -670,7 +670,7 @@ BHM_HD void polar_q0(PolSol &t) {
 }
 
 // lambda int_0^tau dtau / (1 - u^2) at an equatorial crossing (chi = j pi,
-// Q(z+; j pi) = 2 j Q(pi/2)): lambda (tau + (z+ / qsqrt(w)) (2 j Q_c - Q(chi0))).
+// Q(z+; j pi) = 2 j Q(pi/2)): lambda (tau + (z+ / sqrt(w)) (2 j Q_c - Q(chi0))).
 // With 1 - z+ == 0 (lambda == 0, or lambda^2 below the smallest double) the
 // integral is its limit lambda -> 0 from the side of lambda's sign: a turn by
 // copysign(pi, lambda) at each pass over the pole (chi = pi/2 + j pi), so

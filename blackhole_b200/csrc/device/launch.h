@@ -60,7 +60,7 @@ typedef struct BhkImageOut {
 typedef struct BhkLaunch {
   int32_t grid;      // CTAs
   int32_t block;     // threads per CTA
-  int32_t refill;    // integration steps between two refills of finished lanes (>= 1)
+  int32_t refill;    // factor on the steps between two looks at a warp's held lanes (frame_source.cuh), >= 1
   int32_t pad;
 } BhkLaunch;
 

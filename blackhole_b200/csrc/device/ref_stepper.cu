@@ -60,10 +60,10 @@ __device__ __forceinline__ Pot potentials(double r, double theta, double mass, d
 
 // sin^2 and cos^2 of |x| < 2^10. The angle less the nearest multiple of pi / 2,
 // which is taken in two parts, as r + rl; Taylor's series on |r| <= pi / 4 to
-// r^17 and r^16, summed in pairs (G. Estrin's scheme); sine and cosine within
-// 0.83 ulp each (2e7 arguments). CUDA's sincos has a branch for large arguments:
-// four calls a step keep its stages in blocks of their own, and the polar motion
-// is the step's longest chain.
+// r^17 and r^16, summed in pairs (G. Estrin's scheme). Sine and cosine were within
+// 0.83 ulp each at 2e7 arguments; tests/test_gpu_ray_angles.py has the step's. CUDA's
+// sincos has a branch for large arguments: four calls a step keep its stages in
+// blocks of their own, and the polar motion is the step's longest chain.
 __device__ __forceinline__ void sin2_cos2(double x, double &s2, double &c2) {
   const double t = fma(x, 0x1.45f306dc9c883p-1, 0x1.8p52);  // 2 / pi
   const bool odd = __double2loint(t) & 1;

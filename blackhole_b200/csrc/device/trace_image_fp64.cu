@@ -1,11 +1,11 @@
 // trace_image_fp64.cu - FP64 image-plane Kerr tracer (sm_100a).
 //
 // One ray per lane in a persistent grid: each warp keeps 32 rays in
-// registers and, whenever rays terminate (horizon, disk, escape, step
-// budget), refills exactly those lanes from a global work counter with one
-// warp-aggregated atomicAdd (ballot + popc), so finished rays never idle a
-// lane while work remains. The integration follows the reference trace loop
-// order (src/physics/raytracer.h:338-365): step budget, horizon test, escape
+// registers; lanes whose rays cross the equator or terminate (horizon, disk,
+// escape, step budget) are held until the warp serves them together
+// (frame_source.cuh), and take new rays from a global work counter with one
+// warp-aggregated atomicAdd (ballot + popc). The integration
+// follows the reference trace loop order (src/physics/raytracer.h:338-365): step budget, horizon test, escape
 // test, step; then the equatorial-crossing test, located inside the step by
 // Hermite interpolation (hermite.cuh) on the bracket of the
 // src/physics/event_detection.h:127-180 pattern.

@@ -328,7 +328,9 @@ typedef struct BH_KerrBatch BH_KerrBatch;
 typedef struct BH_KerrLaunchConfig {
     int32_t block_threads;  /**< 32..128, multiple of 32 */
     int32_t ctas_per_sm;    /**< resident CTAs per SM (<= occupancy limit) */
-    int32_t refill_steps;   /**< integration steps between refills of finished lanes (>= 1) */
+    int32_t refill_steps;   /**< a warp looks at its finished and crossing lanes every refill_steps x 32 (RK4)
+                                 or x 8 (DP45) steps, and serves them once they have waited 64 lane-steps
+                                 in all; 1..64, 0 = 1. Changes time, not results. */
     int32_t reserved;
 } BH_KerrLaunchConfig;
 
