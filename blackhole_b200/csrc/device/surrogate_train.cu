@@ -14,7 +14,7 @@
 // What bounds it (batch 16384, one B200): 23 GFLOP, 14 us of tensor time at
 // the measured rate. One GEMM launch per product (twenty launches, a tile's
 // loads, MMAs and its row-by-row epilogue one after another, every activation
-// and gradient also written transposed) took 298 us; this takes 85: 45 in the
+// and gradient also written transposed) took 300 us; this takes 84: 45 in the
 // pass, 22 in the weight gradients, 8 in the collection, the rest between
 // them. The pass is bound by the tile's chain of nine products and epilogues
 // and, inside the epilogues, by the L2: its 128 tiles move in step, and write
