@@ -18,7 +18,6 @@ typedef struct BhkImageParams {
   double r_plus, r_minus;  // outer / inner horizon (azimuth conversion)
   double r_hor;            // horizon_factor * r_+
   double r_esc;            // escape_factor * r_obs
-  double inv_r_obs, inv_r_hor, inv_r_esc;  // their reciprocals, as bhh_make_params set them (surrogate refinement)
   double r_in, r_out;      // disk edges
   double sin_o, cos_o;     // observer inclination
   double alpha_min, dalpha, beta_min, dbeta;  // pixel-centre grid

@@ -44,6 +44,13 @@ __device__ __forceinline__ void warp_count(unsigned *stats, int slot, bool pred)
   if ((threadIdx.x & 31u) == 0 && m) atomicAdd(stats + slot, (unsigned)__popc(m));
 }
 
+// 1 / r of the observer, the horizon cut and the escape radius, from the host: an
+// infinite escape radius has 0. Not in BhkImageParams, whose size places the medium in
+// the transfer kernels' constants (24 bytes more: 512^2 mixed 2.29 -> 2.33 ms).
+struct InvRadii {
+  double obs, hor, esc;
+};
+
 // Pixel w of a chunk [p0, p1) of a frame in the order the refinement takes
 // them: the chunk's whole rows [b0, b1) in the tracers' 8 x 4 tiles, so that a
 // warp's rays are neighbours in both directions and take the same branches;
@@ -74,7 +81,8 @@ __global__ void __launch_bounds__(128, FAST ? BH_REFINE_MIN_CTAS : 2) k_surrogat
                                                           double band, int verify, int *__restrict__ list,
                                                           unsigned int *__restrict__ count,
                                                           unsigned int *__restrict__ stats,
-                                                          const __grid_constant__ ChunkRows chunk) {
+                                                          const __grid_constant__ ChunkRows chunk,
+                                                          const __grid_constant__ InvRadii inv) {
   const long long w = chunk.p0 + (long long)blockIdx.x * blockDim.x + threadIdx.x;
   const bool live = w < chunk.p1;
   const long long pix = live ? chunk_pixel(chunk, w, p.width) : 0;
@@ -101,7 +109,7 @@ __global__ void __launch_bounds__(128, FAST ? BH_REFINE_MIN_CTAS : 2) k_surrogat
     if (!(conf >= min_conf)) {
       reason = 1;
     } else {
-      bhmino::Radial q = bhmino::radial_motion(p.a2, p.a2 - a * lam, C, p.r_obs, p.r_plus, p.r_hor, p.inv_r_obs, p.inv_r_hor, p.inv_r_esc);
+      bhmino::Radial q = bhmino::radial_motion(p.a2, p.a2 - a * lam, C, p.r_obs, p.r_plus, p.r_hor, inv.obs, inv.hor, inv.esc);
       if (PHI) bhmino::set_azimuth(q, a, lam);
       const double d = bhmino::critical_distance(q.r_min, q.R_min, a, lam, p.form == 1, p.sin_o, p.cos_o, alpha,
                                                  beta);
@@ -201,7 +209,8 @@ __global__ void __launch_bounds__(BH_REFINE_THREADS, 1)
     k_surrogate_refine_phased(const __grid_constant__ BhkImageParams p, const __grid_constant__ BhkImageOut o,
                               const float *__restrict__ head, float min_conf, double band, int verify,
                               int *__restrict__ list, unsigned int *__restrict__ count,
-                              unsigned int *__restrict__ stats, const __grid_constant__ ChunkRows chunk) {
+                              unsigned int *__restrict__ stats, const __grid_constant__ ChunkRows chunk,
+                              const __grid_constant__ InvRadii inv) {
   const long long w = chunk.p0 + (long long)blockIdx.x * blockDim.x + threadIdx.x;
   const bool live = w < chunk.p1;
   const long long pix = live ? chunk_pixel(chunk, w, p.width) : 0;
@@ -232,7 +241,7 @@ __global__ void __launch_bounds__(BH_REFINE_THREADS, 1)
     if (!(conf >= min_conf)) {
       reason = 1;
     } else {
-      q = bhmino::radial_motion(p.a2, p.a2 - a * lam, C, p.r_obs, p.r_plus, p.r_hor, p.inv_r_obs, p.inv_r_hor, p.inv_r_esc);
+      q = bhmino::radial_motion(p.a2, p.a2 - a * lam, C, p.r_obs, p.r_plus, p.r_hor, inv.obs, inv.hor, inv.esc);
       if (PHI) bhmino::set_azimuth(q, a, lam);
       const double d = bhmino::critical_distance(q.r_min, q.R_min, a, lam, p.form == 1, p.sin_o, p.cos_o, alpha,
                                                  beta);
@@ -373,6 +382,7 @@ extern "C" int bhk_surrogate_refine(const BhkImageParams *p, const BhkImageOut *
   const unsigned blocks = (unsigned)((p1 - p0 + 127) / 128);
   ChunkRows chunk{p0, p1, (p0 + p->width - 1) / p->width * p->width, p1 / p->width * p->width};
   if (chunk.b1 < chunk.b0) chunk.b1 = chunk.b0;
+  const InvRadii inv{1.0 / p->r_obs, 1.0 / p->r_hor, 1.0 / p->r_esc};
   const bool phi = o->phi_hit != nullptr || o->phi_inf != nullptr;
 #if BH_REFINE_PHASED
   // With azimuths the phased kernel is faster (2048^2 frame, serialised:
@@ -381,24 +391,24 @@ extern "C" int bhk_surrogate_refine(const BhkImageParams *p, const BhkImageOut *
   if (!refine_fp64 && phi) {
     const unsigned pb = (unsigned)((p1 - p0 + BH_REFINE_THREADS - 1) / BH_REFINE_THREADS);
     k_surrogate_refine_phased<true, true><<<pb, BH_REFINE_THREADS, 0, s>>>(*p, *o, head, min_conf, band, verify,
-                                                                         list, count, stats, chunk);
+                                                                         list, count, stats, chunk, inv);
     return cudaGetLastError() == cudaSuccess ? 0 : -1;
   }
 #endif
   if (refine_fp64) {
     if (phi)
       k_surrogate_refine<false, true><<<blocks, 128, 0, s>>>(*p, *o, head, min_conf, band, verify, list, count,
-                                                             stats, chunk);
+                                                             stats, chunk, inv);
     else
       k_surrogate_refine<false, false><<<blocks, 128, 0, s>>>(*p, *o, head, min_conf, band, verify, list, count,
-                                                              stats, chunk);
+                                                              stats, chunk, inv);
   } else {
     if (phi)
       k_surrogate_refine<true, true><<<blocks, 128, 0, s>>>(*p, *o, head, min_conf, band, verify, list, count,
-                                                            stats, chunk);
+                                                            stats, chunk, inv);
     else
       k_surrogate_refine<true, false><<<blocks, 128, 0, s>>>(*p, *o, head, min_conf, band, verify, list, count,
-                                                             stats, chunk);
+                                                             stats, chunk, inv);
   }
   return cudaGetLastError() == cudaSuccess ? 0 : -1;
 }

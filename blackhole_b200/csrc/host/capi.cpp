@@ -153,9 +153,6 @@ static BhkImageParams make_params(const BH_KerrScene *s) {
   p.r_minus = k.r_minus;
   p.r_hor = k.r_hor;
   p.r_esc = k.r_esc;
-  p.inv_r_obs = 1.0 / p.r_obs;
-  p.inv_r_hor = 1.0 / p.r_hor;
-  p.inv_r_esc = 1.0 / p.r_esc;
   p.r_in = k.r_in;
   p.r_out = s->disk_r_out;
   p.sin_o = k.sin_o;
