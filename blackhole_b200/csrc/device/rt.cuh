@@ -13,6 +13,7 @@
 // reference GPU kernel's order (src/cuda/device_physics.cuh:1988-2173).
 #pragma once
 
+#include "azimuth_cell.h"
 #include "ieee_fp64.cuh"
 #include "launch.h"
 
@@ -111,13 +112,10 @@ __device__ __forceinline__ bool sample(const BhkRtParams &q, double r, double u,
   j0 = j0 < 0 ? 0 : (j0 > q.n_th - 2 ? q.n_th - 2 : j0);
   double tt = ft - (double)j0;
   tt = tt < 0.0 ? 0.0 : (tt > 1.0 ? 1.0 : tt);
-  const double nph = (double)q.n_ph;
-  const double fp = (phi * (1.0 / kTwoPi)) * nph;
+  const double fp = (phi * (1.0 / kTwoPi)) * (double)q.n_ph;
   const double fl = floor(fp);
   const double tp = fp - fl;
-  int k0 = (int)(fl - nph * floor(fl * q.inv_n_ph));  // the rounded quotient is off by one at most
-  k0 += k0 < 0 ? q.n_ph : (k0 >= q.n_ph ? -q.n_ph : 0);
-  k0 = k0 < 0 ? 0 : (k0 >= q.n_ph ? q.n_ph - 1 : k0);  // an azimuth that is no number
+  const int k0 = azimuth_cell(fl, q.n_ph, q.inv_n_ph);
   const int k1 = k0 + 1 == q.n_ph ? 0 : k0 + 1;
   const float4 *c = reinterpret_cast<const float4 *>(q.cells);
   double acc[3] = {0.0, 0.0, 0.0};
@@ -272,9 +270,7 @@ __device__ __forceinline__ bool sample_f(const MediumF &q, float r, float u, flo
   const float fp = phi * (0.15915494309f * (float)q.n_ph);
   const float fl = floorf(fp);
   const float tp = fp - fl;
-  int k0 = (int)fl - q.n_ph * (int)floorf(fl * q.inv_n_ph);  // the rounded quotient is off by one at most
-  k0 += k0 < 0 ? q.n_ph : (k0 >= q.n_ph ? -q.n_ph : 0);
-  k0 = min(max(k0, 0), q.n_ph - 1);  // an azimuth that is no number
+  const int k0 = azimuth_cell(fl, q.n_ph, q.inv_n_ph);
   const int k1 = (k0 + 1 == q.n_ph) ? 0 : k0 + 1;
   const char *cells = reinterpret_cast<const char *>(q.cells);
   const Off c00 = ((Off)i0 * (Off)q.n_th + (Off)j0) * (Off)q.n_ph * 16u, row = (Off)q.n_th * (Off)q.n_ph * 16u,
