@@ -299,7 +299,8 @@ __global__ void __launch_bounds__(256) k_post_tone(const float *__restrict__ src
     const int64_t g = (int64_t)py * pitch + px;
     const float gch = PLANAR ? src[plane + g] : src[4 * g + 1];
     const float dv = v - 0.5f;
-    const float dist = sqrtf(du * du + dv * dv);
+    // fused as written, for the same values at every ROWS
+    const float dist = sqrtf(__fmaf_rn(du, du, __fmul_rn(dv, dv)));
     const float vig = sqrtf(fmaxf(1.0f - dist * dist * 0.5f, 0.0f));
     fb[i] = make_float4(tone_channel(rb.x, exposure, vig), tone_channel(gch, exposure, vig),
                         tone_channel(rb.y, exposure, vig), 1.0f);
